@@ -168,8 +168,9 @@ void adi_coefficients(double delz, double dgrid, double xks, int ngrid, std::vec
 // x_k = d_k - cwet_{k+1} x_{k+1} backward, forget their starting value by the factor
 // |c_k cbet_k| or |cwet_k| per element (about the step factor dz / (4 xks dgrid^2),
 // a few percent on the grids of these runs). A line can then be split into segments
-// solved in parallel, each started W elements early from zero: the error is below
-// alpha^W <= 2^-bits of the solution (bits = 32 for the FP32 solves), under the
+// solved in parallel, each started W elements early from zero (FP32 solves) or corrected
+// by its neighbours' carries over W elements (FP64 solves): the error is below alpha^W <=
+// 2^-bits of the solution (bits = 32 for the FP32 solves, 62 for the FP64 ones), under the
 // form's rounding. Returns 0 when alpha is too large for a short warm-up (the solves
 // then run one thread per line).
 int segment_warmup(const std::vector<std::complex<double>> &c, const std::vector<std::complex<double>> &cbet,
@@ -400,7 +401,7 @@ void g4gpu_destroy(g4gpu_handle h) {
                   h->wake_tab, h->wake_loss, h->wake_lossf, h->wake_scratch, h->count_buf, h->sort_iscratch,
                   h->sort_scratch[0], h->sort_scratch[1], h->sort_scratch[2], h->sort_scratch[3],
                   h->sort_scratch[4], h->sort_scratch[5], h->isr_ctr, h->sub_theta, h->sub_x, h->sub_y,
-                  h->beam.phasor, h->beam.phasor_ok};
+                  h->beam.phasor, h->beam.phasor_ok, h->seg_pow};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (int k = 0; k < G4GPU_MAX_FIELDS; k++) {
@@ -432,6 +433,7 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
   typedef std::complex<double> cd;
   std::map<std::pair<int, double>, int> sets;  // (field, delz) -> set
   std::vector<cd> coefs;                       // [nset][3][ng]
+  std::vector<cd> pows;                        // plain form: [nset][2][kSegPow]
   std::vector<int> set_tw;                     // warm-up length per coefficient set
   for (int i = 0; i < nsteps; i++) {
     const double *r = tab + (size_t)i * G4GPU_LAT_NCOL;
@@ -514,7 +516,20 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
         coefs.insert(coefs.end(), cc.begin(), cc.end());
         coefs.insert(coefs.end(), cb.begin(), cb.end());
         coefs.insert(coefs.end(), cw.begin(), cw.end());
-        set_tw.push_back(segment_warmup(cc, cb, cw, 32));
+        set_tw.push_back(segment_warmup(cc, cb, cw, h->mixed ? 32 : 62));
+        if (!h->mixed) {
+          // kappa^{j+1} and kappa^{j+1} / (1 - kappa^2) of the settled recurrences,
+          // kappa = -cwet (adi_plain.cuh)
+          const cd kappa = -cw[ng - 1], q = 1. / (1. - kappa * kappa);
+          cd p = kappa;
+          std::vector<cd> pw(g4::kSegPow);
+          for (cd &v : pw) {
+            v = p;
+            p *= kappa;
+          }
+          pows.insert(pows.end(), pw.begin(), pw.end());
+          for (const cd &v : pw) pows.push_back(v * q);
+        }
         it = sets.find(key);
       }
       f.coef = it->second;
@@ -559,6 +574,19 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
     h->bytes -= h->coef_bytes;
     h->coef = nullptr;
     h->coef_bytes = 0;
+  }
+  if (h->seg_pow) {
+    cudaFree(h->seg_pow);
+    h->bytes -= h->seg_pow_bytes;
+    h->seg_pow = nullptr;
+    h->seg_pow_bytes = 0;
+  }
+  if (!pows.empty()) {
+    const size_t nb = pows.size() * sizeof(cd);
+    int rc = alloc(h, &h->seg_pow, nb);
+    if (rc) return rc;
+    h->seg_pow_bytes = nb;
+    G4_CUDA(h, cudaMemcpy(h->seg_pow, pows.data(), nb, cudaMemcpyHostToDevice));
   }
   if (!coefs.empty()) {
     size_t n = coefs.size();
@@ -1355,7 +1383,9 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
           if (h->mixed)
             g4::launch_adi_mixed(L, scf, k, phase, h->field[k], srck, h->tmp, cb, ns, ng);
           else
-            g4::launch_adi_plain(L, sc, k, phase, h->field[k], srck, h->tmp, cb, ns, ng);
+            g4::launch_adi_plain(L, sc, k, phase, h->field[k], h->src[k], h->tmp, cb,
+                                 (const char *)h->seg_pow + (size_t)sc.f[k].coef * 2 * g4::kSegPow * 2 * sizeof(double), ns, ng,
+                                 srck != nullptr);
         }
       }
     }

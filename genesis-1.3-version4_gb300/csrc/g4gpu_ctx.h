@@ -29,6 +29,8 @@ struct g4gpu_ctx {
   void *diag_work = nullptr;  // g4gpu_diag_fft's scratch where tmp is absent
   void *coef = nullptr;      // [nset][3][ngrid] complex of the field type
   size_t coef_bytes = 0;
+  void *seg_pow = nullptr;   // plain form: [nset][2][kSegPow] powers of the segmented solves
+  size_t seg_pow_bytes = 0;
   // FFT solver tables per field: roots of unity [n], Im(K2) and the sigmoid [n^2]
   void *fft_roots[G4GPU_MAX_FIELDS] = {};
   double fft_k2c[G4GPU_MAX_FIELDS] = {};  // -dk^2 / (2 xks): Im(K2) = (dx^2 + dy^2) k2c

@@ -16,6 +16,10 @@ constexpr double kVacimp = 376.73;
 constexpr double kEev = 510998.95069;
 constexpr double kCe = 4.8032045e-11;
 
+// Entries of a coefficient set's powers for the FP64 segmented solves: the largest
+// warm-up length segment_warmup returns for 62 bits
+constexpr int kSegPow = 41;
+
 // Per field, per integration step constants.
 struct FieldStep {
   double rtmp;    // fc(h) / xks of this field (BeamSolver.cpp:28)
@@ -29,7 +33,7 @@ struct FieldStep {
   int dep_on;     // deposition active: in undulator and odd harmonic (FieldSolverADI.cpp:20)
   int coef;       // index of the ADI coefficient set of this (field, delz)
   int first;      // ring start of the field when the step runs (filled at launch)
-  int tw;         // warm-up length of the segmented FP32 tridiagonal solves, 0: not applicable
+  int tw;         // warm-up length of the form's segmented tridiagonal solves, 0: not applicable
   double idgrid;  // 1 / dgrid: the FP64 push's cell lookup multiplies
   double gm_idg;  // gridmax / dgrid: the FP64 cell coordinate is fma(x, idgrid, gm_idg)
   // The FP64 push forms e^{i h theta} at its RK4 stages by rotating e^{i h theta0}: by
@@ -132,9 +136,11 @@ void launch_push_plain(const Launch &L, const StepConst &sc, const DeviceBeam &b
                        int deposit, int block);
 void launch_deposit_plain(const Launch &L, const StepConst &sc, const DeviceBeam &b,
                           void *const *src, int ns, int np, int ngrid);
-// phase 0: implicit along x into tmp; phase 1: implicit along y back into the field
-void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, void *field,
-                      const void *src, void *tmp, const void *coef, int ns, int ngrid);
+// phase 0: implicit along x into tmp; phase 1: implicit along y back into the field.
+// src: the deposited source (has_src), overwritten as scratch between the two phases;
+// pow: the coefficient set's [2][kSegPow] powers
+void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, void *field, void *src, void *tmp,
+                      const void *coef, const void *pow, int ns, int ngrid, int has_src);
 void launch_diag_beam_plain(const Launch &L, const DeviceBeam &b, int ns, int np, int nharm,
                             double *out);
 void launch_diag_field_plain(const Launch &L, const void *field, int ns, int ngrid,

@@ -12,6 +12,9 @@
 // beam slice.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "g4gpu_internal.h"
 #include "philox.cuh"
 
@@ -562,9 +565,10 @@ __global__ void __launch_bounds__(256) k_deposit(StepConst sc, Ptrs p, int ns, i
                        p.theta[o], p.x[o], p.y[o]);
 }
 
-// ADI coefficient set: c[ng], cbet[ng], cwet[ng] (FieldSolverADI.cpp:125-182)
+// ADI coefficient set: c[ng], cbet[ng], cwet[ng] (FieldSolverADI.cpp:125-182), and the
+// segmented solves' powers [2][kSegPow]: kappa^{j+1}, kappa^{j+1} / (1 - kappa^2)
 struct Coef {
-  const double2 *c, *cbet, *cwet;
+  const double2 *c, *cbet, *cwet, *pw;
 };
 
 // Right-hand side term cstep * (second difference) with the reference's operand
@@ -650,6 +654,8 @@ __global__ void __launch_bounds__(128) k_adi_y(double2 *__restrict__ field,
     next = v;
   }
 }
+
+#include "adi_plain.cuh"
 
 // ---- diagnostics: per-slice FP64 sums, finished on the host -----------------
 template <int BS>
@@ -932,24 +938,93 @@ void launch_deposit_plain(const Launch &L, const StepConst &sc, const DeviceBeam
   }
 }
 
-void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, void *field,
-                      const void *src, void *tmp, const void *coef, int ns, int ngrid) {
+namespace {
+// How launch_adi_plain cuts the lines of a window: L lines a CTA, nseg segments a line
+// (0: one thread per line, k_adi_x / k_adi_y), threads a CTA.
+struct AdiShape {
+  int L, nseg, threads;
+};
+// Why these: a warp's FP64 instruction holds its scheduler for 64 cycles whatever lanes
+// are active, so the solve wants full warps, enough of them on every SM, and no more
+// segments than that takes (each adds 16 W instructions a line). Measured (both half
+// steps, step factor 0.034, W 13; in brackets one thread per line):
+//   1 slice x 255^2     L 2, nseg 19   41 us (688)      22 x 101^2   L 4, nseg 6   53 us (292)
+//   4 x 151^2           L 2, nseg 8    45 us (428)      60 x 151^2   L 8, nseg 4  136 us (446)
+//   320 x 151^2         L 8, nseg 4   624 us (870)      320 x 255^2  L 8, nseg 8 1640 us (2350)
+// so: at four CTAs an SM of 8 lines and segments of about 36 elements, that; below, the
+// most segments and fewer lines, down to 2. Two segments of 16 lines fill a warp where
+// the warm-up leaves no more (2000 x 101^2: 1835 us, one thread per line 1925). One
+// segment is slower than one thread per line (320 x 151^2: 967 us), as are lines of which
+// two do not fit shared memory.
+AdiShape adi_shape(int ns, int ng, int W) {
+  const int most = W > 0 ? ng / W : 1;
+  if (most < 2) return {0, 0, 128};
+  AdiShape s{8, 4 * std::max(1, (ng + 70) / 144), 64};
+  const long long bands = (long long)ns * ((ng + 7) / 8);
+  if (bands < 4 * 152) {
+    s.L = bands < 152 ? 2 : 4;
+    s.threads = 128;
+    s.nseg = s.threads / s.L;
+  } else if (most < 4) {
+    s.L = 16;
+  }
+  s.nseg = std::min(s.nseg, most);
+  while (s.L > 2 && (size_t)s.L * (ng | 1) * sizeof(double2) > 100 * 1024) s.L /= 2;
+  if ((size_t)s.L * (ng | 1) * sizeof(double2) > 100 * 1024) return {0, 0, 128};
+  s.threads = std::max(s.threads, (s.L * s.nseg + 31) / 32 * 32);
+  if (s.threads > 512) {
+    s.threads = 512;
+    s.nseg = 512 / s.L;
+  }
+  return s;
+}
+
+template <int L>
+void launch_adi_lines(cudaStream_t st, int phase, const AdiShape &a, double2 *field, double2 *src, double2 *tmp,
+                      const Coef &cf, double c, int ns, int ng, int first, int W, int has_src) {
+  static std::atomic<unsigned long long> configured{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !(configured.load() & (1ull << dev))) {
+    cudaFuncSetAttribute(adi64::k_adi_rows<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+    cudaFuncSetAttribute(adi64::k_adi_cols<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+    if (dev < 64) configured.fetch_or(1ull << dev);
+  }
+  const int nband = (ng + L - 1) / L, nco = std::min(W, ng);
+  const size_t smem = adi64::lines_bytes(L, L * (phase == 0 ? ng | 1 : ng), a.nseg, nco, W);
+  const unsigned blocks = (unsigned)ns * (unsigned)nband;
+  if (phase == 0)
+    adi64::k_adi_rows<L><<<blocks, a.threads, smem, st>>>(field, src, tmp, cf, c, ns, ng, first, nband, a.nseg, nco,
+                                                          W, has_src);
+  else
+    adi64::k_adi_cols<L><<<blocks, a.threads, smem, st>>>(field, src, tmp, cf, c, ns, ng, first, nband, a.nseg, nco,
+                                                          W);
+}
+}  // namespace
+
+void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, void *field, void *src, void *tmp,
+                      const void *coef, const void *pow, int ns, int ngrid, int has_src) {
   const double2 *cb = (const double2 *)coef;
   cudaStream_t s = (cudaStream_t)L.stream;
-  // One thread per grid line over all slices. The FP64 ADI is bound by the FP64 rate
-  // (about 76 FP64 operations per cell and step; GB300 runs FP64 at 1/64 of the FP32
-  // rate), not by memory: these kernels keep every line's sweep as the reference's single
-  // sequential pass. The tiled passes of adi_tiled.cuh, which split lines into segments
-  // with redundant warm-up work, were measured slower for this form.
-  Coef cf{cb, cb + ngrid, cb + 2 * ngrid};
-  long long n = (long long)ns * ngrid;
-  unsigned blocks = (unsigned)((n + 127) / 128);
+  const FieldStep &f = sc.f[k];
+  const Coef cf{cb, cb + ngrid, cb + 2 * ngrid, (const double2 *)pow};
+  double2 *u = (double2 *)field, *sv = (double2 *)src, *w = (double2 *)tmp;
+  const AdiShape a = adi_shape(ns, ngrid, f.tw);
+  switch (a.L) {
+    case 2: return launch_adi_lines<2>(s, phase, a, u, sv, w, cf, f.cstep, ns, ngrid, f.first, f.tw, has_src);
+    case 4: return launch_adi_lines<4>(s, phase, a, u, sv, w, cf, f.cstep, ns, ngrid, f.first, f.tw, has_src);
+    case 8: return launch_adi_lines<8>(s, phase, a, u, sv, w, cf, f.cstep, ns, ngrid, f.first, f.tw, has_src);
+    case 16: return launch_adi_lines<16>(s, phase, a, u, sv, w, cf, f.cstep, ns, ngrid, f.first, f.tw, has_src);
+    default: break;
+  }
+  // one thread per line, each line's sweep the reference's single sequential pass
+  const double2 *sr = has_src ? sv : nullptr;
+  const long long n = (long long)ns * ngrid;
+  const unsigned blocks = (unsigned)((n + 127) / 128);
   if (phase == 0)
-    k_adi_x<<<blocks, 128, 0, s>>>((const double2 *)field, (const double2 *)src, (double2 *)tmp,
-                                   cf, sc.f[k].cstep, ns, ngrid, sc.f[k].first);
+    k_adi_x<<<blocks, 128, 0, s>>>(u, sr, w, cf, f.cstep, ns, ngrid, f.first);
   else
-    k_adi_y<<<blocks, 128, 0, s>>>((double2 *)field, (const double2 *)src, (const double2 *)tmp,
-                                   cf, sc.f[k].cstep, ns, ngrid, sc.f[k].first);
+    k_adi_y<<<blocks, 128, 0, s>>>(u, sr, w, cf, f.cstep, ns, ngrid, f.first);
 }
 
 void launch_diag_beam_plain(const Launch &L, const DeviceBeam &b, int ns, int np, int nharm,
