@@ -284,6 +284,11 @@ int g4_fail(g4gpu_handle h, int code, const std::string &msg) { return fail(h, c
 int g4_cuda_fail(g4gpu_handle h, cudaError_t e, const char *what) { return cuda_fail(h, e, what); }
 int g4_alloc(g4gpu_handle h, void **p, size_t n) { return alloc(h, p, n); }
 int g4_check_device_flag(g4gpu_handle h) { return check_device_flag(h); }
+// The FP64 push's cached phasors no longer match theta (a load, a sort, a restored or
+// copied state, a closure's correction)
+void g4_phasor_stale(g4gpu_handle h) {
+  if (h->beam.phasor_ok) cudaMemsetAsync(h->beam.phasor_ok, 0, sizeof(int), h->stream);
+}
 
 extern "C" {
 
@@ -730,10 +735,7 @@ int g4gpu_set_chicanes(g4gpu_handle h, int nsteps, const double *table) {
   return G4GPU_OK;
 }
 
-// The FP64 push's cached phasors no longer match theta (a load, a sort, a restored state)
-static void phasor_stale(g4gpu_handle h) {
-  if (h->beam.phasor_ok) cudaMemsetAsync(h->beam.phasor_ok, 0, sizeof(int), h->stream);
-}
+static void phasor_stale(g4gpu_handle h) { g4_phasor_stale(h); }
 
 static int ensure_stage(g4gpu_handle h, size_t n) {
   if (h->stage_bytes >= n) return G4GPU_OK;

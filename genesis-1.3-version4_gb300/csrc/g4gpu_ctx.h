@@ -144,3 +144,4 @@ int g4_fail(g4gpu_handle h, int code, const std::string &msg);
 int g4_cuda_fail(g4gpu_handle h, cudaError_t e, const char *what);
 int g4_alloc(g4gpu_handle h, void **p, size_t n);
 int g4_check_device_flag(g4gpu_handle h);
+void g4_phasor_stale(g4gpu_handle h);

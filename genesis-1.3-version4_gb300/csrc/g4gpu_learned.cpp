@@ -467,6 +467,7 @@ int g4gpu_closure_apply(g4gpu_handle h, const float *corr) {
   if (e != cudaSuccess) return g4_cuda_fail(h, e, "closure corrections");
   g4::closure_apply(h->stream, h->beam.theta, h->beam.gamma, h->field[0], h->closure_corr, h->mixed, c.nslice,
                     c.npart, c.ngrid, h->first[0]);
+  g4_phasor_stale(h);
   h->launches[G4GPU_K_MISC]++;
   return G4GPU_OK;
 }
@@ -505,6 +506,7 @@ static int closure_correct(g4gpu_handle h) {
                           m->dims[kLayers]);
   g4::closure_apply(h->stream, h->beam.theta, h->beam.gamma, h->field[0], h->closure_corr, h->mixed, ns,
                     c.npart, c.ngrid, h->first[0]);
+  g4_phasor_stale(h);
   m->stream = saved;
   m->derr = saved_err;
   h->launches[G4GPU_K_MISC] += 3 + kLayers;
@@ -566,6 +568,7 @@ int g4gpu_copy_state(g4gpu_handle dst, g4gpu_handle src) {
     dst->field_loaded[k] = true;
   }
   if (e != cudaSuccess) return g4_cuda_fail(dst, e, "copy_state");
+  g4_phasor_stale(dst);
   dst->beam_loaded = true;
   // the source must not be modified before the copy has read it
   cudaEvent_t ev2;
