@@ -406,7 +406,7 @@ void g4gpu_destroy(g4gpu_handle h) {
                   h->wake_tab, h->wake_loss, h->wake_lossf, h->wake_scratch, h->count_buf, h->sort_iscratch,
                   h->sort_scratch[0], h->sort_scratch[1], h->sort_scratch[2], h->sort_scratch[3],
                   h->sort_scratch[4], h->sort_scratch[5], h->isr_ctr, h->sub_theta, h->sub_x, h->sub_y,
-                  h->beam.phasor, h->beam.phasor_ok, h->seg_pow};
+                  h->beam.phasor, h->beam.phasor_ok, h->seg_pow, h->diag_part, h->diag_count};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (int k = 0; k < G4GPU_MAX_FIELDS; k++) {
@@ -1512,6 +1512,27 @@ size_t diag_record_doubles(const g4gpu_config &c, int nharm) {
   return (size_t)c.nslice * g4::beam_diag_width(nharm) + (size_t)c.nfield * c.nslice * (g4::kFieldSums + 2);
 }
 
+// The plain form's diagnostic scratch for nharm harmonics.
+int diag_scratch(g4gpu_handle h, int nharm) {
+  if (h->mixed) return G4GPU_OK;
+  const g4gpu_config &c = h->cfg;
+  size_t counters;
+  const size_t n = g4::diag_plain_scratch(c.nslice, c.npart, nharm, c.ngrid, c.nfield, &counters);
+  int rc;
+  if (!h->diag_count) {
+    if ((rc = alloc(h, (void **)&h->diag_count, counters * sizeof(unsigned)))) return rc;
+    G4_CUDA(h, cudaMemsetAsync(h->diag_count, 0, counters * sizeof(unsigned), h->stream));
+  }
+  if (n <= h->diag_part_n) return G4GPU_OK;
+  if (h->diag_part) cudaFree(h->diag_part);
+  h->bytes -= h->diag_part_n * sizeof(double);
+  h->diag_part = nullptr;
+  h->diag_part_n = 0;
+  if ((rc = alloc(h, (void **)&h->diag_part, n * sizeof(double)))) return rc;
+  h->diag_part_n = n;
+  return G4GPU_OK;
+}
+
 // Queues the kernels of one diagnostic record of the current state into `rec`.
 void enqueue_diag(g4gpu_handle h, int nharm, double *rec, bool beam, bool field) {
   const g4gpu_config &c = h->cfg;
@@ -1519,20 +1540,24 @@ void enqueue_diag(g4gpu_handle h, int nharm, double *rec, bool beam, bool field)
   int bw = g4::beam_diag_width(nharm), fw = g4::kFieldSums + 2;
   g4::Launch L{h->stream, h->derr};
   double *db = rec, *dfd = rec + (size_t)ns * bw;
+  if (!h->mixed) {
+    if (!beam && !field) return;
+    int h1 = -1;
+    for (int k = 0; k < c.nfield && h1 < 0; k++)
+      if (c.harm[k] == 1) h1 = k;
+    Timed t(h, G4GPU_K_DIAG);
+    g4::launch_diag_plain(L, h->beam, h->field, c.nfield, h1, ns, np, ng, nharm, beam, field, rec, h->diag_part,
+                          h->diag_count);
+    return;
+  }
   if (beam) {
     Timed t(h, G4GPU_K_DIAG);
-    if (h->mixed)
-      g4::launch_diag_beam_mixed(L, h->beam, c.gammaref, ns, np, nharm, db);
-    else
-      g4::launch_diag_beam_plain(L, h->beam, ns, np, nharm, db);
+    g4::launch_diag_beam_mixed(L, h->beam, c.gammaref, ns, np, nharm, db);
   }
   if (field) {
     for (int k = 0; k < c.nfield; k++) {
       Timed t(h, G4GPU_K_DIAG);
-      if (h->mixed)
-        g4::launch_diag_field_mixed(L, h->field[k], ns, ng, dfd + (size_t)k * ns * fw);
-      else
-        g4::launch_diag_field_plain(L, h->field[k], ns, ng, dfd + (size_t)k * ns * fw);
+      g4::launch_diag_field_mixed(L, h->field[k], ns, ng, dfd + (size_t)k * ns * fw);
     }
   }
 }
@@ -1632,7 +1657,7 @@ int g4gpu_diag(g4gpu_handle h, int nharm, double *beam_out, double *field_out) {
   cudaSetDevice(h->cfg.device);
   const size_t need = diag_record_doubles(h->cfg, nharm) * sizeof(double);
   int rc = diag_buffers(h, need);
-  if (rc) return rc;
+  if (rc || (rc = diag_scratch(h, nharm))) return rc;
   enqueue_diag(h, nharm, h->ddiag, beam_out != nullptr, field_out != nullptr);
   G4_CUDA(h, cudaGetLastError());
   G4_CUDA(h, cudaMemcpyAsync(h->hdiag, h->ddiag, need, cudaMemcpyDeviceToHost, h->stream));
@@ -1791,7 +1816,7 @@ int g4gpu_run_diag(g4gpu_handle h, int istep0, int nsteps, int nharm, double *be
   const g4gpu_config &c = h->cfg;
   const size_t rec = diag_record_doubles(c, nharm);
   int rc = diag_buffers(h, (size_t)nsteps * rec * sizeof(double));
-  if (rc) return rc;
+  if (rc || (rc = diag_scratch(h, nharm))) return rc;
   std::vector<int> firsts((size_t)nsteps * G4GPU_MAX_FIELDS);
   // each step's record is copied back as soon as it is formed and finished on the host
   // while the device runs the later steps

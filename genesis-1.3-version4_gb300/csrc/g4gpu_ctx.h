@@ -37,6 +37,11 @@ struct g4gpu_ctx {
   void *fft_sig[G4GPU_MAX_FIELDS] = {};
   g4::FFTPlan fft_plan{};
   int *derr = nullptr;
+  // plain form: partial sums and per-slice tickets of the diagnostic kernel, for up to
+  // diag_part_n doubles
+  double *diag_part = nullptr;
+  unsigned *diag_count = nullptr;
+  size_t diag_part_n = 0;
   double *ddiag = nullptr;
   size_t ddiag_bytes = 0;
   double *hdiag = nullptr;  // pinned host copy of ddiag (the per-step read-back)

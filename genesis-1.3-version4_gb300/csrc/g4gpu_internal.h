@@ -141,10 +141,13 @@ void launch_deposit_plain(const Launch &L, const StepConst &sc, const DeviceBeam
 // pow: the coefficient set's [2][kSegPow] powers
 void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, void *field, void *src, void *tmp,
                       const void *coef, const void *pow, int ns, int ngrid, int has_src);
-void launch_diag_beam_plain(const Launch &L, const DeviceBeam &b, int ns, int np, int nharm,
-                            double *out);
-void launch_diag_field_plain(const Launch &L, const void *field, int ns, int ngrid,
-                             double *out);
+// One diagnostic record (beam [nslice][beam_diag_width(nharm)], then per field
+// [nslice][kFieldSums + 2] in storage order) of the current state in one launch. h1: the
+// field of harmonic 1 (its cached phasors are e^{i theta}), -1 without one. scratch and
+// count: diag_plain_scratch's doubles and counters (zeroed once, left zero).
+size_t diag_plain_scratch(int ns, int np, int nharm, int ng, int nfield, size_t *counters);
+void launch_diag_plain(const Launch &L, const DeviceBeam &b, void *const *field, int nfield, int h1, int ns, int np,
+                       int ngrid, int nharm, bool beam, bool fields, double *rec, double *scratch, unsigned *count);
 
 // kernels_mixed.cu (FP32 field, FP64 phase)
 void launch_push_mixed(const Launch &L, const StepConstF &sc, const DeviceBeam &b,

@@ -30,7 +30,6 @@ __device__ __forceinline__ C2 ld(const double2 *p) {
 }
 __device__ __forceinline__ void st(double2 *p, C2 v) { *p = make_double2(v.x, v.y); }
 __device__ __forceinline__ C2 cadd(C2 a, C2 b) { return {a.x + b.x, a.y + b.y}; }
-__device__ __forceinline__ C2 csub(C2 a, C2 b) { return {a.x - b.x, a.y - b.y}; }
 // The std::complex<double> product (ac - bd, ad + bc), with each component's first
 // product fused into its sum: one rounding fewer per component than GCC's evaluation
 // (a last-bit difference), and two FP64 instructions instead of three
@@ -657,115 +656,7 @@ __global__ void __launch_bounds__(128) k_adi_y(double2 *__restrict__ field,
 
 #include "adi_plain.cuh"
 
-// ---- diagnostics: per-slice FP64 sums, finished on the host -----------------
-template <int BS>
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  double r = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < BS / 32; i++) r += sh[i];
-  return r;
-}
-template <int BS, bool MAX>
-__device__ __forceinline__ double block_ext(double v, double *sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double w = __shfl_down_sync(0xffffffffu, v, o);
-    v = MAX ? fmax(v, w) : fmin(v, w);
-  }
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  double r = sh[0];
-  if (threadIdx.x == 0)
-    for (int i = 1; i < BS / 32; i++) r = MAX ? fmax(r, sh[i]) : fmin(r, sh[i]);
-  return r;
-}
-
-// DiagBeam::getValues sums (Diagnostic.cpp:415-456): one block per slice.
-template <int BS>
-__global__ void __launch_bounds__(BS) k_diag_beam(Ptrs p, int np, int nharm, double *out) {
-  __shared__ double sh[BS / 32];
-  int is = blockIdx.x;
-  size_t base = (size_t)is * np;
-  const int n = slice_np(p, is, np);
-  double s[kBeamSums] = {0};
-  double mn[5] = {1e5, 1e5, 1e5, 1e5, 1e7}, mx[5] = {-1e5, -1e5, -1e5, -1e5, 1};
-  double br[G4GPU_MAX_HARM], bi[G4GPU_MAX_HARM];
-  for (int h = 0; h < G4GPU_MAX_HARM; h++) br[h] = bi[h] = 0;
-  for (int ip = threadIdx.x; ip < n; ip += BS) {
-    double x = p.x[base + ip], y = p.y[base + ip], g = p.gamma[base + ip];
-    double px = p.px[base + ip], py = p.py[base + ip], th = p.theta[base + ip];
-    s[0] += g; s[1] += g * g; s[2] += x; s[3] += x * x; s[4] += y; s[5] += y * y;
-    s[6] += px; s[7] += px * px; s[8] += py; s[9] += py * py; s[10] += x * px; s[11] += y * py;
-    mn[0] = fmin(mn[0], x); mx[0] = fmax(mx[0], x);
-    mn[1] = fmin(mn[1], px); mx[1] = fmax(mx[1], px);
-    mn[2] = fmin(mn[2], y); mx[2] = fmax(mx[2], y);
-    mn[3] = fmin(mn[3], py); mx[3] = fmax(mx[3], py);
-    mn[4] = fmin(mn[4], g); mx[4] = fmax(mx[4], g);
-    for (int h = 0; h < nharm && h < G4GPU_MAX_HARM; h++) {
-      double sn, cs;
-      sincos((h + 1) * th, &sn, &cs);
-      br[h] += cs;
-      bi[h] += sn;
-    }
-  }
-  int w = beam_diag_width(nharm);
-  double *o = out + (size_t)is * w;
-  for (int k = 0; k < kBeamSums; k++) {
-    double r = block_sum<BS>(s[k], sh);
-    if (threadIdx.x == 0) o[k] = r;
-  }
-  for (int k = 0; k < 5; k++) {
-    double a = block_ext<BS, false>(mn[k], sh);
-    if (threadIdx.x == 0) o[kBeamSums + 2 * k] = a;
-    double b = block_ext<BS, true>(mx[k], sh);
-    if (threadIdx.x == 0) o[kBeamSums + 2 * k + 1] = b;
-  }
-  for (int h = 0; h < nharm && h < G4GPU_MAX_HARM; h++) {
-    double a = block_sum<BS>(br[h], sh);
-    double b = block_sum<BS>(bi[h], sh);
-    if (threadIdx.x == 0) {
-      o[kBeamSums + kBeamMinMax + 2 * h] = a;
-      o[kBeamSums + kBeamMinMax + 2 * h + 1] = b;
-    }
-  }
-}
-
-// DiagField::getValues sums (Diagnostic.cpp:754-776): one block per storage slot.
-template <int BS>
-__global__ void __launch_bounds__(BS) k_diag_field(const double2 *field, int ng, double *out) {
-  __shared__ double sh[BS / 32];
-  int is0 = blockIdx.x;
-  size_t ncell = (size_t)ng * ng;
-  const double2 *f = field + (size_t)is0 * ncell;
-  double shift = -0.5 * (double)(ng - 1);
-  double s[7] = {0};
-  for (size_t i = threadIdx.x; i < ncell; i += BS) {
-    int iy = (int)(i / ng), ix = (int)(i % ng);
-    double dx = (double)ix + shift, dy = (double)iy + shift;
-    double2 v = f[i];
-    double wei = v.x * v.x + v.y * v.y;
-    s[0] += wei; s[1] += dx * wei; s[2] += dx * dx * wei; s[3] += dy * wei; s[4] += dy * dy * wei;
-    s[5] += v.x; s[6] += v.y;
-  }
-  double *o = out + (size_t)is0 * (kFieldSums + 2);
-  for (int k = 0; k < 7; k++) {
-    double r = block_sum<BS>(s[k], sh);
-    if (threadIdx.x == 0) o[k] = r;
-  }
-  if (threadIdx.x == 0) {
-    double2 v = f[(size_t)(ng / 2) * ng + ng / 2];
-    o[7] = v.x;
-    o[8] = v.y;
-  }
-}
+#include "diag_plain.cuh"
 
 Ptrs make_ptrs(const DeviceBeam &b, void *const *field, void *const *src, int nfld) {
   Ptrs p{};
@@ -1027,15 +918,73 @@ void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, vo
     k_adi_y<<<blocks, 128, 0, s>>>(u, sr, w, cf, f.cstep, ns, ngrid, f.first);
 }
 
-void launch_diag_beam_plain(const Launch &L, const DeviceBeam &b, int ns, int np, int nharm,
-                            double *out) {
-  Ptrs p = make_ptrs(b, nullptr, nullptr, 0);
-  k_diag_beam<256><<<ns, 256, 0, (cudaStream_t)L.stream>>>(p, np, nharm, out);
+namespace {
+// One CTA of threads per column width of the grid (two or more columns a thread above
+// 256), so that the FP64 pipe, which a warp's instruction holds whatever lanes are active,
+// runs full warps.
+int diag_threads(int ng) {
+  const int per = (ng + 255) / 256, cols = (ng + per - 1) / per;
+  return std::max(128, (cols + 31) / 32 * 32);
+}
+// Particles a thread: the reduction over a CTA costs its threads about 35 FP64
+// instructions each, a particle 14, so 8 of them where that still leaves two CTAs an SM,
+// fewer in a window of few slices (1 slice x 8192: 32 CTAs of 256).
+int diag_chunk(int ns, int np, int nt) {
+  int m = 8;
+  while (m > 1 && (long long)ns * ((np + m * nt - 1) / (m * nt)) < 2 * 152) m /= 2;
+  return m * nt;
+}
+// Rows a CTA: 32, or fewer down to 2 for about four CTAs an SM.
+int diag_rows(int nslice, int ng) {
+  return (int)std::max(2LL, std::min(32LL, (long long)nslice * ng / (4 * 152)));
+}
+template <int NH>
+void launch_diag_nh(cudaStream_t s, const diag64::Args &a, unsigned blocks, int nt) {
+  static std::atomic<unsigned long long> configured{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !(configured.load() & (1ull << dev))) {
+    cudaFuncSetAttribute(diag64::k_diag<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+    if (dev < 64) configured.fetch_or(1ull << dev);
+  }
+  const size_t smem = (size_t)diag64::kSlots<NH> * (nt + 1) * sizeof(double);
+  diag64::k_diag<NH><<<blocks, nt, smem, s>>>(a);
+}
+}  // namespace
+
+size_t diag_plain_scratch(int ns, int np, int nharm, int ng, int nfield, size_t *counters) {
+  const int nt = diag_threads(ng), chunk = diag_chunk(ns, np, nt), rows = diag_rows(ns * nfield, ng);
+  *counters = (size_t)ns * (1 + nfield);
+  return (size_t)ns * ((np + chunk - 1) / chunk) * beam_diag_width(nharm <= 1 ? 1 : nharm <= 3 ? 3 : G4GPU_MAX_HARM) +
+         (size_t)nfield * ns * ((ng + rows - 1) / rows) * kFieldSums;
 }
 
-void launch_diag_field_plain(const Launch &L, const void *field, int ns, int ngrid,
-                             double *out) {
-  k_diag_field<256><<<ns, 256, 0, (cudaStream_t)L.stream>>>((const double2 *)field, ngrid, out);
+void launch_diag_plain(const Launch &L, const DeviceBeam &b, void *const *field, int nfield, int h1, int ns, int np,
+                       int ngrid, int nharm, bool beam, bool fields, double *rec, double *scratch, unsigned *count) {
+  diag64::Args a{};
+  a.p = make_ptrs(b, field, nullptr, nfield);
+  const int nt = diag_threads(ngrid);
+  a.ns = ns;
+  a.np = np;
+  a.nharm = nharm;
+  a.ng = ngrid;
+  a.chunk = diag_chunk(ns, np, nt);
+  a.nbc = beam ? (np + a.chunk - 1) / a.chunk : 0;
+  a.rows = diag_rows(ns * nfield, ngrid);
+  a.nfc = (ngrid + a.rows - 1) / a.rows;
+  a.ph1 = h1 >= 0 && b.phasor ? (const double2 *)b.phasor + (size_t)h1 * ns * np : nullptr;
+  a.rec = rec;
+  a.part = scratch;
+  a.count = count;
+  const unsigned blocks = (unsigned)ns * a.nbc + (fields ? (unsigned)nfield * ns * a.nfc : 0u);
+  if (!blocks) return;
+  cudaStream_t s = (cudaStream_t)L.stream;
+  if (nharm <= 1)
+    launch_diag_nh<1>(s, a, blocks, nt);
+  else if (nharm <= 3)
+    launch_diag_nh<3>(s, a, blocks, nt);
+  else
+    launch_diag_nh<G4GPU_MAX_HARM>(s, a, blocks, nt);
 }
 
 }  // namespace g4
