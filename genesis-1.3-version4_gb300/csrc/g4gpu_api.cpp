@@ -548,6 +548,8 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
     s.half_delz = s.delz * 0.5;
     s.aw_t2 = s.aw_t * s.aw_t;
     s.aw2 = s.aw * s.aw;
+    s.qdx2 = s.qx * s.half_delz * s.half_delz;
+    s.qdy2 = s.qy * s.half_delz * s.half_delz;
     {
       // dtheta/dz of the ODE (BeamSolver.cpp:144-163) at gammaref, on axis, no field
       const double bpar = std::sqrt(1. - (1. + aw * aw) / (gamma0 * gamma0));
@@ -934,6 +936,18 @@ int g4gpu_get_field(g4gpu_handle h, int ifld, double *field, int *first, double 
   return check_device_flag(h);
 }
 
+// Threads a block of the push: as set (g4gpu_set_launch_shapes, g4gpu_autotune), else by
+// the window. The FP64 push holds a scheduler for ~400 x 64 cycles a warp, so a window of
+// few particles takes small blocks that spread over the SMs (64 against 256 threads:
+// 1 x 8192 particles 26 / 40 us, 22 x 2052 49 / 71, 4 x 8192 41 / 43; 64 x 4096 235 / 231).
+// The mixed push is bound by memory and issue: 128 (700 x 8192 94.7 us, 256 threads 97.1,
+// 512 104.6, 32 115).
+static int push_threads(g4gpu_handle h) {
+  if (h->push_block > 0) return h->push_block;
+  if (h->mixed) return 128;
+  return (long long)h->cfg.nslice * h->cfg.npart < 512 * 152 ? 64 : 256;
+}
+
 // Queues the kernels and copies of steps istep0 .. istep0+nsteps-1 on the handle's
 // stream and advances the host-side ring state (first, accuslip) accordingly.
 int g4gpu_set_efield(g4gpu_handle h, double rmax, int ngrid, int nz, int nphi, int longrange) {
@@ -1168,7 +1182,7 @@ static int enqueue_coarse_step(g4gpu_handle h, int istep, int cnt) {
   const void *wake = h->wake_on ? (const void *)h->wake_lossf : nullptr;
   {
     Timed t(h, G4GPU_K_PUSH);
-    g4::launch_push_mixed_sc(L, scf, h->beam, h->field, nullptr, ns, np, ng, 0, h->push_block, 0, nullptr, nullptr,
+    g4::launch_push_mixed_sc(L, scf, h->beam, h->field, nullptr, ns, np, ng, 0, push_threads(h), 0, nullptr, nullptr,
                              wake, g4::IsrStream{});
   }
   // the sources of the c periods, each followed by its slippage
@@ -1247,10 +1261,10 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       if (!h->sc_on) {
         Timed t(h, G4GPU_K_PUSH);
         if (h->mixed)
-          g4::launch_push_mixed_sc(L, scf_push, h->beam, h->field, src, ns, np, ng, deposit, h->push_block, 0,
+          g4::launch_push_mixed_sc(L, scf_push, h->beam, h->field, src, ns, np, ng, deposit, push_threads(h), 0,
                                    nullptr, nullptr, wake, isr);
         else
-          g4::launch_push_plain_sc(L, sc, h->beam, h->field, src, ns, np, ng, deposit, h->push_block, 0,
+          g4::launch_push_plain_sc(L, sc, h->beam, h->field, src, ns, np, ng, deposit, push_threads(h), 0,
                                    nullptr, nullptr, wake, isr);
         if (isr.ctr) g4::launch_isr_advance(h->stream, h->isr_ctr);
         return G4GPU_OK;
@@ -1290,10 +1304,10 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       }
       Timed t(h, G4GPU_K_PUSH);
       if (h->mixed)
-        g4::launch_push_mixed_sc(L, scf_push, h->beam, h->field, src, ns, np, ng, deposit, h->push_block, 2, ez,
+        g4::launch_push_mixed_sc(L, scf_push, h->beam, h->field, src, ns, np, ng, deposit, push_threads(h), 2, ez,
                                  eloss, wake, isr);
       else
-        g4::launch_push_plain_sc(L, sc, h->beam, h->field, src, ns, np, ng, deposit, h->push_block, 2, ez,
+        g4::launch_push_plain_sc(L, sc, h->beam, h->field, src, ns, np, ng, deposit, push_threads(h), 2, ez,
                                  eloss, wake, isr);
       if (isr.ctr) g4::launch_isr_advance(h->stream, h->isr_ctr);
       return G4GPU_OK;

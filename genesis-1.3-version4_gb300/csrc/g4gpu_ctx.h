@@ -97,8 +97,9 @@ struct g4gpu_ctx {
   bool beam_loaded = false;
   bool field_loaded[G4GPU_MAX_FIELDS] = {};
 
-  // launch shapes (chosen by g4gpu_autotune, defaults otherwise)
-  int push_block = 256;
+  // launch shapes (chosen by g4gpu_autotune, defaults otherwise; push_block 0: by the
+  // window's size)
+  int push_block = 0;
   int field_threads = 512;
   // mixed ADI with the slice in shared memory: 0 one CTA per slice (k_field_fused_f),
   // 1 a cluster pair (k_field_band_f<2>), 2 the whole step per CTA (k_step_fused_f)
