@@ -548,6 +548,8 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
     s.half_delz = s.delz * 0.5;
     s.aw_t2 = s.aw_t * s.aw_t;
     s.aw2 = s.aw * s.aw;
+    s.one_aw_t2 = 1. + s.aw_t2;
+    s.centred = s.ax == 0 && s.ay == 0 && s.gradx == 0 && s.grady == 0;
     s.qdx2 = s.qx * s.half_delz * s.half_delz;
     s.qdy2 = s.qy * s.half_delz * s.half_delz;
     {

@@ -66,8 +66,9 @@ struct StepConst {
   double ztemp1;      // -2 / xks (BeamSolver.cpp:147), the same value the ODE computes
   // exact products of the step's constants the FP64 push would otherwise form per
   // particle: delz / 2, aw_t^2, aw^2 (each the same IEEE product on the host), and qx and
-  // qy times (delz / 2)^2
-  double half_delz, aw_t2, aw2, qdx2, qdy2;
+  // qy times (delz / 2)^2, 1 + aw_t^2
+  double half_delz, aw_t2, aw2, qdx2, qdy2, one_aw_t2;
+  int centred;  // ax, ay, gradx and grady all zero: faw without them is the same value
   // nominal phase advance over half a step and over the step: delz / 2 and delz times
   // dtheta/dz of a particle at gammaref on axis without field (BeamSolver.cpp:144-163)
   double dnom_half, dnom_full;

@@ -92,9 +92,20 @@ __device__ __forceinline__ void plane_step(int kind, double q, double qd2, doubl
   p = fma(-a2 * q, xtmp, a1 * p);  // a3 gammaz = -a2 foc^2 gammaz = -a2 q
 }
 
+// 1 / gammaz of TrackBeam::track (gammaz^2 = gamma^2 - 1 - aw^2 - px^2 - py^2) given itg =
+// 1 / gamma: with h = (1 + aw^2 + px^2 + py^2) / gamma^2, itg (1 - h)^(-1/2) by its series,
+// 1 + h/2 + 3h^2/8, for h below 2^-18 (the next term is below 2^-55; h is 3e-8 at 5.8 GeV);
+// else one reciprocal square root. Both are within an ulp or two of the reference's sqrt
+// and quotients.
+__device__ __forceinline__ double inv_gammaz(const StepConst &sc, double g, double itg, double px, double py) {
+  const double h = fma(py, py, fma(px, px, sc.one_aw_t2)) * (itg * itg);
+  if (below_pow2(h, 1023 - 18)) return itg * fma(h, fma(h, 0.375, 0.5), 1.);
+  return rsqrt(fma(-py, py, fma(-px, px, fma(g, g, -1.) - sc.aw_t2)));
+}
+
 // TrackBeam::track over half a step (TrackBeam.cpp:66-76); `last` applies the
-// corrector kick first (TrackBeam.cpp:37-38, 118-128).
-__device__ __forceinline__ void transverse(const StepConst &sc, bool last, double g, double &x,
+// corrector kick first (TrackBeam.cpp:37-38, 118-128). itg: 1 / g.
+__device__ __forceinline__ void transverse(const StepConst &sc, bool last, double g, double itg, double &x,
                                            double &y, double &px, double &py) {
   if (last && sc.corr) {
     px += sc.cxk;
@@ -111,10 +122,7 @@ __device__ __forceinline__ void transverse(const StepConst &sc, bool last, doubl
     py = sc.cm[6] * tmp * gz + sc.cm[7] * py;
   }
   const double delz = sc.half_delz;
-  // 1 / gammaz by one reciprocal square root, within an ulp or two of the reference's sqrt
-  // and quotients
-  const double gz2 = fma(-py, py, fma(-px, px, fma(g, g, -1.) - sc.aw_t2));
-  const double igz = rsqrt(gz2);
+  const double igz = inv_gammaz(sc, g, itg, px, py);
   plane_step(sc.kindx, sc.qx, sc.qdx2, sc.xoff, delz, x, px, igz);
   plane_step(sc.kindy, sc.qy, sc.qdy2, sc.yoff, delz, y, py, igz);
 }
@@ -180,16 +188,13 @@ __device__ __forceinline__ bool ll_gridpoint(double gm, double idg, double gmi, 
   return false;
 }
 
-// 1 / x given r, the reciprocal of a nearby value: two Newton steps, each squaring
-// the relative error e = 1 - x r, when |e| < 2^-17 (then the error is below 1e-20
-// before rounding), else the division. The RK4 stages of a step change gamma by far
-// less than that, so each stage's 1 / gamma follows from the previous one.
+// 1 / x given r, the reciprocal of a nearby value: for e = 1 - x r below 2^-18, r (1 + e +
+// e^2) (the omitted e^3 is below 2^-54), else the division. The RK4 stages of a step change
+// gamma by far less than that, so each stage's 1 / gamma follows from the previous one.
 __device__ __forceinline__ double recip_near(double x, double r) {
-  double e = fma(-x, r, 1.);
-  if (!below_pow2(e, 1023 - 17)) return 1. / x;
-  r = fma(r, e, r);
-  e = fma(-x, r, 1.);
-  return fma(r, e, r);
+  const double e = fma(-x, r, 1.);
+  if (!below_pow2(e, 1023 - 18)) return 1. / x;
+  return fma(r, fma(e, e, e), r);
 }
 
 // 1 / sqrt(a) as the correctly rounded quotient of 1 by the correctly rounded square
@@ -225,30 +230,56 @@ __device__ __forceinline__ double recip_sqrt_near1(double a) {
   return q;
 }
 
-// BeamSolver::ODE (BeamSolver.cpp:144-163) for NF fields, given cs[i] = (cos, sin) of
-// rharm_i * tthet and itg = 1 / tgam. Two of the reference's four divisions become
+// The same on the integer pipe, which the push leaves idle while a warp's FP64 instruction
+// holds its scheduler for 64 cycles: ib = 1 / btpar0 and om = 1 - ib (exact), for a = 1 - M
+// 2^-53 with 0 < M < 2^31 (a 5.8 GeV beam has M of 3e8; others take recip_sqrt_near1).
+//   sqrt(a) = 1 - S 2^-53:  S = M/2 + M^2 2^-56 + M^3 2^-110, to the nearest integer;
+//   1 / sqrt = 1 + Q 2^-52: Q = S/2 + S^2 2^-54 + S^3 2^-107, to the nearest integer;
+// the terms left out are below 2^-44 of a unit, and neither value is ever halfway between
+// two doubles. Equal to 1. / sqrt(a) on 3e8 random M and the first 5e6. About 45 integer
+// instructions for 12 FP64 ones, four times a particle.
+__device__ __forceinline__ void recip_sqrt_1m(double a, double &ib, double &om) {
+  constexpr long long kOne = 0x3FF0000000000000LL;
+  const long long m = kOne - __double_as_longlong(a);
+  if ((unsigned long long)(m - 1) >= 0x7fffffffULL) {
+    ib = recip_sqrt_near1(a);
+    om = 1. - ib;
+    return;
+  }
+  const unsigned M = (unsigned)m;
+  const unsigned long long M2 = (unsigned long long)M * M;
+  const unsigned long long M3 = ((unsigned long long)(unsigned)(M2 >> 31) * M) >> 23;  // M^3 2^-54
+  const unsigned long long t = ((unsigned long long)(M & 1u) << 55) + M2 + M3 + (1ULL << 55);
+  const unsigned S = (M >> 1) + (unsigned)(t >> 56);
+  const unsigned long long S2 = (unsigned long long)S * S;
+  const unsigned long long S3 = ((unsigned long long)(unsigned)(S2 >> 30) * S) >> 23;  // S^3 2^-53
+  const unsigned long long t2 = ((unsigned long long)(S & 1u) << 53) + S2 + S3 + (1ULL << 53);
+  const unsigned Q = (S >> 1) + (unsigned)(t2 >> 54);
+  ib = __longlong_as_double(kOne + Q);
+  // -Q 2^-52, Q in [1, 2^30): its leading one at bit 31 - lz
+  const int lz = __clz((int)Q);
+  const unsigned long long mant = ((unsigned long long)Q << (21 + lz)) & 0xfffffffffffffULL;
+  om = __longlong_as_double((long long)(0x8000000000000000ULL | ((unsigned long long)(1023 - 52 + 31 - lz) << 52) | mant));
+}
+
+// BeamSolver::ODE (BeamSolver.cpp:144-163), given ctmp = sum over the fields of rpart
+// e^{-i rharm tthet} and itg = 1 / tgam. Two of the reference's four divisions become
 // products with the reciprocals 1 / tgam and 1 / btpar0 (the latter rounded as the
-// reference's sqrt and quotient round it, by recip_sqrt_near1, so that xks (1 - 1/btpar0),
-// which xks ~ 1e11 amplifies, is the reference's value; a last-bit change of 1 / tgam changes btper0 / tgam^2 ~ 1e-8
-// far below the last bit of btpar0); ztemp1 = -2 / xks comes with the step constants.
+// reference's sqrt and quotient round it, so that xks (1 - 1/btpar0), which xks ~ 1e11
+// amplifies, is the reference's value; a last-bit change of 1 / tgam changes btper0 /
+// tgam^2 ~ 1e-8 far below the last bit of btpar0); ztemp1 = -2 / xks comes with the step
+// constants.
 // ACC: how the stage's derivative f enters the RK4 accumulators k2: 0 k2 = f (the first
 // two stages, where the reference adds f to zero), 1 k2 = -k2 / 2 + f and 2 k2 = 2 k2 + f
 // (the third and fourth, where the reference scales k2 by -0.5 or 2 first): each one
 // fma, exact as the reference's product (a scaling by a power of two) and rounded sum.
-template <int NF, int ACC>
-__device__ __forceinline__ void ode(const StepConst &sc, const C2 *rpart, const C2 *cs, double btpar, double ez,
-                                    double itg, double &k2gg, double &k2pp) {
-  // sum of rpart_i conj(cs_i), products fused into the sums
-  C2 ctmp = {fma(rpart[0].x, cs[0].x, rpart[0].y * cs[0].y), fma(rpart[0].y, cs[0].x, -rpart[0].x * cs[0].y)};
-#pragma unroll
-  for (int i = 1; i < NF; i++) {
-    if (i >= sc.nfld) break;
-    ctmp.x = fma(rpart[i].x, cs[i].x, fma(rpart[i].y, cs[i].y, ctmp.x));
-    ctmp.y = fma(rpart[i].y, cs[i].x, fma(-rpart[i].x, cs[i].y, ctmp.y));
-  }
-  double btper0 = fma(sc.ztemp1, ctmp.x, btpar);
-  const double ib = recip_sqrt_near1(fma(-btper0, itg * itg, 1.));
-  const double fpp = fma(sc.xks, 1. - ib, sc.xku), fgg = fma(ctmp.y * ib, itg, -ez);
+template <int ACC>
+__device__ __forceinline__ void ode(const StepConst &sc, C2 ctmp, double btpar, double ez, double itg, double &k2gg,
+                                    double &k2pp) {
+  const double btper0 = fma(sc.ztemp1, ctmp.x, btpar);
+  double ib, om;
+  recip_sqrt_1m(fma(-btper0, itg * itg, 1.), ib, om);
+  const double fpp = fma(sc.xks, om, sc.xku), fgg = fma(ctmp.y * ib, itg, -ez);
   if (ACC == 0) {
     k2pp = fpp;
     k2gg = fgg;
@@ -280,47 +311,43 @@ __device__ __forceinline__ C2 expi_small(double e) {
 }
 // The same for |eps| < 1/16, the usual case (the remainder is the phase slip of the
 // particle's energy and angle offsets over a stage, ~1e-2 rad at 3 sigma of the
-// benchmark beam): the first omitted terms, eps^10 / 10! and eps^11 / 11!, are below
-// 2.6e-19. Ten FP64 instructions instead of thirteen.
+// benchmark beam), on the integer pipe: z = eps^2 and the series
+//   1 - cos = z/2 - z^2/24 + z^3/720 - z^4/40320,   1 - sin/eps = z/6 - z^2/120 + z^3/5040
+//   - z^4/362880
+// in fixed point (2^-64 units, the two highest terms in 32 bits), each within 2^-58, the
+// first omitted terms below 2^-61; both are then subtracted from 1 in the bit pattern,
+// rounded to its 2^-53 spacing. One FP64 instruction (the product with eps) instead of ten.
 __device__ __forceinline__ C2 expi_tiny(double e) {
-  const double z = e * e;
-  double c = fma(z, 1. / 40320., -1. / 720.);
-  c = fma(z, c, 1. / 24.);
-  c = fma(z, c, -0.5);
-  c = fma(z, c, 1.);
-  double sn = fma(z, 1. / 362880., -1. / 5040.);
-  sn = fma(z, sn, 1. / 120.);
-  sn = fma(z, sn, -1. / 6.);
-  sn = fma(z, sn, 1.);
-  return {c, sn * e};
+  constexpr long long kOne = 0x3FF0000000000000LL;
+  constexpr unsigned long long kMant = (1ULL << 52) - 1;
+  const unsigned long long b = (unsigned long long)(__double_as_longlong(e) & 0x7fffffffffffffffLL);
+  const int sh = (int)(b >> 52) - 1011;  // |e| 2^64 = significand 2^sh; sh <= 7
+  const unsigned long long m = (b & kMant) | (1ULL << 52);
+  const unsigned long long ef = sh >= 0 ? m << sh : (sh > -64 ? m >> -sh : 0ULL);
+  const unsigned long long z = __umul64hi(ef, ef);  // z 2^64 < 2^56
+  const unsigned zh = (unsigned)(z >> 24);          // z 2^40
+  // 2^41 (1/720 - z/40320), 2^44 (1/5040 - z/362880)
+  const unsigned c3 = 3054198966u - __umulhi(zh, 213044u), s3 = 3490513104u - __umulhi(zh, 189372u);
+  const unsigned long long c2 = 768614336404564650ULL - (((unsigned long long)zh * c3) >> 17);  // 2^64 / 24 - ..
+  const unsigned long long s2 = 153722867280912930ULL - (((unsigned long long)zh * s3) >> 20);  // 2^64 / 120 - ..
+  const unsigned long long oc = (z >> 1) - __umul64hi(z, __umul64hi(z, c2));
+  const unsigned long long os = __umul64hi(z, 3074457345618258602ULL - __umul64hi(z, s2));     // 2^64 / 6
+  const double c = __longlong_as_double(kOne - (long long)((oc + 1024) >> 11));
+  const double f = __longlong_as_double(kOne - (long long)((os + 1024) >> 11));
+  return {c, f * e};
 }
 
-// (cos, sin) of h theta for a phase theta = theta0 + dth near theta0 + dnom: the
-// particle's e^{i h theta0} rotated by e^{i h dnom} (brot: their product, formed once
-// per particle and harmonic) and by e^{i h (dth - dnom)}; sincos of h theta where the
-// remainder is not small.
-__device__ __forceinline__ C2 rotated(C2 brot, double h, double theta, double dth, double dnom) {
-  const double e = h * (dth - dnom);
-  if (below_pow2(e, 1023 - 4)) return cmul_fma(brot, expi_tiny(e));
-  if (below_pow2(e, 1023 - 2)) return cmul_fma(brot, expi_small(e));
+// e^{i e} for the remainder e of a rotation
+__device__ __forceinline__ C2 expi(double e) {
+  if (below_pow2(e, 1023 - 4)) return expi_tiny(e);
+  if (below_pow2(e, 1023 - 2)) return expi_small(e);
   double sn, c;
-  sincos(h * theta, &sn, &c);
+  sincos(e, &sn, &c);
   return {c, sn};
 }
-
-// cs = e^{i h theta_p} rotated on to e^{i h theta} for a phase theta a small step dth =
-// theta - theta_p past theta_p (RK4 stage 3 after stage 2, the deposition after stage 4:
-// the stages' phase velocities differ by a few parts in 1e5 of a radian per step): for
-// d = h dth below 2^-12, (1 - z/2 + z^2/24, d - d z/6) with z = d^2 (the first omitted terms
-// are below 2^-72 / 720 and 2^-60 / 120); else `rotated` from the step's start.
-__device__ __forceinline__ C2 rotated_on(C2 cs, double dth, C2 brot, double h, double theta, double theta0,
-                                         double dnom) {
-  const double d = h * dth;
-  if (below_pow2(d, 1023 - 12)) {
-    const double z = d * d;
-    return cmul_fma(cs, C2{fma(z, fma(z, 1. / 24., -0.5), 1.), fma(d * z, -1. / 6., d)});
-  }
-  return rotated(brot, h, theta, theta - theta0, dnom);
+// a conj(b)
+__device__ __forceinline__ C2 cmul_conj(C2 a, C2 b) {
+  return {fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y)};
 }
 
 // sqrt(1 + d): for |d| < 2^-10 its Taylor series to d^5 (the next term, 21/1024 d^6, is
@@ -358,8 +385,13 @@ __device__ __forceinline__ void deposit_particle(const StepConst &sc, double2 *c
     Cell c;
     if (!ll_gridpoint(fs.gridmax, fs.idgrid, fs.gm_idg, ng, x, y, c)) continue;
     const double scl = scls ? scls[k] : deposit_scale(sc, fs, cur, npd);
-    double dx = x - sc.ax, dy = y - sc.ay;
-    const double dfaw2 = fma(2., fma(sc.grady, dy, sc.gradx * dx), fma(sc.ky * dy, dy, sc.kx * dx * dx));
+    double dfaw2;
+    if (sc.centred) {
+      dfaw2 = fma(sc.ky * y, y, sc.kx * x * x);
+    } else {
+      const double dx = x - sc.ax, dy = y - sc.ay;
+      dfaw2 = fma(2., fma(sc.grady, dy, sc.gradx * dx), fma(sc.ky * dy, dy, sc.kx * dx * dx));
+    }
     const double faw = sqrt_1p(dfaw2);
     double part = ig != 0. ? faw * scl * ig : faw * scl / g;
     double s, co;
@@ -434,7 +466,8 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
   double g = p.gamma[o], th = p.theta[o], x = p.x[o], y = p.y[o], px = p.px[o], py = p.py[o];
   size_t ncell = (size_t)ng * ng;
 
-  if (p.mode != 2) transverse(sc, false, g, x, y, px, py);
+  double itg = 1. / g;  // 1 / gamma, of each RK4 stage from the previous one's
+  if (p.mode != 2) transverse(sc, false, g, itg, x, y, px, py);
   if (p.mode == 1) {
     p.x[o] = x;
     p.y[o] = y;
@@ -446,11 +479,23 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
   const double ez = (p.ez ? p.ez[o] : 0.) + (p.eloss ? p.eloss[is] : 0.);
 
   // BeamSolver::advance, BeamSolver.cpp:53-80
-  double gamma = g, theta = th + sc.autophase;
-  double dx = x - sc.ax, dy = y - sc.ay;
-  const double awloc = fma(sc.grady, dy, fma(sc.gradx, dx, fma(0.5, fma(sc.ky * dy, dy, sc.kx * dx * dx), 1.)));
+  double gamma = g;
+  const double theta0 = sc.autophase != 0. ? th + sc.autophase : th;
+  double awloc;
+  if (sc.centred) {
+    awloc = fma(0.5, fma(sc.ky * y, y, sc.kx * x * x), 1.);
+  } else {
+    const double dx = x - sc.ax, dy = y - sc.ay;
+    awloc = fma(sc.grady, dy, fma(sc.gradx, dx, fma(0.5, fma(sc.ky * dy, dy, sc.kx * dx * dx), 1.)));
+  }
   const double btpar = fma(sc.aw2 * awloc, awloc, fma(py, py, fma(px, px, 1.)));
-  C2 rpart[NF];
+  // Each field's drive rpart e^{-i h theta} at the start of the step (cs: e^{i h theta}, the
+  // phasor the last push left, turned by the step's phase offset, or a sincos), and turned
+  // by the step's nominal phase advance over half a step and over the step: a stage then
+  // multiplies by e^{-i e}, e = h (its phase advance - the nominal one), one complex product
+  // instead of a rotated phasor's and the drive's.
+  const bool cached = p.phasor && *p.phasor_ok;
+  C2 c0 = {0, 0}, chalf[NF], cfull[NF], bfull[NF];
 #pragma unroll
   for (int k = 0; k < NF; k++) {
     if (k >= sc.nfld) break;
@@ -458,82 +503,78 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
     int islice = (is + fs.first) % ns;
     const double2 *f = p.field[k] + (size_t)islice * ncell;
     Cell c;
+    C2 drive = {0, 0};
     if (ll_gridpoint(fs.gridmax, fs.idgrid, fs.gm_idg, ng, x, y, c)) {
-      // bilinear weights formed once, the four terms fused into their sum
-      const double w00 = c.wx * c.wy, w10 = c.ux * c.wy, w01 = c.wx * c.uy, w11 = c.ux * c.uy;
+      // bilinear: along x on both rows, then along y
       const C2 f00 = ld(f + c.i00), f10 = ld(f + c.i10), f01 = ld(f + c.i01), f11 = ld(f + c.i11);
-      C2 cpart;
-      cpart.x = fma(f11.x, w11, fma(f01.x, w01, fma(f10.x, w10, f00.x * w00)));
-      cpart.y = fma(f11.y, w11, fma(f01.y, w01, fma(f10.y, w10, f00.y * w00)));
-      rpart[k] = rmul(fs.rtmp * awloc, C2{cpart.x, -cpart.y});
-    } else {
-      rpart[k] = C2{0, 0};
+      const C2 lo = {fma(c.ux, f10.x - f00.x, f00.x), fma(c.ux, f10.y - f00.y, f00.y)};
+      const C2 hi = {fma(c.ux, f11.x - f01.x, f01.x), fma(c.ux, f11.y - f01.y, f01.y)};
+      drive = rmul(fs.rtmp * awloc, C2{fma(c.uy, hi.x - lo.x, lo.x), -fma(c.uy, hi.y - lo.y, lo.y)});
     }
-  }
-
-  // e^{i h theta} of every field at the start, and rotated towards the stages: one
-  // sincos per harmonic and particle instead of one per stage, or none where the last
-  // push left it (the phasor of the stored phase, turned by the step's phase offset)
-  const double theta0 = theta;
-  const bool cached = p.phasor && *p.phasor_ok;
-  C2 bhalf[NF], bfull[NF], cs[NF];
-#pragma unroll
-  for (int k = 0; k < NF; k++) {
-    if (k >= sc.nfld) break;
+    C2 cs;
     if (cached) {
-      const C2 c = ld(p.phasor + k * p.pstride + o);
-      cs[k] = sc.autophase != 0. ? cmul_fma(c, C2{sc.f[k].rot_auto[0], sc.f[k].rot_auto[1]}) : c;
+      cs = ld(p.phasor + k * p.pstride + o);
+      if (sc.autophase != 0.) cs = cmul_fma(cs, C2{fs.rot_auto[0], fs.rot_auto[1]});
     } else {
-      double sn, c;
-      sincos(sc.f[k].rharm * theta0, &sn, &c);
-      cs[k] = C2{c, sn};
+      double sn, co;
+      sincos(fs.rharm * theta0, &sn, &co);
+      cs = C2{co, sn};
     }
-    bhalf[k] = cmul_fma(cs[k], C2{sc.f[k].rot_half[0], sc.f[k].rot_half[1]});
-    bfull[k] = cmul_fma(cs[k], C2{sc.f[k].rot_full[0], sc.f[k].rot_full[1]});
+    drive = cmul_conj(drive, cs);
+    c0 = k == 0 ? drive : cadd(c0, drive);
+    chalf[k] = cmul_conj(drive, C2{fs.rot_half[0], fs.rot_half[1]});
+    cfull[k] = cmul_conj(drive, C2{fs.rot_full[0], fs.rot_full[1]});
+    bfull[k] = cmul_fma(cs, C2{fs.rot_full[0], fs.rot_full[1]});
   }
-  auto stage = [&](const C2 *b, double dnom) {
+  // sum over the fields of their nominal drives turned by the remainder of the advance dth
+  auto drive_at = [&](const C2 *cn, double dth, double dnom) {
+    const double d = dth - dnom;
+    C2 sum = {0, 0};
 #pragma unroll
     for (int k = 0; k < NF; k++) {
       if (k >= sc.nfld) break;
-      cs[k] = rotated(b[k], sc.f[k].rharm, theta, theta - theta0, dnom);
+      const C2 v = cmul_conj(cn[k], expi(sc.f[k].rharm == 1. ? d : sc.f[k].rharm * d));
+      sum = k == 0 ? v : cadd(sum, v);
     }
+    return sum;
   };
 
-  // BeamSolver::RungeKutta, BeamSolver.cpp:89-141
+  // BeamSolver::RungeKutta, BeamSolver.cpp:89-141, the phase as its advance dth from theta0
   double k2gg, k2pp, k3gg, k3pp;
-  double itg = 1. / gamma;  // 1 / gamma of the stage, each stage's from the previous one
-  ode<NF, 0>(sc, rpart, cs, btpar, ez, itg, k2gg, k2pp);
+  ode<0>(sc, c0, btpar, ez, itg, k2gg, k2pp);
   double stpz = sc.half_delz;
   gamma = fma(stpz, k2gg, gamma);
-  theta = fma(stpz, k2pp, theta);
+  double dth = stpz * k2pp;
   k3gg = k2gg;
   k3pp = k2pp;
-  stage(bhalf, sc.dnom_half);
   itg = recip_near(gamma, itg);
-  ode<NF, 0>(sc, rpart, cs, btpar, ez, itg, k2gg, k2pp);
+  ode<0>(sc, drive_at(chalf, dth, sc.dnom_half), btpar, ez, itg, k2gg, k2pp);
   gamma = fma(stpz, k2gg - k3gg, gamma);
-  const double theta1 = theta;
-  theta = fma(stpz, k2pp - k3pp, theta);
+  dth = fma(stpz, k2pp - k3pp, dth);
   k3gg *= kSixth;
   k3pp *= kSixth;
-#pragma unroll
-  for (int k = 0; k < NF; k++) {
-    if (k >= sc.nfld) break;
-    cs[k] = rotated_on(cs[k], theta - theta1, bhalf[k], sc.f[k].rharm, theta, theta0, sc.dnom_half);
-  }
   itg = recip_near(gamma, itg);
-  ode<NF, 1>(sc, rpart, cs, btpar, ez, itg, k2gg, k2pp);  // k2 = -k2 / 2 + f
+  ode<1>(sc, drive_at(chalf, dth, sc.dnom_half), btpar, ez, itg, k2gg, k2pp);  // k2 = -k2 / 2 + f
   stpz = sc.delz;
   gamma = fma(stpz, k2gg, gamma);
-  theta = fma(stpz, k2pp, theta);
+  dth = fma(stpz, k2pp, dth);
   k3gg -= k2gg;
   k3pp -= k2pp;
-  stage(bfull, sc.dnom_full);
   itg = recip_near(gamma, itg);
-  ode<NF, 2>(sc, rpart, cs, btpar, ez, itg, k2gg, k2pp);  // k2 = 2 k2 + f
-  const double theta3 = theta;
+  ode<2>(sc, drive_at(cfull, dth, sc.dnom_full), btpar, ez, itg, k2gg, k2pp);  // k2 = 2 k2 + f
   gamma = fma(stpz, fma(k2gg, kSixth, k3gg), gamma);
-  theta = fma(stpz, fma(k2pp, kSixth, k3pp), theta);
+  dth = fma(stpz, fma(k2pp, kSixth, k3pp), dth);
+  double theta = theta0 + dth;
+  // the deposition's phasors, kept for the next push
+  C2 cs[NF];
+  if (deposit || p.phasor) {
+#pragma unroll
+    for (int k = 0; k < NF; k++) {
+      if (k >= sc.nfld) break;
+      const double d = dth - sc.dnom_full;
+      cs[k] = cmul_fma(bfull[k], expi(sc.f[k].rharm == 1. ? d : sc.f[k].rharm * d));
+    }
+  }
 
   // Incoherent::apply (Incoherent.cpp:66-77): one draw per beamlet of nbins particles
   if (p.isr.ctr) {
@@ -543,9 +584,22 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
   // Collective::apply (Collective.cpp:119-128), before the second half step
   if (p.wake) gamma += p.wake[is] * sc.delz / kEev;
   // TrackBeam::applyR56 (TrackBeam.cpp:260-277)
-  if (sc.chic) theta += sc.r56 * (gamma - sc.gammaref);
+  if (sc.chic) {
+    const double r = sc.r56 * (gamma - sc.gammaref);
+    theta += r;
+    if (deposit || p.phasor) {
+#pragma unroll
+      for (int k = 0; k < NF; k++) {
+        if (k >= sc.nfld) break;
+        double sn, co;
+        sincos(sc.f[k].rharm * r, &sn, &co);
+        cs[k] = cmul_fma(cs[k], C2{co, sn});
+      }
+    }
+  }
 
-  transverse(sc, true, gamma, x, y, px, py);
+  itg = recip_near(gamma, itg);
+  transverse(sc, true, gamma, itg, x, y, px, py);
 
   p.gamma[o] = gamma;
   p.theta[o] = theta;
@@ -553,19 +607,16 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
   p.y[o] = y;
   p.px[o] = px;
   p.py[o] = py;
-
-  if (deposit || p.phasor) {
-    // the deposition's phases, rotated on from stage 4's, kept for the next push
+  if (p.phasor) {
 #pragma unroll
     for (int k = 0; k < NF; k++) {
       if (k >= sc.nfld) break;
-      cs[k] = rotated_on(cs[k], theta - theta3, bfull[k], sc.f[k].rharm, theta, theta0, sc.dnom_full);
-      if (p.phasor) st(p.phasor + k * p.pstride + o, cs[k]);
+      st(p.phasor + k * p.pstride + o, cs[k]);
     }
   }
   if (deposit) {
     deposit_particle<NF>(sc, p.src, (size_t)is * ncell, ng, p.current[is], (double)n, gamma,
-                         theta, x, y, cs, scls, recip_near(gamma, itg));
+                         theta, x, y, cs, scls, itg);
   }
 }
 
@@ -705,7 +756,7 @@ struct PlainSC {
   static __device__ __forceinline__ double gamma(const StepConst &, double g) { return g; }
   static __device__ __forceinline__ void half(const StepConst &s, double g, double &x, double &y, double &px,
                                               double &py) {
-    transverse(s, false, g, x, y, px, py);
+    transverse(s, false, g, 1. / g, x, y, px, py);
   }
   static __device__ __forceinline__ double2 eil(double th, int l) {
     double s, c;
