@@ -68,27 +68,19 @@ __device__ __forceinline__ void solve_lines(const Lines &s, int nline, int lstri
   if (seg < nseg) {
     const int b = seg * ng / nseg, e = (seg + 1) * ng / nseg;
     C2 *L = s.T + (size_t)line * lstride;
+    // one loop for all segments (the tables' last entry is their constant): lanes of
+    // different segments stay together, and a warp's FP64 instruction costs the same for
+    // one lane as for 32
     C2 d = {0, 0};
-    int k = b;
-    for (; k < min(e, nco); k++) {
-      d = cmul_fma(add_imul(L[k * estride], c, d), s.cbet[k]);
-      L[k * estride] = d;
-    }
-    const C2 cb = s.cbet[nco - 1], cw = s.cwet[nco - 1];
-    for (; k < e; k++) {
-      d = cmul_fma(add_imul(L[k * estride], c, d), cb);
+    for (int k = b; k < e; k++) {
+      d = cmul_fma(add_imul(L[k * estride], c, d), s.cbet[min(k, nco - 1)]);
       L[k * estride] = d;
     }
     s.edge_d[seg * nline + line] = d;
     // x_{e-1} = d_{e-1}, what the forward sweep ended with
     C2 x = d;
-    k = e - 2;
-    for (; k >= max(b, nco); k--) {
-      x = sub_cmul(L[k * estride], cw, x);
-      L[k * estride] = x;
-    }
-    for (; k >= b; k--) {
-      x = sub_cmul(L[k * estride], s.cwet[k], x);
+    for (int k = e - 2; k >= b; k--) {
+      x = sub_cmul(L[k * estride], s.cwet[min(k, nco - 1)], x);
       L[k * estride] = x;
     }
     s.edge_x[seg * nline + line] = x;
@@ -139,7 +131,9 @@ __global__ void k_adi_rows(const double2 *__restrict__ field, double2 *__restric
     for (int r = 0; r < L; r++) {
       C2 v = {0, 0};
       if (r < nr) {
-        v = add_imul(uu[r + 1], c, lap(r0 + r > 0, r0 + r < ng - 1, uu[r], uu[r + 1], uu[r + 2]));
+        // the rows outside the grid are zeros: (next - 2 u) + prev is then the reference's
+        // one-sided difference, bit for bit
+        v = add_imul(uu[r + 1], c, cadd(sub2(uu[r + 2], uu[r + 1]), uu[r]));
         st(s + (size_t)r * ng + k, v);
       }
       T[r * st1 + k] = cadd(v, sv[r]);

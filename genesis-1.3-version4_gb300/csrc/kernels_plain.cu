@@ -906,16 +906,15 @@ struct AdiShape {
 };
 // Why these: a warp's FP64 instruction holds its scheduler for 64 cycles whatever lanes
 // are active, so the solve wants full warps, enough of them on every SM, and no more
-// segments than that takes (each adds 16 W instructions a line). Measured (both half
+// segments than that takes (each adds 8 W instructions a line). Measured (both half
 // steps, step factor 0.034, W 13; in brackets one thread per line):
-//   1 slice x 255^2     L 2, nseg 19   41 us (688)      22 x 101^2   L 4, nseg 6   53 us (292)
-//   4 x 151^2           L 2, nseg 8    45 us (428)      60 x 151^2   L 8, nseg 4  136 us (446)
-//   320 x 151^2         L 8, nseg 4   624 us (870)      320 x 255^2  L 8, nseg 8 1640 us (2350)
+//   1 slice x 255^2     L 2, nseg 19   33 us (688)      22 x 101^2   L 4, nseg 6   40 us (292)
+//   4 x 151^2           L 2, nseg 8    33 us (428)      60 x 151^2   L 8, nseg 4  111 us (446)
+//   320 x 151^2         L 8, nseg 4   510 us (870)      2000 x 101^2 L 8, nseg 4 1480 us (1925)
 // so: at four CTAs an SM of 8 lines and segments of about 36 elements, that; below, the
 // most segments and fewer lines, down to 2. Two segments of 16 lines fill a warp where
-// the warm-up leaves no more (2000 x 101^2: 1835 us, one thread per line 1925). One
-// segment is slower than one thread per line (320 x 151^2: 967 us), as are lines of which
-// two do not fit shared memory.
+// the warm-up leaves no more (2000 x 101^2: 1567 us). One segment is slower than one thread
+// per line (320 x 151^2: 967 us), as are lines of which two do not fit shared memory.
 AdiShape adi_shape(int ns, int ng, int W) {
   const int most = W > 0 ? ng / W : 1;
   if (most < 2) return {0, 0, 128};
