@@ -283,7 +283,7 @@ struct FFTPlan {
 int fft_max_ngrid(int mixed);
 // lines of a slice one CTA transforms at a time in a pass with `bufs` tile buffers
 // and `per_sm` CTAs on an SM (es: bytes of a complex element; at most maxL)
-int fft_lines_per_cta(const FFTPlan &pl, int es, int bufs, int maxL, int per_sm);
+int fft_lines_per_cta(const FFTPlan &pl, int es, int bufs, int maxL, int per_sm, size_t table = 0);
 // whether the kernels can take the plan's stages (one butterfly per thread for a
 // line of each register stage, at most 8 outputs per thread of a generic one)
 int fft_plan_fits(const FFTPlan &pl);

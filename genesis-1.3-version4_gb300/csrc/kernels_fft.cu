@@ -20,6 +20,15 @@
 // that a warp reads consecutive entries. Templated on the precision: double2 for
 // the plain form, float2 for the mixed form, whose complex arithmetic uses the
 // paired FP32 instructions (both lanes of a float2 in one instruction).
+//
+// Every transform is a forward one. The inverse is the forward transform of the data with
+// real and imaginary parts exchanged, exchanged back, and each exchange falls where the data
+// is written anyway: the column pass writes its product with the propagator exchanged and
+// leaves the columns so, and the inverse row pass exchanges what it writes last. The roots
+// are then compile-time constants with their signs (a run-time sign cost a multiplication
+// per root, difference and twiddle: FP64 instructions that hold a warp's scheduler for 64
+// cycles, a tenth of the FP32 passes' issue slots), and multiples of a quarter turn are no
+// products at all.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -48,10 +57,11 @@ __device__ __forceinline__ T2 mk(typename Real<T2>::T x, typename Real<T2>::T y)
   return r;
 }
 
-// Complex arithmetic: add, sub; axpy(c, a, y) = y + c a (c real); cm(a, w) = a w;
+// Complex arithmetic: add, sub; mul(c, a) = c a, axpy(c, a, y) = y + c a (c real); cm(a, w) = a w;
 // addi(a, b) = a + i b; subi(a, b) = a - i b.
 __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 mul(float c, float2 a) { return __fmul2_rn(make_float2(c, c), a); }
 __device__ __forceinline__ float2 axpy(float c, float2 a, float2 y) { return __ffma2_rn(make_float2(c, c), a, y); }
 __device__ __forceinline__ float2 cm(float2 a, float2 w) {
   return __ffma2_rn(make_float2(-a.y, a.y), make_float2(w.y, w.x), __fmul2_rn(make_float2(a.x, a.x), w));
@@ -65,6 +75,7 @@ __device__ __forceinline__ float2 subi(float2 a, float2 b) {
 
 __device__ __forceinline__ double2 add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 sub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 mul(double c, double2 a) { return make_double2(c * a.x, c * a.y); }
 __device__ __forceinline__ double2 axpy(double c, double2 a, double2 y) {
   return make_double2(y.x + c * a.x, y.y + c * a.y);
 }
@@ -117,11 +128,9 @@ struct Roots {
   }
 };
 
-// R-point DFT y_t = sum_q x_q w^{q t} of x[0..R), w = exp(-2 pi i / R) forward and
-// exp(+2 pi i / R) inverse (sgn = +1 forward, -1 inverse: the sine of every root
-// is scaled by sgn; the roots themselves are compile-time constants). OUT 0: y
+// R-point DFT y_t = sum_q x_q w^{q t} of x[0..R), w = exp(-2 pi i / R). OUT 0: y
 // replaces x; 1: y_t is written to dst[t ds] as it is formed; 2: likewise through
-// the epilogue (scale, + 2 src at the same offset).
+// the epilogue (exchange, scale, + 2 src at the same offset).
 // Odd prime R: with a_m = x_m + x_{R-m} and b_m = x_m - x_{R-m},
 //   y_t = A_t + i B_t,  y_{R-t} = A_t - i B_t,
 //   A_t = x_0 + sum_m a_m Re(w^{m t}),  B_t = sum_m b_m Im(w^{m t}),
@@ -156,20 +165,31 @@ __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// What the last stage of a row pass writes to global memory: scale y (+ 2 src).
-template <typename T2>
+// What the last stage of a row pass writes to global memory: y (EXCH 0, the forward
+// pass), or y with its parts exchanged, scaled, and + 2 src (EXCH 1, the inverse pass).
+template <typename T2, int EXCH>
 struct Epilogue {
   typename Real<T2>::T scale;
   const T2 *src;  // the source at the same place as the output, or null
   __device__ __forceinline__ void put(T2 *g, int off, T2 v) const {
-    v = axpy(scale, v, mk<T2>(0, 0));
-    if (src) v = axpy((typename Real<T2>::T)2, src[off], v);
+    if constexpr (EXCH == 1) {
+      v = mul(scale, mk<T2>(v.y, v.x));
+      if (src) v = axpy((typename Real<T2>::T)2, src[off], v);
+    }
     *g = v;
   }
 };
-template <int R, int OUT, typename T2>
-__device__ __forceinline__ void dft(T2 *x, T2 *dst, int ds, typename Real<T2>::T sgn,
-                                    const Epilogue<T2> &epi = Epilogue<T2>{}) {
+// a w^m for the root w = exp(-2 pi i / R): quarter turns exchange and negate
+template <int R, typename T2>
+__device__ __forceinline__ T2 turn(T2 a, int m, const Roots<R> &w) {
+  if (4 * m == R) return mk<T2>(a.y, -a.x);
+  if (2 * m == R) return mk<T2>(-a.x, -a.y);
+  if (4 * m == 3 * R) return mk<T2>(-a.y, a.x);
+  typedef typename Real<T2>::T Rt;
+  return cm(a, mk<T2>((Rt)w.c[m], (Rt)w.s[m]));
+}
+template <int R, int OUT, typename T2, int EXCH = 0>
+__device__ __forceinline__ void dft(T2 *x, T2 *dst, int ds, const Epilogue<T2, EXCH> &epi = Epilogue<T2, EXCH>{}) {
   typedef typename Real<T2>::T Rt;
   constexpr Roots<R> w{};
   if constexpr (R == 1) {
@@ -179,9 +199,8 @@ __device__ __forceinline__ void dft(T2 *x, T2 *dst, int ds, typename Real<T2>::T
     G4_PUT(0, add(a, b));
     G4_PUT(1, sub(a, b));
   } else if constexpr (R == 4) {
-    // w = -i sgn: exact
-    const T2 t0 = add(x[0], x[2]), t1 = sub(x[0], x[2]), t2 = add(x[1], x[3]);
-    const T2 t3 = axpy(sgn, sub(x[1], x[3]), mk<T2>(0, 0));
+    // w = -i: exact
+    const T2 t0 = add(x[0], x[2]), t1 = sub(x[0], x[2]), t2 = add(x[1], x[3]), t3 = sub(x[1], x[3]);
     G4_PUT(0, add(t0, t2));
     G4_PUT(2, sub(t0, t2));
     G4_PUT(1, subi(t1, t3));
@@ -194,21 +213,21 @@ __device__ __forceinline__ void dft(T2 *x, T2 *dst, int ds, typename Real<T2>::T
 #pragma unroll
       for (int i = 0; i < M; i++) part[s][i] = x[P * i + s];
 #pragma unroll
-    for (int s = 0; s < P; s++) dft<M, 0>(part[s], (T2 *)nullptr, 0, sgn);
+    for (int s = 0; s < P; s++) dft<M, 0>(part[s], (T2 *)nullptr, 0);
 #pragma unroll
     for (int k = 0; k < M; k++) {
       T2 y[P];
 #pragma unroll
       for (int s = 0; s < P; s++)
-        y[s] = (s == 0 || k == 0) ? part[s][k] : cm(part[s][k], mk<T2>((Rt)w.c[s * k], sgn * (Rt)w.s[s * k]));
+        y[s] = (s == 0 || k == 0) ? part[s][k] : turn<R>(part[s][k], s * k, w);
       if constexpr (OUT == 0) {
-        dft<P, 0>(y, (T2 *)nullptr, 0, sgn);
+        dft<P, 0>(y, (T2 *)nullptr, 0);
 #pragma unroll
         for (int t = 0; t < P; t++) x[k + t * M] = y[t];
       } else {
-        Epilogue<T2> e2 = epi;
+        Epilogue<T2, EXCH> e2 = epi;
         if (OUT == 2 && e2.src) e2.src += k * ds;
-        dft<P, OUT>(y, dst + k * ds, M * ds, sgn, e2);
+        dft<P, OUT>(y, dst + k * ds, M * ds, e2);
       }
     }
   } else {
@@ -219,15 +238,15 @@ __device__ __forceinline__ void dft(T2 *x, T2 *dst, int ds, typename Real<T2>::T
 #pragma unroll
     for (int m = 1; m <= H; m++) {
       a[m] = add(x[m], x[R - m]);
-      b[m] = axpy(sgn, sub(x[m], x[R - m]), mk<T2>(0, 0));
+      b[m] = sub(x[m], x[R - m]);
       y0 = add(y0, a[m]);
     }
     G4_PUT(0, y0);
 #pragma unroll
     for (int t = 1; t <= H; t++) {
-      T2 A = x0, B = mk<T2>(0, 0);
+      T2 A = axpy((Rt)w.c[t], a[1], x0), B = mul((Rt)w.s[t], b[1]);
 #pragma unroll
-      for (int m = 1; m <= H; m++) {
+      for (int m = 2; m <= H; m++) {
         const int id = (m * t) % R;
         A = axpy((Rt)w.c[id], a[m], A);
         B = axpy((Rt)w.s[id], b[m], B);
@@ -249,24 +268,20 @@ __device__ __forceinline__ int fdiv(int x, int d, unsigned m) {
 // synchronises, and every thread writes its outputs (stage_store). With ns the
 // product of the earlier radices and nb = n / R, butterfly j (k = j mod ns) of a
 // line reads in[j + q nb], q < R, multiplies input q by the twiddle
-// exp(-+2 pi i q k / (ns R)), takes the R-point DFT, and writes output t to
+// exp(-2 pi i q k / (ns R)), takes the R-point DFT, and writes output t to
 // out[(j - k) R + t ns + k]:
-//   out[...] = sum_q in[j + q nb] W^{q (k n/(ns R) + t n/R)},  W = exp(-+2 pi i / n).
-// The twiddles are tw[(q - 1) ns + k] (forward; conjugated when inverse). The
+//   out[...] = sum_q in[j + q nb] W^{q (k n/(ns R) + t n/R)},  W = exp(-2 pi i / n).
+// The twiddles are tw[(q - 1) ns + k]. The
 // butterfly lives in one register array of the largest radix for every stage, so
 // that the stages' code paths share the registers held across the barrier.
 constexpr int MAX_RADIX = 17;
 template <int R, typename T2>
-__device__ __forceinline__ void stage_load(T2 *x, const T2 *src, int nb, int ns, int k, const T2 *tw,
-                                           typename Real<T2>::T sgn) {
+__device__ __forceinline__ void stage_load(T2 *x, const T2 *src, int nb, int ns, int k, const T2 *tw) {
 #pragma unroll
   for (int q = 0; q < R; q++) x[q] = src[q * nb];
   if (ns > 1) {
 #pragma unroll
-    for (int q = 1; q < R; q++) {
-      const T2 w = tw[(q - 1) * ns + k];
-      x[q] = cm(x[q], mk<T2>(w.x, sgn * w.y));
-    }
+    for (int q = 1; q < R; q++) x[q] = cm(x[q], tw[(q - 1) * ns + k]);
   }
 }
 
@@ -277,7 +292,7 @@ __device__ __forceinline__ void stage_load(T2 *x, const T2 *src, int nb, int ns,
 constexpr int STAGE_ANY_OUT = 8;
 template <typename T2>
 __device__ __forceinline__ void any_load(T2 *acc, const T2 *A, int ls, int lines, int n, int ns, int r,
-                                         const T2 *W, bool inverse) {
+                                         const T2 *W) {
   const int nb = n / r, nsr = ns * r;
 #pragma unroll
   for (int u = 0; u < STAGE_ANY_OUT; u++) {
@@ -293,17 +308,15 @@ __device__ __forceinline__ void any_load(T2 *acc, const T2 *A, int ls, int lines
       for (int q = 1; q < r; q++) {
         m += e;
         if (m >= n) m -= n;
-        T2 w = W[m];
-        if (inverse) w.y = -w.y;
-        v = add(v, cm(src[q * nb], w));
+        v = add(v, cm(src[q * nb], W[m]));
       }
       acc[u] = v;
     }
   }
 }
-template <typename T2>
+template <typename T2, int EXCH>
 __device__ __forceinline__ void any_store(const T2 *acc, T2 *A, int ls, int lines, int n, T2 *gout,
-                                          const Epilogue<T2> &epi) {
+                                          const Epilogue<T2, EXCH> &epi) {
 #pragma unroll
   for (int u = 0; u < STAGE_ANY_OUT; u++) {
     const int t = threadIdx.x + u * blockDim.x;
@@ -324,16 +337,13 @@ __host__ __device__ constexpr bool register_radix(int r) {
 }
 
 // One 1-D Stockham FFT of length n, in place over `lines` lines of A stored with
-// line stride `ls`, the stages of the plan's radices in turn, forward or inverse
-// (the direction is a run-time argument, so that a kernel with several transforms
-// holds one copy of the code). W: the n roots exp(-2 pi i m / n), followed by the
+// line stride `ls`, the stages of the plan's radices in turn. W: the n roots exp(-2 pi i m / n), followed by the
 // stage twiddle table (stage s's at W + n + plan.tw_off[s]).
-template <typename T2>
-__device__ __forceinline__ void fft_lines(T2 *A, int ls, int lines, const FFTPlan &pl, const T2 *W, bool inverse,
-                                          T2 *gout = nullptr, const Epilogue<T2> &epi = Epilogue<T2>{},
+template <typename T2, int EXCH = 0>
+__device__ __forceinline__ void fft_lines(T2 *A, int ls, int lines, const FFTPlan &pl, const T2 *W,
+                                          T2 *gout = nullptr,
+                                          const Epilogue<T2, EXCH> &epi = Epilogue<T2, EXCH>{},
                                           bool wait_epi_copy = false) {
-  typedef typename Real<T2>::T Rt;
-  const Rt sgn = inverse ? (Rt)-1 : (Rt)1;
   int ns = 1;
   for (int s = 0; s < pl.nstage; s++) {
     // the last stage of a pass with a global output writes it there (line stride ls)
@@ -349,12 +359,12 @@ __device__ __forceinline__ void fft_lines(T2 *A, int ls, int lines, const FFTPla
     switch (r) {
 #define G4_LOAD(R) \
   case R:          \
-    if (act) stage_load<R>(x, src, nb, ns, k, tw, sgn); \
+    if (act) stage_load<R>(x, src, nb, ns, k, tw); \
     break;
       G4_LOAD(2) G4_LOAD(3) G4_LOAD(4) G4_LOAD(5) G4_LOAD(7) G4_LOAD(8) G4_LOAD(9) G4_LOAD(11) G4_LOAD(13)
       G4_LOAD(15) G4_LOAD(16) G4_LOAD(17)
 #undef G4_LOAD
-      default: any_load(x, A, ls, lines, pl.n, ns, r, W, inverse); break;
+      default: any_load(x, A, ls, lines, pl.n, ns, r, W); break;
     }
     // the epilogue's source, copied asynchronously by the caller, must have landed
     // before the barrier ahead of the last stage's stores (all but the most recent
@@ -362,16 +372,16 @@ __device__ __forceinline__ void fft_lines(T2 *A, int ls, int lines, const FFTPla
     if (to_global && wait_epi_copy) cp_wait<1>();
     __syncthreads();
     const int o = line * ls + (j - k) * r + k;
-    Epilogue<T2> e = epi;
+    Epilogue<T2, EXCH> e = epi;
     if (e.src) e.src += o;
     switch (r) {
 #define G4_STORE(R)                                      \
   case R:                                                \
     if (act) {                                           \
       if (to_global)                                     \
-        dft<R, 2>(x, gout + o, ns, sgn, e);              \
+        dft<R, 2>(x, gout + o, ns, e);                   \
       else                                               \
-        dft<R, 1>(x, dst, ns, sgn);                      \
+        dft<R, 1>(x, dst, ns);                           \
     }                                                    \
     break;
       G4_STORE(2) G4_STORE(3) G4_STORE(4) G4_STORE(5) G4_STORE(7) G4_STORE(8) G4_STORE(9) G4_STORE(11)
@@ -393,10 +403,10 @@ constexpr int FFT_CTAS_FP32 = 3, FFT_CTAS_FP64 = 2;
 // prefetches its next tile by asynchronous copies into the second of two tile
 // buffers while it transforms the current one in place.
 
-// Row pass over tiles of L rows. MODE 0: forward FFT of the rows of `in` into `out`
-// (the same place of slice (ii + first) mod ns of each); MODE 1: inverse FFT of
-// the rows of `in`, times `scale`, plus 2 src (slice ii) when src is given, into
-// `out`, with the source rows in a third tile buffer and one CTA per SM fewer.
+// Row pass over tiles of L rows. MODE 0: FFT of the rows of `in` into `out` (the same
+// place of slice (ii + first) mod ns of each); MODE 1: FFT of the rows of `in`, whose real
+// and imaginary parts are exchanged, exchanged back (the inverse transform), times `scale`,
+// plus 2 src (slice ii) when src is given, into `out`, with the source rows in a third tile buffer and one CTA per SM fewer.
 // in == out transforms in place.
 template <typename T2, int MODE>
 __global__ void __launch_bounds__(256, (sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64) - MODE)
@@ -438,16 +448,15 @@ __global__ void __launch_bounds__(256, (sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CT
     __syncthreads();
     // the last stage writes the rows to global memory, scaled and with 2 src (MODE 1)
     T2 *o = out + (size_t)((ii + first) % ns) * ncell + (size_t)r0 * n;
-    fft_lines(A, n, lines, pl, W, MODE == 1, o, Epilogue<T2>{(R)scale, sb ? S : nullptr}, sb != nullptr);
+    fft_lines(A, n, lines, pl, W, o, Epilogue<T2, MODE>{(R)scale, sb ? S : nullptr}, sb != nullptr);
     __syncthreads();  // A is free for the copies of the next iteration
   }
   cp_wait<0>();
 }
 
-// sin and cos of the propagator's phase: FP64 library sincos for the plain form;
-// in FP32 the phase is first reduced to [-pi, pi] (the FP32 phase itself carries
-// an error of ~6e-8 of its size) and the fast hardware approximation taken
-__device__ __forceinline__ void phase_sincos(double a, double *sn, double *cs) { sincos(a, sn, cs); }
+// sin and cos of the propagator's phase in FP32: the phase is first reduced to [-pi, pi]
+// (the FP32 phase itself carries an error of ~6e-8 of its size) and the fast hardware
+// approximation taken
 __device__ __forceinline__ void phase_sincos(float a, float *sn, float *cs) {
   const float two_pi = 6.283185307179586f;
   a -= two_pi * rintf(a * (1.0f / two_pi));
@@ -465,14 +474,17 @@ __device__ __forceinline__ void load_cols(T2 *dst, const T2 *g, int n, int c0, i
       cp_elem(dst + tc * n + row, g + (size_t)row * n + c0 + tc);
 }
 
-// Column pass over tiles of L (<= 16) columns: forward FFT of the columns, the
-// propagator exp(K2 dz) (and the filtered source 2 FFT(src) sigmoid), inverse FFT
-// of the columns, written back in place. The propagator's phase at the FFT index
+// Column pass over tiles of L (<= 16) columns: FFT of the columns, the propagator exp(K2
+// dz) (and the filtered source 2 FFT(src) sigmoid), FFT of the columns with real and
+// imaginary parts exchanged (their inverse transform, exchanged), written back in place so. The propagator's phase at the FFT index
 // (ky, kx) is (dx^2 + dy^2) k2dz, k2dz = -dk^2 dz / (2 xks), with dx = ix - (n-1)/2
 // and ix = (kx + n - (n+1)/2) mod n (the reference's shifted frequency map), and
 // likewise dy; sigt holds the sigmoid transposed, sigt[kx n + ky], so that the
 // reads of a column are contiguous; srcf (filtered) holds the row-transformed
-// source of slice ii, staged in a third tile buffer.
+// source of slice ii, staged in a third tile buffer. In FP64 the propagator is the
+// product of a row and a column factor, exp(i dx^2 k2dz) exp(i dy^2 k2dz), from a table of n
+// entries a CTA forms once (both frequency maps are the same): a sincos per cell, about 35
+// FP64 instructions with its phase, would be a fifth of the pass.
 template <typename T2>
 __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64)
     k_fft_cols(T2 *__restrict__ field, const T2 *__restrict__ srcf, const T2 *__restrict__ roots, double k2dz,
@@ -483,6 +495,7 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
   const int n = pl.n;
   T2 *Abuf = W + 2 * n;
   T2 *SA = Abuf + 2 * L * n;  // filtered source columns (only with srcf)
+  T2 *E = SA + (srcf ? L * n : 0);  // FP64: exp(i dx^2 k2dz) by FFT index
   const int nblk = (n + L - 1) / L, ntiles = ns * nblk;
   const size_t ncell = (size_t)n * n;
   const R kdz = (R)k2dz, half = (R)(0.5 * (n - 1));
@@ -491,6 +504,16 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
   const int c_init = fdiv(threadIdx.x, n, pl.mn), ky_init = threadIdx.x - c_init * n;
   const int dc = fdiv(blockDim.x, n, pl.mn), dky = blockDim.x - dc * n;
   for (int t = threadIdx.x; t < 2 * n - 1; t += blockDim.x) cp_elem(W + t, roots + t);
+  if constexpr (sizeof(T2) == 16) {
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+      int ix = t + off;
+      ix -= ix >= n ? n : 0;
+      const R d = (R)ix - half;
+      R sn, cs;
+      sincos(d * d * kdz, &sn, &cs);
+      E[t] = mk<T2>(cs, sn);
+    }
+  }
   int tile = blockIdx.x;
   if (tile < ntiles) {
     const int ii = tile / nblk, c0 = (tile - ii * nblk) * L;
@@ -512,29 +535,32 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
     cp_commit();
     cp_wait<2>();
     __syncthreads();
-    // the transforms in one loop, so that the kernel holds one copy of their code:
-    // forward on the field's columns, (filtered) forward on the source's, then the
-    // propagator and the inverse on the field's
+    // the transforms in one loop, so that the kernel holds one copy of their code: the
+    // field's columns, (filtered) the source's, then the propagator and the field's again
     const int njob = srcf ? 3 : 2;
     for (int job = 0; job < njob; job++) {
-      const bool inverse = job == njob - 1;
       if (job == 1 && srcf) {
         cp_wait<1>();
         __syncthreads();
       }
-      if (inverse) {
+      if (job == njob - 1) {
         const R *st = sigt + (size_t)c0 * n;
         int c = c_init, ky = ky_init;
         for (int t = threadIdx.x; t < lines * n; t += blockDim.x) {
-          int ix = c0 + c + off, iy = ky + off;
-          ix -= ix >= n ? n : 0;
-          iy -= iy >= n ? n : 0;
-          const R dx = (R)ix - half, dy = (R)iy - half;
-          R sn, cs;
-          phase_sincos((dx * dx + dy * dy) * kdz, &sn, &cs);
-          T2 v = cm(A[t], mk<T2>(cs, sn));
+          T2 v;
+          if constexpr (sizeof(T2) == 16) {
+            v = cm(cm(A[t], E[c0 + c]), E[ky]);
+          } else {
+            int ix = c0 + c + off, iy = ky + off;
+            ix -= ix >= n ? n : 0;
+            iy -= iy >= n ? n : 0;
+            const R dx = (R)ix - half, dy = (R)iy - half;
+            R sn, cs;
+            phase_sincos((dx * dx + dy * dy) * kdz, &sn, &cs);
+            v = cm(A[t], mk<T2>(cs, sn));
+          }
           if (srcf) v = axpy((R)2 * st[t], SA[t], v);
-          A[t] = v;
+          A[t] = mk<T2>(v.y, v.x);
           c += dc;
           ky += dky;
           if (ky >= n) {
@@ -544,7 +570,7 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
         }
         __syncthreads();
       }
-      fft_lines(job == 1 && srcf ? SA : A, n, lines, pl, W, inverse);
+      fft_lines(job == 1 && srcf ? SA : A, n, lines, pl, W);
     }
     const int tc = threadIdx.x & 15;
     if (tc < lines)
@@ -597,7 +623,7 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
     cp_commit();
     cp_wait<1>();
     __syncthreads();
-    fft_lines(A, n, lines, pl, W, false);
+    fft_lines(A, n, lines, pl, W);
     R m[5] = {0, 0, 0, 0, 0};
     int c = c_init, ky = ky_init;
     for (int t = threadIdx.x; t < lines * n; t += blockDim.x) {
@@ -700,8 +726,9 @@ void launch_fft(void *stream, void *field, const void *src, void *work, const vo
   if (sfw) k_fft_rows<T2, 0><<<gr, FFT_THREADS, mr, s>>>(sr, sfw, nullptr, rt, pl, ns, 0, 1.0, Lr);
   // columns
   const int bc = sfw ? 3 : 2;
-  const int Lc = fft_lines_per_cta(pl, es, bc, 16, cols_ctas);
-  const size_t mc = fft_smem(n, Lc, bc, (size_t)es);
+  const size_t table = es == 16 ? (size_t)n * es : 0;  // the propagator's factors
+  const int Lc = fft_lines_per_cta(pl, es, bc, 16, cols_ctas, table);
+  const size_t mc = fft_smem(n, Lc, bc, (size_t)es) + table;
   k_fft_cols<T2><<<grid(Lc, mc, cols_ctas), FFT_THREADS, mc, s>>>(f, sfw, rt, k2c * delz, (const R *)sig, pl,
                                                                  ns, first, Lc);
   // inverse rows, 1/n^2, + 2 src when unfiltered (the source rows in a third tile
@@ -752,7 +779,7 @@ void launch_fft_diag_t(void *stream, const void *field, void *work, const void *
 // the generic stages at most 8 outputs per thread (L n <= 8 T), and the shared
 // memory of `per_sm` CTAs fits an SM (or one CTA's, in 227 KB, where not even
 // L = 1 fits that).
-int fft_lines_per_cta(const FFTPlan &pl, int es, int bufs, int maxL, int per_sm) {
+int fft_lines_per_cta(const FFTPlan &pl, int es, int bufs, int maxL, int per_sm, size_t table) {
   const int n = pl.n;
   int L = maxL;
   for (int s = 0; s < pl.nstage; s++) {
@@ -761,18 +788,18 @@ int fft_lines_per_cta(const FFTPlan &pl, int es, int bufs, int maxL, int per_sm)
     if (lim < L) L = lim;
   }
   if (L < 1) L = 1;
-  (void)es;
   const size_t cap = 228u * 1024u / per_sm - 1024;
-  while (L > 1 && fft_smem(n, L, bufs, es) > cap) L--;
+  while (L > 1 && fft_smem(n, L, bufs, es) + table > cap) L--;
   return L;
 }
 
 int fft_max_ngrid(int mixed) {
   // a register stage of one line with n / R <= 256 butterflies, the generic stages
   // of one line with at most 8 outputs per thread (n <= 2048), and one line in
-  // each of three tile buffers plus the roots and twiddles in 227 KB
+  // each of three tile buffers plus the roots, the twiddles and (FP64) the propagator's
+  // factors in 227 KB
   int es = mixed ? (int)sizeof(float2) : (int)sizeof(double2);
-  int m = (int)(227u * 1024u / (5u * (unsigned)es));
+  int m = (int)(227u * 1024u / ((mixed ? 5u : 6u) * (unsigned)es));
   return m < STAGE_ANY_OUT * FFT_THREADS ? m : STAGE_ANY_OUT * FFT_THREADS;
 }
 
