@@ -1,0 +1,372 @@
+// The fused field step with the first right-hand side's stencil term in tensor memory
+// (deposition and ADI of one slice in one CTA, FieldSolverADI.cpp:9-122; mixed form).
+// Included by kernels_mixed.cu.
+//
+// As in k_field_fused_f the slice's system is solved in shared memory, S [ng][st]:
+//   S = S1 = (I + c Dy) u    every column cut into segments of rows, one thread each, u
+//                            straight from global memory; S1 is kept in tensor memory
+//   S = S1 + src             deposition
+//   S = Thomas_x(S)          rows, segments
+//   u = Thomas_y(2 S - S1)   columns: the segments of the first phase, so that each thread
+//                            finds its own S1
+// What bounded k_field_fused_f was the sum of its phases' latencies (one CTA an SM: the
+// slice's bulk load, the deposition's reads, the reread of u from L2 for the second
+// right-hand side, the bulk store) and the shared-memory wavefronts of the solves. Here a
+// persistent CTA takes slice after slice and prefetches the next one's field and particles
+// into L2 while it solves; S1 costs no shared-memory or L2 traffic (tensor memory holds 64
+// words a thread at 1024 threads: 32 rows of a column); and a solve reads and writes each
+// row once (solve_window), without a barrier inside. The segments are solved as if the
+// field were zero outside them, with the settled coefficients (cbet and cwet reach their
+// limits within W rows): (I - i c D) is then the same convolution everywhere, whose response
+// fades by kappa = -c cbet per row on both sides, so
+//   x_k = x0_k + kappa^{k-b+1} l + kappa^{e-k} r
+// with l and r the neighbours' x0 next to the segment, or at the grid's edges, where the
+// field is zero one row outside, minus kappa times its own first or last x0 (the mirror
+// image). The terms are kept for W rows, kappa^W below 2^-32 (the host's segment_warmup;
+// every segment is longer than W). The columns' rows next to a segment's ends get them as
+// they are written to u. Rows have an odd stride st, so that the row solve, whose lanes walk
+// different rows, finds different banks on even grids too.
+// Measured (after 20 steps, k_field_fused_f at its best CTA size before): 4096 slices x 8192
+// particles, 151^2 1000 -> 641 us (3.4 TB/s of the algorithmic bytes, half of the copy
+// bandwidth); 700 x 8192, 151^2 197 -> 134 us; 2000 x 4096, 117^2 253 -> 197 us; 700 x 8192,
+// 128^2 336 -> 112 us. Of a slice's 46 thousand cycles the deposition takes 12, the column solve
+// 10, the row solve 7, the last pass 7, S1 5, the rows' carries 3.
+
+// Sixteen words (eight complex values) of this thread's tensor memory.
+#define G4_TM_W(v, j) "r"(__float_as_uint(v[j].x)), "r"(__float_as_uint(v[j].y))
+__device__ __forceinline__ void tm_put8(uint32_t a, const float2 *v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16};" ::"r"(a),
+      G4_TM_W(v, 0), G4_TM_W(v, 1), G4_TM_W(v, 2), G4_TM_W(v, 3), G4_TM_W(v, 4), G4_TM_W(v, 5), G4_TM_W(v, 6),
+      G4_TM_W(v, 7)
+      : "memory");
+}
+#undef G4_TM_W
+__device__ __forceinline__ void tm_get8(uint32_t a, float2 *v) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(a)
+      : "memory");
+#pragma unroll
+  for (int j = 0; j < 8; j++) v[j] = make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+}
+
+// v + w x for complex w
+__device__ __forceinline__ float2 add_cmulf(float2 v, float2 w, float2 x) {
+  return make_float2(fmaf(w.x, x.x, fmaf(-w.y, x.y, v.x)), fmaf(w.x, x.y, fmaf(w.y, x.x, v.y)));
+}
+
+constexpr int kTmLook = 16;   // the longest look-ahead of the solves
+constexpr int kTmChunk = 8;   // rows a window of the solves loads and delivers at a time
+// 85 registers a thread hold the windows (1024 threads, 64 registers, spilled)
+constexpr int kTmMaxThreads = 768;
+struct TmShape {
+  int threads, nseg, words, cols;  // words of tensor memory a thread, columns a CTA allocates
+};
+// The shape for CTAs of `threads`: as many segments as the threads and the warm-up allow,
+// up to 8 (threads 0: none fits).
+inline TmShape tm_shape(int ng, int threads, int W) {
+  threads = std::min(threads, kTmMaxThreads);
+  TmShape t{threads, std::min(std::min(threads / ng, 8), ng / (W + 1)), 0, 0};
+  if (W < 1 || W > kTmLook + 1 || t.nseg < 2) return TmShape{0, 0, 0, 0};
+  const int len = (ng + t.nseg - 1) / t.nseg, per = (threads / 32 + 3) / 4;  // warps a lane quarter
+  t.words = (len + 7) / 8 * 16;
+  int c = 32;
+  while (c < per * t.words) c *= 2;
+  if (c > 512) return TmShape{0, 0, 0, 0};
+  t.cols = c;
+  return t;
+}
+inline size_t tm_smem_bytes(int ng, int W, int threads) {
+  return (((size_t)W + 1) / 2 * 2 + ((size_t)ng * (ng | 1) + 1) / 2 * 2) * sizeof(float2) +
+         (size_t)(threads / 32 + 1) * kFieldSums * sizeof(double);
+}
+
+// The solve of rows [b, e) of a line, zeros outside, in one pass over it: the forward values d
+// of a window of CH + LA rows stay in registers, and the back substitution runs over the
+// window from zero, LA rows ahead of the CH rows it delivers (LA + 1 >= W: the part left out
+// is below kappa^W). So a row is read once and
+// written once, where a pass down and one up move it four times: the solves are bound by
+// shared-memory wavefronts and issue. load(r, v) gives the right-hand sides of CH rows from
+// r, zeros for rows >= e (every thread of a warp calls it together), emit(r, x) takes the
+// solution of row r < e.
+template <int LA, class LD, class EM>
+__device__ __forceinline__ void solve_window(int b, int e, int nchunk, float cs, float2 cb, float2 kap, LD load,
+                                             EM emit) {
+  constexpr int CH = kTmChunk;
+  float2 d[CH + LA], last = make_float2(0.f, 0.f);
+  auto forward = [&](int r, float2 *o) {
+    load(r, o);
+#pragma unroll
+    for (int j = 0; j < CH; j++) {
+      last = cmulf(sub_imulf(o[j], -cs, last), cb);
+      o[j] = last;
+    }
+  };
+#pragma unroll
+  for (int p = 0; p < LA; p += CH) forward(b + p, d + p);
+#pragma unroll 1
+  for (int q = 0; q < nchunk; q++) {
+    const int r0 = b + q * CH;
+    forward(r0 + LA, d + LA);
+    float2 x = d[CH + LA - 1];
+#pragma unroll
+    for (int j = CH + LA - 2; j >= 0; j--) {
+      x = add_cmulf(d[j], kap, x);
+      if (j < CH && r0 + j < e) emit(r0 + j, x);
+    }
+#pragma unroll
+    for (int j = 0; j < LA; j++) d[j] = d[CH + j];
+  }
+}
+
+// Prefetches [p, p + bytes) of an array into L2, rounded inwards to 16 bytes.
+__device__ __forceinline__ void l2_prefetch(const void *p, size_t bytes) {
+  const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
+  const uintptr_t z = (reinterpret_cast<uintptr_t>(p) + bytes) & ~(uintptr_t)15;
+  if (z > a)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(z - a)) : "memory");
+}
+
+// Sums of v[0..8) over a warp: lane 4 k holds the sum of v[k] (nine shuffles: each step
+// halves the values a lane carries).
+__device__ __forceinline__ float warp_sums8(float (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16, n = 4; o >= 4; o >>= 1, n >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (j < n) {
+        const float send = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
+        v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+  }
+  float s = v[0];
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
+
+// REC: the field record of every slice (k_diag_field_f's sums) is formed too.
+template <int LA, bool REC>
+__global__ void __launch_bounds__(kTmMaxThreads, 1)
+    k_field_tm_f(StepConstF sc, int k, PtrsF p, float2 *__restrict__ field, const float2 *__restrict__ coef,
+                 const float2 *__restrict__ pows, int ns, int np, int ng, int deposit, int nseg, int W, int words,
+                 int cols, double *dfield) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t tm_base;
+  const int tid = threadIdx.x, warp = tid >> 5, st = ng | 1;
+  const FieldStepF &fs = sc.f[k];
+  float2 *PW = reinterpret_cast<float2 *>(smem_raw);  // kappa^{j+1}
+  float2 *S = PW + (W + 1) / 2 * 2;
+  double *red = reinterpret_cast<double *>(S + (ng * st + 1) / 2 * 2);
+  if (warp == 0) {
+    const uint32_t sadr = (uint32_t)__cvta_generic_to_shared(&tm_base);
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sadr), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  for (int t = tid; t < W; t += blockDim.x) PW[t] = pows[t];
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tm = tm_base + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * words);
+
+  // line (a column in the column phases, a row in the row solve) and segment of the thread
+  const int line = tid % ng, seg = tid / ng;
+  const bool act = seg < nseg;
+  const int b = act ? seg * ng / nseg : 0, e = act ? (seg + 1) * ng / nseg : 0;
+  const bool left = act && seg > 0, right = act && seg + 1 < nseg;
+  const int nq = words >> 4;  // batches of eight rows
+  const int nchunk = ((ng + nseg - 1) / nseg + kTmChunk - 1) / kTmChunk;
+  const float cs = fs.cstep;
+  const float2 cb = coef[2 * ng - 1], kap = PW[0], zero = make_float2(0.f, 0.f);
+  // the part of a segment's solution that reaches it over its ends: its neighbour's at the
+  // end, times kappa per row; at the grid's edges minus the mirror image of its own (the
+  // field is zero one row outside)
+  auto carry = [&](bool inner, float2 other, float2 own) { return inner ? other : cmulf(make_float2(-kap.x, -kap.y), own); };
+
+#pragma unroll 1
+  for (int is = blockIdx.x; is < ns; is += gridDim.x) {
+    const int i = ring_slot(is, fs.first, ns);
+    float2 *u = field + (size_t)i * ng * ng;
+    // the first particles' loads in flight while S1 is formed (the vector path: full slices
+    // of a multiple of 4 particles)
+    const size_t base = (size_t)is * np;
+    const bool vec = deposit && (np & 3) == 0 && !p.count;
+    Quad quad{};
+    if (vec && tid < (np >> 2)) quad = load_quad(p, base, tid);
+    // S1 of the thread's rows of its column, eight rows' loads at a time; rows outside the
+    // grid are zeros, which gives the one-sided differences at the edges
+    {
+      float2 prev = left ? u[(b - 1) * ng + line] : zero;
+      float2 cur = act ? u[b * ng + line] : zero;
+#pragma unroll 1
+      for (int q = 0; q < nq; q++) {
+        float2 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const int r = b + 8 * q + j;
+          v[j] = r < e && r + 1 < ng ? u[(r + 1) * ng + line] : zero;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float2 nx = v[j];
+          v[j] = stencil(cs, cur, make_float2(nx.x - 2.f * cur.x + prev.x, nx.y - 2.f * cur.y + prev.y));
+          prev = cur;
+          cur = nx;
+          const int r = b + 8 * q + j;
+          if (r < e) S[r * st + line] = v[j];
+        }
+        __syncwarp();
+        tm_put8(tm + 16 * q, v);
+      }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    __syncthreads();
+    if (deposit) {  // S = S1 + src
+      if (vec) {
+        const float scl = fs.dep_scl * (float)p.current[is];
+#pragma unroll 1
+        for (int q = tid; q < (np >> 2); q += blockDim.x) {
+          const Quad v = quad;
+          if (q + (int)blockDim.x < (np >> 2)) quad = load_quad(p, base, q + blockDim.x);
+          deposit_quad(sc, fs, scl, S, Grid(ng, st), v);
+        }
+      } else {
+        deposit_smem(sc, fs, p, S, is, np, Grid(ng, st));
+      }
+      __syncthreads();
+    }
+    // the next slice's field and particles on their way to L2 while this one is solved
+    if (tid < 5 && is + (int)gridDim.x < ns) {
+      const int nx = is + gridDim.x;
+      const size_t o = (size_t)nx * np;
+      const size_t n = p.count ? min(p.count[nx], np) : np;
+      if (tid == 0) l2_prefetch(field + (size_t)ring_slot(nx, fs.first, ns) * ng * ng, (size_t)ng * ng * 8);
+      if (deposit && tid == 1) l2_prefetch(p.x + o, n * 4);
+      if (deposit && tid == 2) l2_prefetch(p.y + o, n * 4);
+      if (deposit && tid == 3) l2_prefetch(p.dg + o, n * 4);
+      if (deposit && tid == 4) l2_prefetch(p.theta + o, n * 8);
+    }
+    // rows: u', zero carries, then the neighbours'
+    {
+      float2 *L = S + line * st;
+      solve_window<LA>(
+          b, e, nchunk, cs, cb, kap,
+          [&](int r, float2 *v) {
+#pragma unroll
+            for (int j = 0; j < kTmChunk; j++) v[j] = r + j < e ? L[r + j] : zero;
+          },
+          [&](int r, float2 x) { L[r] = x; });
+      __syncthreads();
+      float2 lc = zero, rc = zero;
+      if (act) {
+        lc = carry(left, left ? L[b - 1] : zero, L[b]);
+        rc = carry(right, right ? L[e] : zero, L[e - 1]);
+      }
+      __syncthreads();
+      if (act)
+        for (int j = 0; j < W; j++) {
+          L[b + j] = add_cmulf(L[b + j], PW[j], lc);
+          L[e - 1 - j] = add_cmulf(L[e - 1 - j], PW[j], rc);
+        }
+    }
+    __syncthreads();
+    // columns: the second right-hand side 2 u' - S1, solved, then written with the
+    // neighbours' carries (writing the rows without carries from the solve itself: 631 against
+    // 640 us for 4096 slices of 151^2, 257 against 250 us for 2000 of 117^2)
+    float2 *L = S + line;
+    const int lo = b + W, hi = e - W;  // [lo, hi): no carry
+    solve_window<LA>(
+        b, e, nchunk, cs, cb, kap,
+        [&](int r, float2 *v) {
+          const int q = (r - b) >> 3;
+          if (q < nq) {
+            float2 s1[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = r + j < e ? L[(r + j) * st] : zero;
+            __syncwarp();
+            tm_get8(tm + 16 * q, s1);
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+              v[j] = r + j < e ? make_float2(2.f * v[j].x - s1[j].x, 2.f * v[j].y - s1[j].y) : zero;
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = zero;
+          }
+        },
+        [&](int r, float2 x) { L[r * st] = x; });
+    __syncthreads();
+    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    {
+      float2 lc = zero, rc = zero;
+      if (act) {
+        lc = carry(left, left ? L[(b - 1) * st] : zero, L[b * st]);
+        rc = carry(right, right ? L[e * st] : zero, L[(e - 1) * st]);
+      }
+      const float shift = -0.5f * (float)(ng - 1);
+      float dy = (float)b + shift;
+      auto put = [&](int r, float2 x) {
+        u[r * ng + line] = x;
+        if constexpr (REC) {
+          const float w = fmaf(x.x, x.x, x.y * x.y), t = dy * w;
+          f[0] += w;
+          f[3] += t;
+          f[4] = fmaf(dy, t, f[4]);
+          f[5] += x.x;
+          f[6] += x.y;
+          dy += 1.f;
+        }
+      };
+      const int mid = min(lo, e);
+#pragma unroll 4
+      for (int r = b; r < mid; r++) {
+        float2 x = add_cmulf(L[r * st], PW[r - b], lc);
+        if (r >= hi) x = add_cmulf(x, PW[e - 1 - r], rc);
+        put(r, x);
+      }
+#pragma unroll 4
+      for (int r = mid; r < hi; r++) put(r, L[r * st]);
+#pragma unroll 4
+      for (int r = max(mid, hi); r < e; r++) put(r, add_cmulf(L[r * st], PW[e - 1 - r], rc));
+      if constexpr (REC) {
+        const float dx = (float)line + shift;
+        f[1] = dx * f[0];
+        f[2] = dx * f[1];
+      }
+    }
+    if constexpr (REC) {
+      double *o = dfield + (size_t)i * (kFieldSums + 2);
+      if (line == ng / 2 && b <= ng / 2 && ng / 2 < e) {  // the value on the axis
+        const float2 v = u[(ng / 2) * ng + ng / 2];
+        o[7] = v.x;
+        o[8] = v.y;
+      }
+      const float v = warp_sums8(f);
+      if ((tid & 3) == 0 && (tid & 31) < 4 * kFieldSums) red[warp * kFieldSums + ((tid & 31) >> 2)] = (double)v;
+      __syncthreads();
+      // the last warp folds the warps' sums in FP64, four lanes a value, while the others go on
+      if (warp == (int)(blockDim.x >> 5) - 1) {
+        const int k2 = (tid & 31) >> 2;
+        double t = 0;
+        if (k2 < kFieldSums)
+          for (int w = tid & 3; w < (int)(blockDim.x >> 5); w += 4) t += red[w * kFieldSums + k2];
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        if ((tid & 3) == 0 && k2 < kFieldSums) o[k2] = t;
+      }
+    } else {
+      __syncthreads();
+    }
+  }
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(cols) : "memory");
+}

@@ -438,7 +438,7 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
   typedef std::complex<double> cd;
   std::map<std::pair<int, double>, int> sets;  // (field, delz) -> set
   std::vector<cd> coefs;                       // [nset][3][ng]
-  std::vector<cd> pows;                        // plain form: [nset][2][kSegPow]
+  std::vector<cd> pows;                        // [nset][2][kSegPow]
   std::vector<int> set_tw;                     // warm-up length per coefficient set
   for (int i = 0; i < nsteps; i++) {
     const double *r = tab + (size_t)i * G4GPU_LAT_NCOL;
@@ -522,9 +522,9 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
         coefs.insert(coefs.end(), cb.begin(), cb.end());
         coefs.insert(coefs.end(), cw.begin(), cw.end());
         set_tw.push_back(segment_warmup(cc, cb, cw, h->mixed ? 32 : 62));
-        if (!h->mixed) {
+        {
           // kappa^{j+1} and kappa^{j+1} / (1 - kappa^2) of the settled recurrences,
-          // kappa = -cwet (adi_plain.cuh)
+          // kappa = -cwet (adi_plain.cuh, field_tm.cuh)
           const cd kappa = -cw[ng - 1], q = 1. / (1. - kappa * kappa);
           cd p = kappa;
           std::vector<cd> pw(g4::kSegPow);
@@ -591,11 +591,14 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
     h->seg_pow_bytes = 0;
   }
   if (!pows.empty()) {
-    const size_t nb = pows.size() * sizeof(cd);
+    const size_t nb = pows.size() * h->csize;
     int rc = alloc(h, &h->seg_pow, nb);
     if (rc) return rc;
     h->seg_pow_bytes = nb;
-    G4_CUDA(h, cudaMemcpy(h->seg_pow, pows.data(), nb, cudaMemcpyHostToDevice));
+    std::vector<std::complex<float>> pf;
+    if (h->mixed) pf.assign(pows.begin(), pows.end());
+    G4_CUDA(h, cudaMemcpy(h->seg_pow, h->mixed ? (const void *)pf.data() : (const void *)pows.data(), nb,
+                          cudaMemcpyHostToDevice));
   }
   if (!coefs.empty()) {
     size_t n = coefs.size();
@@ -938,6 +941,15 @@ int g4gpu_get_field(g4gpu_handle h, int ifld, double *field, int *first, double 
   return check_device_flag(h);
 }
 
+// The powers of a coefficient set's segmented solves.
+static const void *seg_powers(g4gpu_handle h, int set) {
+  return (const char *)h->seg_pow + (size_t)set * 2 * g4::kSegPow * h->csize;
+}
+// Threads a CTA of the fused field kernel: as set, else by the grid and the window.
+static int field_threads(g4gpu_handle h, int W) {
+  return h->field_threads > 0 ? h->field_threads : g4::field_threads_auto(h->cfg.ngrid, h->cfg.nslice, W);
+}
+
 // Threads a block of the push: as set (g4gpu_set_launch_shapes, g4gpu_autotune), else by
 // the window. The FP64 push holds a scheduler for ~400 x 64 cycles a warp, so a window of
 // few particles takes small blocks that spread over the SMs (64 against 256 threads:
@@ -1206,8 +1218,8 @@ static int enqueue_coarse_step(g4gpu_handle h, int istep, int cnt) {
   const char *cb = (const char *)h->coef + (size_t)sc.f[0].coef * 3 * ng * h->csize;
   {
     Timed t(h, G4GPU_K_ADI_X);
-    g4::launch_field_fused_mixed(L, scf, 0, h->beam, h->field[0], cb, ns, np, ng, 0, h->field_threads, nullptr,
-                                 nullptr, 1, c.gammaref);
+    g4::launch_field_fused_mixed(L, scf, 0, h->beam, h->field[0], cb, seg_powers(h, sc.f[0].coef), ns, np, ng, 0,
+                                 field_threads(h, sc.f[0].tw), nullptr, nullptr, 1, c.gammaref);
   }
   G4_CUDA(h, cudaGetLastError());
   return G4GPU_OK;
@@ -1331,16 +1343,17 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
     bool pair = band_cl > 0 && (h->field_kernel == 1 || !fused);
     // the whole step in one kernel (push, deposition, ADI; one CTA per slice): chosen
     // by the autotuner (field_kernel 2) for one-field windows without space charge
-    const bool rec_ok = h->diag_rec && g4::fused_diag_fits(ng, h->field_threads, h->diag_nharm);
+    const int step_threads = h->field_threads > 0 ? h->field_threads : 512;
+    const bool rec_ok = h->diag_rec && g4::fused_diag_fits(ng, step_threads, h->diag_nharm);
     const bool step_fused = fused && h->field_kernel == 2 && do_push && do_field && !h->sc_on &&
-                            g4::step_fused_ok(c.nfield, ng, h->field_threads, rec_ok, rec_ok, h->diag_nharm);
+                            g4::step_fused_ok(c.nfield, ng, step_threads, rec_ok, rec_ok, h->diag_nharm);
     if (step_fused) {
       const char *cb = (const char *)h->coef + (size_t)sc.f[0].coef * 3 * ng * h->csize;
       const int bw = g4::beam_diag_width(h->diag_nharm);
       {
         Timed t(h, G4GPU_K_STEP);
         g4::launch_step_fused_mixed(L, scf_push, h->beam, h->field[0], cb, ns, np, ng, sc.f[0].dep_on,
-                                    h->field_threads, wake, isr, rec_ok ? h->diag_rec : nullptr,
+                                    step_threads, wake, isr, rec_ok ? h->diag_rec : nullptr,
                                     rec_ok ? h->diag_rec + (size_t)ns * bw : nullptr, h->diag_nharm, c.gammaref);
       }
       if (isr.ctr) g4::launch_isr_advance(h->stream, h->isr_ctr);
@@ -1351,7 +1364,9 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       if (do_field) {
         // the diagnostic record of a step run by g4gpu_run_diag, formed by the fused
         // kernel itself when it holds the scratch for it
-        const bool rec = h->diag_rec && !pair && g4::fused_diag_fits(ng, h->field_threads, h->diag_nharm);
+        bool rec = h->diag_rec && !pair;
+        for (int k = 0; k < c.nfield && rec; k++)
+          rec = g4::field_record_fits(ng, field_threads(h, sc.f[k].tw), sc.f[k].tw, h->diag_nharm);
         const int bw = g4::beam_diag_width(h->diag_nharm), fw = g4::kFieldSums + 2;
         for (int k = 0; k < c.nfield; k++) {
           const char *cb = (const char *)h->coef + (size_t)sc.f[k].coef * 3 * ng * h->csize;
@@ -1360,8 +1375,8 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
             g4::launch_field_band_mixed(L, scf, k, h->beam, h->field[k], cb, ns, np, ng, sc.f[k].dep_on,
                                         band_cl);
           else
-            g4::launch_field_fused_mixed(L, scf, k, h->beam, h->field[k], cb, ns, np, ng, sc.f[k].dep_on,
-                                         h->field_threads, nullptr,
+            g4::launch_field_fused_mixed(L, scf, k, h->beam, h->field[k], cb, seg_powers(h, sc.f[k].coef), ns, np, ng,
+                                         sc.f[k].dep_on, field_threads(h, sc.f[k].tw), nullptr,
                                          rec ? h->diag_rec + (size_t)ns * bw + (size_t)k * ns * fw : nullptr,
                                          h->diag_nharm, c.gammaref);
         }
@@ -1402,8 +1417,7 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
             g4::launch_adi_mixed(L, scf, k, phase, h->field[k], srck, h->tmp, cb, ns, ng);
           else
             g4::launch_adi_plain(L, sc, k, phase, h->field[k], h->src[k], h->tmp, cb,
-                                 (const char *)h->seg_pow + (size_t)sc.f[k].coef * 2 * g4::kSegPow * 2 * sizeof(double), ns, ng,
-                                 srck != nullptr);
+                                 seg_powers(h, sc.f[k].coef), ns, ng, srck != nullptr);
         }
       }
     }

@@ -29,7 +29,7 @@ struct g4gpu_ctx {
   void *diag_work = nullptr;  // g4gpu_diag_fft's scratch where tmp is absent
   void *coef = nullptr;      // [nset][3][ngrid] complex of the field type
   size_t coef_bytes = 0;
-  void *seg_pow = nullptr;   // plain form: [nset][2][kSegPow] powers of the segmented solves
+  void *seg_pow = nullptr;   // [nset][2][kSegPow] powers (complex of the field type) of the segmented solves
   size_t seg_pow_bytes = 0;
   // FFT solver tables per field: roots of unity [n], Im(K2) and the sigmoid [n^2]
   void *fft_roots[G4GPU_MAX_FIELDS] = {};
@@ -97,10 +97,9 @@ struct g4gpu_ctx {
   bool beam_loaded = false;
   bool field_loaded[G4GPU_MAX_FIELDS] = {};
 
-  // launch shapes (chosen by g4gpu_autotune, defaults otherwise; push_block 0: by the
-  // window's size)
+  // launch shapes (chosen by g4gpu_autotune, defaults otherwise; 0: by the window's size)
   int push_block = 0;
-  int field_threads = 512;
+  int field_threads = 0;
   // mixed ADI with the slice in shared memory: 0 one CTA per slice (k_field_fused_f),
   // 1 a cluster pair (k_field_band_f<2>), 2 the whole step per CTA (k_step_fused_f)
   int field_kernel = 0;

@@ -100,6 +100,7 @@ struct StepConstF {
   float aw_t, qx, qy, xoff, yoff, cxk, cyk;
   int kindx, kindy, corr, nfld;
   float aw, ax, ay, kx, ky, gradx, grady;
+  int centred;  // StepConst::centred
   float xks, xku, delz, ztemp1;
   double autophase;
   long long autophase_q;  // autophase as a Q32.32 turn count
@@ -178,9 +179,14 @@ void launch_field_band_mixed(const Launch &L, const StepConstF &sc, int k, const
 // threads: CTA size, a multiple of 32 in [2 ngrid, 1024]. dbeam / dfield (may be
 // null): the step's diagnostic record, beam [nslice][beam_diag_width(nharm)] (formed by
 // the launch of field 0) and this field's [nslice][kFieldSums + 2] in storage order.
+// pow: the coefficient set's [2][kSegPow] powers.
 void launch_field_fused_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b,
-                              void *field, const void *coef, int ns, int np, int ngrid, int deposit,
+                              void *field, const void *coef, const void *pow, int ns, int np, int ngrid, int deposit,
                               int threads, double *dbeam, double *dfield, int nharm, double gref);
+// the CTA size of a handle without a set one, and whether the kernel that size and warm-up
+// length W select records the field's diagnostics
+int field_threads_auto(int ngrid, int ns, int W);
+bool field_record_fits(int ngrid, int threads, int W, int nharm);
 // One source sub-step of a coarse step (g4gpu_set_field_substeps; k_source_f): the
 // deposition of every beam slice into field 0's slot (is + sc.f[0].first) % ns, u +=
 // scale * src, from phases and positions interpolated at frac between tp, xp, yp (the

@@ -24,6 +24,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include <cmath>
@@ -67,6 +68,7 @@ StepConstF to_float(const StepConst &s, int npart) {
   f.xku = (float)s.xku;
   f.delz = (float)s.delz;
   f.ztemp1 = (float)(-2. / s.xks);
+  f.centred = s.centred;
   f.autophase = s.autophase;
   f.autophase_q = (long long)llrint(s.autophase * (4294967296.0 / kTwoPiHost));
   f.gammaref = s.gammaref;
@@ -178,7 +180,14 @@ struct CellF {
   int i00, i10, i01, i11;
   float wx, wy;
 };
-__device__ __forceinline__ bool ll_gridpoint_f(float gm, float dg, int ng, float x, float y, CellF &c) {
+// ng x ng cells in rows of st elements
+struct Grid {
+  int ng, st;
+  __device__ __forceinline__ Grid(int n) : ng(n), st(n) {}
+  __device__ __forceinline__ Grid(int n, int stride) : ng(n), st(stride) {}
+};
+__device__ __forceinline__ bool ll_gridpoint_f(float gm, float dg, Grid g, float x, float y, CellF &c) {
+  const int ng = g.ng;
   if ((x > -gm) && (x < gm) && (y > -gm) && (y < gm)) {
     float wx = (x + gm) / dg, wy = (y + gm) / dg;
     float fx = floorf(wx), fy = floorf(wy);
@@ -187,10 +196,10 @@ __device__ __forceinline__ bool ll_gridpoint_f(float gm, float dg, int ng, float
     c.wy = 1.f + fy - wy;
     int ix1 = ix + 1 < ng ? ix + 1 : ix;
     int iy1 = iy + 1 < ng ? iy + 1 : iy;
-    c.i00 = ix + iy * ng;
-    c.i10 = ix1 + iy * ng;
-    c.i01 = ix + iy1 * ng;
-    c.i11 = ix1 + iy1 * ng;
+    c.i00 = ix + iy * g.st;
+    c.i10 = ix1 + iy * g.st;
+    c.i01 = ix + iy1 * g.st;
+    c.i11 = ix1 + iy1 * g.st;
     return true;
   }
   return false;
@@ -757,6 +766,23 @@ __device__ __forceinline__ void r2_cols_seg(float2 *S, const float2 *__restrict_
   }
 }
 
+// Adds v[0..3] to the four cells i00, i10, i01, i11 of S (shared or global memory). Odd lanes
+// add their imaginary parts first: a warp's addresses then lie in all banks of shared memory
+// instead of every other one (the deposition's 512 warp-wide additions for 2048 quads took 7
+// of its 15 thousand cycles). Measured and slower: one 64-bit compare-and-swap loop per cell
+// for both parts, in turn or the four side by side (field step of 4096 slices 709 -> 712 and
+// 737 us).
+__device__ __forceinline__ void add_to_cells(float2 *S, int i00, int i10, int i01, int i11, const float2 *v) {
+  const int i[4] = {i00, i10, i01, i11};
+  const bool odd = threadIdx.x & 1u;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    float *c = reinterpret_cast<float *>(S + i[q]);
+    atomicAdd(c + (odd ? 1 : 0), odd ? v[q].y : v[q].x);
+    atomicAdd(c + (odd ? 0 : 1), odd ? v[q].x : v[q].y);
+  }
+}
+
 // Adds the source contribution of the 32 particles held by the lanes of a warp (one
 // each; lanes past the end carry x = 1e30, off the grid) to S with shared-memory
 // atomics. Lanes whose particles share the lower-left cell (quiet loading stores
@@ -766,7 +792,7 @@ __device__ __forceinline__ void r2_cols_seg(float2 *S, const float2 *__restrict_
 // the atomics (and their same-address conflicts) by the run length and keeps the
 // result exact up to FP32 summation order. Every lane of the warp must call it.
 __device__ __forceinline__ void deposit_lanes(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                              int ng, float x, float y, long long th, float dgam) {
+                                              Grid ng, float x, float y, long long th, float dgam) {
   const unsigned lane = threadIdx.x & 31u;
   CellF c;
   bool on = ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c);
@@ -818,21 +844,16 @@ __device__ __forceinline__ void deposit_lanes(const StepConstF &sc, const FieldS
     }
   }
   if (on && run_head) {
-    atomicAdd(&S[c.i00].x, v[0]);
-    atomicAdd(&S[c.i00].y, v[1]);
-    atomicAdd(&S[c.i10].x, v[2]);
-    atomicAdd(&S[c.i10].y, v[3]);
-    atomicAdd(&S[c.i01].x, v[4]);
-    atomicAdd(&S[c.i01].y, v[5]);
-    atomicAdd(&S[c.i11].x, v[6]);
-    atomicAdd(&S[c.i11].y, v[7]);
+    const float2 w[4] = {make_float2(v[0], v[1]), make_float2(v[2], v[3]), make_float2(v[4], v[5]),
+                         make_float2(v[6], v[7])};
+    add_to_cells(S, c.i00, c.i10, c.i01, c.i11, w);
   }
 }
 
 // Adds the deposited source of beam slice `is` to S, the particles read from global
 // memory (used when no staging buffer fits beside the slice).
 __device__ __forceinline__ void deposit_smem(const StepConstF &sc, const FieldStepF &fs,
-                                             const PtrsF &p, float2 *S, int is, int np, int ng) {
+                                             const PtrsF &p, float2 *S, int is, int np, Grid ng) {
   const float scl = fs.dep_scl * slice_cur_f(p, is, np);
   const size_t base = (size_t)is * np;
   const int n = slice_np_f(p, is, np);
@@ -858,7 +879,7 @@ __device__ __forceinline__ void deposit_smem(const StepConstF &sc, const FieldSt
 
 // The contribution of one particle to the four cells around it (no aggregation).
 __device__ __forceinline__ void deposit_one(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                            int ng, float x, float y, long long th, float dgam) {
+                                            Grid ng, float x, float y, long long th, float dgam) {
   CellF c;
   if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c)) return;
   float dx = x - sc.ax, dy = y - sc.ay;
@@ -868,21 +889,16 @@ __device__ __forceinline__ void deposit_one(const StepConstF &sc, const FieldSte
   __sincosf(phase_of(th, (unsigned)fs.harm), &sn, &co);
   float cpx = sn * part, cpy = co * part;
   float w00 = c.wx * c.wy, w10 = (1.f - c.wx) * c.wy, w01 = c.wx * (1.f - c.wy), w11 = (1.f - c.wx) * (1.f - c.wy);
-  atomicAdd(&S[c.i00].x, w00 * cpx);
-  atomicAdd(&S[c.i00].y, w00 * cpy);
-  atomicAdd(&S[c.i10].x, w10 * cpx);
-  atomicAdd(&S[c.i10].y, w10 * cpy);
-  atomicAdd(&S[c.i01].x, w01 * cpx);
-  atomicAdd(&S[c.i01].y, w01 * cpy);
-  atomicAdd(&S[c.i11].x, w11 * cpx);
-  atomicAdd(&S[c.i11].y, w11 * cpy);
+  const float2 v[4] = {make_float2(w00 * cpx, w00 * cpy), make_float2(w10 * cpx, w10 * cpy),
+                       make_float2(w01 * cpx, w01 * cpy), make_float2(w11 * cpx, w11 * cpy)};
+  add_to_cells(S, c.i00, c.i10, c.i01, c.i11, v);
 }
 
 // The summed contribution of n particles that share x and y (one cell, one set of
 // weights, one undulator factor), n = 2 or 4.
 template <int N>
 __device__ __forceinline__ void deposit_group(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                              int ng, float x, float y, const long long *th, const float *dgam) {
+                                              Grid ng, float x, float y, const long long *th, const float *dgam) {
   CellF c;
   if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c)) return;
   float dx = x - sc.ax, dy = y - sc.ay;
@@ -898,55 +914,70 @@ __device__ __forceinline__ void deposit_group(const StepConstF &sc, const FieldS
     cpy += co * part;
   }
   float w00 = c.wx * c.wy, w10 = (1.f - c.wx) * c.wy, w01 = c.wx * (1.f - c.wy), w11 = (1.f - c.wx) * (1.f - c.wy);
-  atomicAdd(&S[c.i00].x, w00 * cpx);
-  atomicAdd(&S[c.i00].y, w00 * cpy);
-  atomicAdd(&S[c.i10].x, w10 * cpx);
-  atomicAdd(&S[c.i10].y, w10 * cpy);
-  atomicAdd(&S[c.i01].x, w01 * cpx);
-  atomicAdd(&S[c.i01].y, w01 * cpy);
-  atomicAdd(&S[c.i11].x, w11 * cpx);
-  atomicAdd(&S[c.i11].y, w11 * cpy);
+  const float2 v[4] = {make_float2(w00 * cpx, w00 * cpy), make_float2(w10 * cpx, w10 * cpy),
+                       make_float2(w01 * cpx, w01 * cpy), make_float2(w11 * cpx, w11 * cpy)};
+  add_to_cells(S, c.i00, c.i10, c.i01, c.i11, v);
+}
+
+__device__ __forceinline__ float sqrt_approx(float a) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
 }
 
 // Four particles that lie in one cell without sharing x and y exactly: a beamlet's
 // mirrored members once their energies, and with them their transverse steps, differ in
 // the last bits. Each particle's own weights and phasor are summed in registers, then
 // one set of eight atomics (exact up to FP32 summation order). Returns false, having
-// deposited nothing, unless all four lie inside the grid in the same cell.
+// deposited nothing, unless all four lie inside the grid in the same cell. The cells are
+// compared as floats and converted once; dx, dy and the gradients drop out of a centred
+// undulator's factor.
 __device__ __forceinline__ bool deposit_cell4(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                              int ng, const float *x, const float *y, const long long *th,
+                                              Grid ng, const float *x, const float *y, const long long *th,
                                               const float *dgam) {
-  CellF c;
-  if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x[0], y[0], c)) return false;
-#pragma unroll
-  for (int m = 1; m < 4; m++) {
-    CellF cm;
-    if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x[m], y[m], cm) || cm.i00 != c.i00) return false;
-  }
-  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const float gm = fs.gridmax, dg = fs.dgrid;
+  float wx[4], wy[4];
+  const float fx = floorf((x[0] + gm) / dg), fy = floorf((y[0] + gm) / dg);
+  bool same = true;
 #pragma unroll
   for (int m = 0; m < 4; m++) {
-    CellF cm;
-    ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x[m], y[m], cm);
-    const float dx = x[m] - sc.ax, dy = y[m] - sc.ay;
-    const float faw2 = 1.f + sc.kx * dx * dx + sc.ky * dy * dy + 2.f * (sc.gradx * dx + sc.grady * dy);
-    const float part = sqrtf(faw2) * scl / ((float)sc.gammaref + dgam[m]);
+    const float tx = (x[m] + gm) / dg, ty = (y[m] + gm) / dg;
+    same = same && fabsf(x[m]) < gm && fabsf(y[m]) < gm && floorf(tx) == fx && floorf(ty) == fy;
+    wx[m] = 1.f + fx - tx;
+    wy[m] = 1.f + fy - ty;
+  }
+  if (!same) return false;
+  const float g0 = (float)sc.gammaref;
+  float2 v00 = make_float2(0.f, 0.f), v10 = v00, v01 = v00, v11 = v00;
+#pragma unroll
+  for (int m = 0; m < 4; m++) {
+    float faw2;
+    if (sc.centred) {
+      faw2 = fmaf(sc.kx * x[m], x[m], fmaf(sc.ky * y[m], y[m], 1.f));
+    } else {
+      const float dx = x[m] - sc.ax, dy = y[m] - sc.ay;
+      faw2 = 1.f + sc.kx * dx * dx + sc.ky * dy * dy + 2.f * (sc.gradx * dx + sc.grady * dy);
+    }
+    const float part = sqrt_approx(faw2) * scl * rcp_approx(g0 + dgam[m]);
     float sn, co;
     __sincosf(phase_of(th[m], (unsigned)fs.harm), &sn, &co);
-    const float cpx = sn * part, cpy = co * part;
-    const float w00 = cm.wx * cm.wy, w10 = (1.f - cm.wx) * cm.wy, w01 = cm.wx * (1.f - cm.wy),
-                w11 = (1.f - cm.wx) * (1.f - cm.wy);
-    v[0] += w00 * cpx; v[1] += w00 * cpy; v[2] += w10 * cpx; v[3] += w10 * cpy;
-    v[4] += w01 * cpx; v[5] += w01 * cpy; v[6] += w11 * cpx; v[7] += w11 * cpy;
+    const float2 cp = make_float2(sn * part, co * part);
+    const float ux = 1.f - wx[m], uy = 1.f - wy[m];
+    const float2 a = make_float2(wy[m] * cp.x, wy[m] * cp.y), b = make_float2(uy * cp.x, uy * cp.y);
+    v00 = make_float2(fmaf(wx[m], a.x, v00.x), fmaf(wx[m], a.y, v00.y));
+    v10 = make_float2(fmaf(ux, a.x, v10.x), fmaf(ux, a.y, v10.y));
+    v01 = make_float2(fmaf(wx[m], b.x, v01.x), fmaf(wx[m], b.y, v01.y));
+    v11 = make_float2(fmaf(ux, b.x, v11.x), fmaf(ux, b.y, v11.y));
   }
-  atomicAdd(&S[c.i00].x, v[0]);
-  atomicAdd(&S[c.i00].y, v[1]);
-  atomicAdd(&S[c.i10].x, v[2]);
-  atomicAdd(&S[c.i10].y, v[3]);
-  atomicAdd(&S[c.i01].x, v[4]);
-  atomicAdd(&S[c.i01].y, v[5]);
-  atomicAdd(&S[c.i11].x, v[6]);
-  atomicAdd(&S[c.i11].y, v[7]);
+  const int ix = min((int)fx, ng.ng - 1), iy = min((int)fy, ng.ng - 1);
+  const int i = ix + iy * ng.st, ex = ix + 1 < ng.ng ? 1 : 0, ey = iy + 1 < ng.ng ? ng.st : 0;
+  const float2 v[4] = {v00, v10, v01, v11};
+  add_to_cells(S, i, i + ex, i + ey, i + ey + ex, v);
   return true;
 }
 
@@ -958,38 +989,48 @@ __device__ __forceinline__ bool deposit_cell4(const StepConstF &sc, const FieldS
 // phasors, pairs that share x and y like the first, anything else particle by particle.
 // No warp-level exchange is needed, and the loads are 16-byte vectors. Needs
 // npart % 4 == 0.
-__device__ __forceinline__ void deposit_quads(const StepConstF &sc, const FieldStepF &fs, const PtrsF &p,
-                                              float2 *S, int is, int np, int ng) {
-  const float scl = fs.dep_scl * (float)p.current[is];
-  const size_t base = (size_t)is * np;
-  const float4 *X = reinterpret_cast<const float4 *>(p.x + base);
-  const float4 *Y = reinterpret_cast<const float4 *>(p.y + base);
-  const float4 *G = reinterpret_cast<const float4 *>(p.dg + base);
+// Four consecutive particles (16-byte vectors), as loaded.
+struct Quad {
+  float4 x, y, g;
+  longlong2 t01, t23;
+};
+__device__ __forceinline__ Quad load_quad(const PtrsF &p, size_t base, int q) {
   const longlong2 *T = reinterpret_cast<const longlong2 *>(p.theta + base);
-  for (int q = threadIdx.x; q < (np >> 2); q += blockDim.x) {
-    const float4 x = X[q], y = Y[q], g = G[q];
-    const longlong2 t01 = T[2 * q], t23 = T[2 * q + 1];
-    const long long th[4] = {t01.x, t01.y, t23.x, t23.y};
-    const float dg[4] = {g.x, g.y, g.z, g.w};
-    const bool p01 = x.x == x.y && y.x == y.y, p23 = x.z == x.w && y.z == y.w;
-    const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
-    if (p01 && p23 && x.x == x.z && y.x == y.z) {
-      deposit_group<4>(sc, fs, scl, S, ng, x.x, y.x, th, dg);
-    } else if (!deposit_cell4(sc, fs, scl, S, ng, xs, ys, th, dg)) {
-      if (p01) {
-        deposit_group<2>(sc, fs, scl, S, ng, x.x, y.x, th, dg);
-      } else {
-        deposit_one(sc, fs, scl, S, ng, x.x, y.x, th[0], dg[0]);
-        deposit_one(sc, fs, scl, S, ng, x.y, y.y, th[1], dg[1]);
-      }
-      if (p23) {
-        deposit_group<2>(sc, fs, scl, S, ng, x.z, y.z, th + 2, dg + 2);
-      } else {
-        deposit_one(sc, fs, scl, S, ng, x.z, y.z, th[2], dg[2]);
-        deposit_one(sc, fs, scl, S, ng, x.w, y.w, th[3], dg[3]);
-      }
+  return Quad{reinterpret_cast<const float4 *>(p.x + base)[q], reinterpret_cast<const float4 *>(p.y + base)[q],
+              reinterpret_cast<const float4 *>(p.dg + base)[q], T[2 * q], T[2 * q + 1]};
+}
+__device__ __forceinline__ void deposit_quad(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S, Grid ng,
+                                             const Quad &v) {
+  const float4 &x = v.x, &y = v.y, &g = v.g;
+  const long long th[4] = {v.t01.x, v.t01.y, v.t23.x, v.t23.y};
+  const float dg[4] = {g.x, g.y, g.z, g.w};
+  const bool p01 = x.x == x.y && y.x == y.y, p23 = x.z == x.w && y.z == y.w;
+  const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+  // members that share x and y are deposited once where the whole warp's do (else both paths
+  // would run, and the one for members in one cell gives them the same value)
+  const bool equal = p01 && p23 && x.x == x.z && y.x == y.z;
+  if (__all_sync(__activemask(), equal)) {
+    deposit_group<4>(sc, fs, scl, S, ng, x.x, y.x, th, dg);
+  } else if (!deposit_cell4(sc, fs, scl, S, ng, xs, ys, th, dg)) {
+    if (p01) {
+      deposit_group<2>(sc, fs, scl, S, ng, x.x, y.x, th, dg);
+    } else {
+      deposit_one(sc, fs, scl, S, ng, x.x, y.x, th[0], dg[0]);
+      deposit_one(sc, fs, scl, S, ng, x.y, y.y, th[1], dg[1]);
+    }
+    if (p23) {
+      deposit_group<2>(sc, fs, scl, S, ng, x.z, y.z, th + 2, dg + 2);
+    } else {
+      deposit_one(sc, fs, scl, S, ng, x.z, y.z, th[2], dg[2]);
+      deposit_one(sc, fs, scl, S, ng, x.w, y.w, th[3], dg[3]);
     }
   }
+}
+__device__ __forceinline__ void deposit_quads(const StepConstF &sc, const FieldStepF &fs, const PtrsF &p,
+                                              float2 *S, int is, int np, Grid ng) {
+  const float scl = fs.dep_scl * (float)p.current[is];
+  const size_t base = (size_t)is * np;
+  for (int q = threadIdx.x; q < (np >> 2); q += blockDim.x) deposit_quad(sc, fs, scl, S, ng, load_quad(p, base, q));
 }
 
 
@@ -1368,6 +1409,8 @@ __global__ void __launch_bounds__(kFusedMaxThreads, 1)
   }
   if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
+
+#include "field_tm.cuh"
 
 // ---- the whole step of one slice in one CTA: push, deposition and ADI -----------
 //
@@ -2409,6 +2452,64 @@ int fused_threads(int ngrid, int threads) {
   if (threads > kFusedMaxThreads) threads = kFusedMaxThreads;
   return threads;
 }
+namespace {
+// Whether the field kernel with S1 in tensor memory takes a step: its solves are
+// segmented, a segment's S1 fits a thread's words and the slice with its odd row stride fits
+// shared memory (ngrid 165 with the field record's scratch).
+bool field_tm_fits(int ngrid, int threads, int W) {
+  return tm_shape(ngrid, threads, W).threads > 0 && tm_smem_bytes(ngrid, W, threads) <= 227u * 1024u - 16;
+}
+int field_sms() {
+  static std::atomic<int> sms[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int n = dev < 64 ? sms[dev].load() : 0;
+  if (!n) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 152;
+    if (dev < 64) sms[dev].store(n);
+  }
+  return n;
+}
+// CTAs of k_field_tm_f an SM holds: one, or two where the shared memory and the tensor memory
+// of two fit (its 80 registers a thread allow two of 384)
+int field_tm_per_sm(size_t smem, int threads) {
+  return threads <= 384 && 2 * (smem + 1024 + 16) <= 228 * 1024 ? 2 : 1;
+}
+template <int LA, bool REC>
+void launch_field_tm(const Launch &L, const StepConstF &sc, int k, const PtrsF &p, void *field, const void *coef,
+                     const void *pow, int ns, int np, int ngrid, int deposit, int threads, double *dfield) {
+  static std::atomic<unsigned long long> configured{0};  // one bit per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !(configured.load() & (1ull << dev))) {
+    cudaFuncSetAttribute(k_field_tm_f<LA, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 16);
+    if (dev < 64) configured.fetch_or(1ull << dev);
+  }
+  const int W = sc.f[k].tw;
+  const TmShape t = tm_shape(ngrid, threads, W);
+  threads = t.threads;
+  const size_t smem = tm_smem_bytes(ngrid, W, threads);
+  k_field_tm_f<LA, REC><<<std::min(ns, field_sms() * field_tm_per_sm(smem, threads)), threads, smem,
+                          (cudaStream_t)L.stream>>>(sc, k, p, (float2 *)field, (const float2 *)coef, (const float2 *)pow,
+                                                    ns, np, ngrid, deposit, t.nseg, W, t.words, t.cols, dfield);
+}
+}  // namespace
+
+// CTA size of the field kernel where none is set: all the registers allow, or two CTAs of 384
+// threads where two slices fit an SM and the window has more slices than SMs (one CTA's
+// memory phases then run beside the other's solves): 2000 x 4096, 117^2 197 us (one CTA of 768
+// 251); 700 x 8192, 101^2 85 (95); 200 x 4096, 101^2 30 (34).
+int field_threads_auto(int ngrid, int ns, int W) {
+  if (!field_tm_fits(ngrid, kTmMaxThreads, W)) return 512;
+  const int two = (2 * ngrid + 31) / 32 * 32 > 384 ? 0 : 384;
+  if (two && ns > field_sms() && field_tm_fits(ngrid, two, W) && field_tm_per_sm(tm_smem_bytes(ngrid, W, two), two) == 2)
+    return two;
+  return kTmMaxThreads;
+}
+bool field_record_fits(int ngrid, int threads, int W, int nharm) {
+  return field_tm_fits(ngrid, fused_threads(ngrid, threads), W) || fused_diag_fits(ngrid, threads, nharm);
+}
+
 bool fused_diag_fits(int ngrid, int threads, int nharm) {
   return nharm <= kFusedDiagHarm && fused_diag_smem_bytes(ngrid, fused_threads(ngrid, threads)) <= 227u * 1024u;
 }
@@ -2420,10 +2521,18 @@ int fused_max_ngrid() {
 }
 
 void launch_field_fused_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b,
-                              void *field, const void *coef, int ns, int np, int ngrid, int deposit,
+                              void *field, const void *coef, const void *pow, int ns, int np, int ngrid, int deposit,
                               int threads, double *dbeam, double *dfield, int nharm, double gref) {
   static std::atomic<unsigned long long> configured{0};  // one bit per device
   threads = fused_threads(ngrid, threads);
+  const int W = sc.f[k].tw;
+  if (!dbeam && field_tm_fits(ngrid, threads, W)) {
+    PtrsF p = make_ptrs_f(b, nullptr, nullptr, 0);
+    const auto launch = W <= 9 ? (dfield ? launch_field_tm<8, true> : launch_field_tm<8, false>)
+                               : (dfield ? launch_field_tm<kTmLook, true> : launch_field_tm<kTmLook, false>);
+    launch(L, sc, k, p, field, coef, pow, ns, np, ngrid, deposit, threads, dfield);
+    return;
+  }
   size_t smem = (dbeam || dfield) ? fused_diag_smem_bytes(ngrid, threads) : fused_smem_bytes(ngrid);
   int dev = 0;
   cudaGetDevice(&dev);
