@@ -1664,15 +1664,35 @@ __device__ __forceinline__ void block_reduce_all(const KahanF *s, const float *m
 // taken about gammaref: sum g = N gref + sum dg and sum g^2 = N gref^2 + 2 gref sum dg
 // + sum dg^2, without the cancellation of squaring g itself. NH: compile-time bound on
 // the number of harmonics (the arrays stay in registers).
+//
+// Memory bounds it (28 bytes a particle against ~100 instructions), so what matters is
+// how many bytes are on their way. Four particles at a time are copied to shared memory in
+// 16-byte pieces, kDiagAhead groups ahead of the arithmetic; every thread reads back what
+// it copied itself, so no barrier is needed. The arrays of a slice start at any multiple
+// of np elements: the particles in front of the first one on a 16-byte boundary, and those
+// behind the last whole group, are read on their own.
+constexpr int kDiagAhead = 2, kDiagBlock = 128;
+__device__ __forceinline__ void copy16(void *s, const void *g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(s)), "l"(g)
+               : "memory");
+}
+
 template <int BS, int NH>
 __global__ void __launch_bounds__(BS) k_diag_beam_f(PtrsF p, double gref, int np, int nharm, double *out) {
   constexpr int NSUM = kBeamSums + 2 * NH;
-  __shared__ double sh[(BS / 32) * (NSUM + 10)];
+  // [stage][x, y, dg, px, py, theta, theta][thread]; the reductions follow in the same
+  // place once the last group has been read
+  constexpr int kStages = kDiagAhead + 1, kRed = (BS / 32) * (NSUM + 10);
+  static_assert(kRed * sizeof(double) <= sizeof(float4) * kStages * 7 * BS, "");
+  __shared__ float4 ring[kStages][7][BS];
   __shared__ double res[NSUM + 10];
-  const int is = blockIdx.x;
+  double *sh = reinterpret_cast<double *>(ring);
+  const int is = blockIdx.x, tid = threadIdx.x;
   const size_t base = (size_t)is * np;
   const int cnt = slice_np_f(p, is, np);
   const int nh = min(nharm, NH);
+  const int head = min((int)((4 - (base & 3)) & 3), cnt), ngrp = (cnt - head) >> 2;
+  const size_t o4 = base + head;
   // dg, dg^2, x, x^2, y, y^2, px, px^2, py, py^2, x px, y py, then (Re, Im) b_h
   KahanF c[NSUM];
   float mn[5], mx[5];  // x, px, y, py, dg
@@ -1681,11 +1701,7 @@ __global__ void __launch_bounds__(BS) k_diag_beam_f(PtrsF p, double gref, int np
     mn[k] = INFINITY;
     mx[k] = -INFINITY;
   }
-#pragma unroll 4
-  for (int ip = threadIdx.x; ip < cnt; ip += BS) {
-    const float x = p.x[base + ip], y = p.y[base + ip], dg = p.dg[base + ip];
-    const float px = p.px[base + ip], py = p.py[base + ip];
-    const long long th = p.theta[base + ip];
+  auto add = [&](float x, float y, float dg, float px, float py, unsigned th) {
     c[0].add(dg); c[1].add(dg * dg); c[2].add(x); c[3].add(x * x); c[4].add(y); c[5].add(y * y);
     c[6].add(px); c[7].add(px * px); c[8].add(py); c[9].add(py * py); c[10].add(x * px); c[11].add(y * py);
     mn[0] = fminf(mn[0], x); mx[0] = fmaxf(mx[0], x);
@@ -1702,18 +1718,53 @@ __global__ void __launch_bounds__(BS) k_diag_beam_f(PtrsF p, double gref, int np
         c[kBeamSums + 2 * h + 1].add(sn);
       }
     }
+  };
+  auto fetch = [&](int st, int i) {
+    if (i < ngrp) {
+      const size_t o = o4 + 4 * (size_t)i;
+      copy16(&ring[st][0][tid], p.x + o);
+      copy16(&ring[st][1][tid], p.y + o);
+      copy16(&ring[st][2][tid], p.dg + o);
+      copy16(&ring[st][3][tid], p.px + o);
+      copy16(&ring[st][4][tid], p.py + o);
+      copy16(&ring[st][5][tid], p.theta + o);
+      copy16(&ring[st][6][tid], p.theta + o + 2);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int q = 0; q < kDiagAhead; q++) fetch(q, tid + q * BS);
+  if (tid < cnt - 4 * ngrp) {  // at most six particles outside the groups
+    const size_t o = base + (tid < head ? tid : tid + 4 * ngrp);
+    add(p.x[o], p.y[o], p.dg[o], p.px[o], p.py[o], (unsigned)p.theta[o]);
   }
+  int st = 0;
+  for (int i = tid; i < ngrp; i += BS) {
+    // the stage read one group ago takes the group kDiagAhead ahead
+    fetch(st == 0 ? kStages - 1 : st - 1, i + kDiagAhead * BS);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDiagAhead) : "memory");
+    const float4 x = ring[st][0][tid], y = ring[st][1][tid], dg = ring[st][2][tid], px = ring[st][3][tid],
+                 py = ring[st][4][tid], t0 = ring[st][5][tid], t1 = ring[st][6][tid];
+    add(x.x, y.x, dg.x, px.x, py.x, __float_as_uint(t0.x));  // the low word holds the phase
+    add(x.y, y.y, dg.y, px.y, py.y, __float_as_uint(t0.z));
+    add(x.z, y.z, dg.z, px.z, py.z, __float_as_uint(t1.x));
+    add(x.w, y.w, dg.w, px.w, py.w, __float_as_uint(t1.z));
+    st = st + 1 < kStages ? st + 1 : 0;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
   block_reduce_all<BS, NSUM, 5>(c, mn, mx, sh, res);
   __syncthreads();
   const int w = beam_diag_width(nharm);
   double *o = out + (size_t)is * w;
-  const int k = threadIdx.x;
   const double n = (double)cnt;
-  if (k == 0) o[0] = n * gref + res[0];
-  if (k == 1) o[1] = n * gref * gref + 2.0 * gref * res[0] + res[1];
-  if (k >= 2 && k < kBeamSums) o[k] = res[k];
-  if (k >= kBeamSums && k < kBeamSums + 2 * nh) o[kBeamMinMax + k] = res[k];  // bunching after min/max
-  if (k < 10) o[kBeamSums + k] = (k >= 8 ? gref : 0.0) + res[NSUM + k];
+  for (int k = tid; k < NSUM || k < 10; k += BS) {
+    if (k == 0) o[0] = n * gref + res[0];
+    if (k == 1) o[1] = n * gref * gref + 2.0 * gref * res[0] + res[1];
+    if (k >= 2 && k < kBeamSums) o[k] = res[k];
+    if (k >= kBeamSums && k < kBeamSums + 2 * nh) o[kBeamMinMax + k] = res[k];  // bunching after min/max
+    if (k < 10) o[kBeamSums + k] = (k >= 8 ? gref : 0.0) + res[NSUM + k];
+  }
 }
 
 // Per-slice field sums of the mixed form (layout of k_diag_field): a flat walk over
@@ -2426,13 +2477,13 @@ void launch_diag_beam_mixed(const Launch &L, const DeviceBeam &b, double gammare
   PtrsF p = make_ptrs_f(b, nullptr, nullptr, 0);
   cudaStream_t s = (cudaStream_t)L.stream;
   if (nharm <= 1)
-    k_diag_beam_f<256, 1><<<ns, 256, 0, s>>>(p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, 1><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
   else if (nharm <= 3)
-    k_diag_beam_f<256, 3><<<ns, 256, 0, s>>>(p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, 3><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
   else if (nharm <= 5)
-    k_diag_beam_f<256, 5><<<ns, 256, 0, s>>>(p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, 5><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
   else
-    k_diag_beam_f<256, G4GPU_MAX_HARM><<<ns, 256, 0, s>>>(p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, G4GPU_MAX_HARM><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
 }
 
 void launch_diag_field_mixed(const Launch &L, const void *field, int ns, int ngrid, double *out) {
