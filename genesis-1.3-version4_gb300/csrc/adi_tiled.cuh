@@ -143,8 +143,12 @@ __global__ void __launch_bounds__(BS) k_adi_xt(const typename P::G *__restrict__
   }
   for (int e = threadIdx.x; e < nr * ng; e += BS) Sb[e] = s ? P::ld(s + (size_t)r0 * ng + e) : P::zero();
   __syncthreads();
-  // r1 on rows 1..nr of the tile: lines are the columns, elements the rows
-  stencil_seg<P>(T + ng, ng, 1, ng, nr, max(1, min(BS / ng, 8)), Sb, 1, ng, cstep, r0, ng);
+  // r1 on rows 1..nr of the tile: lines are the columns (as many at a time as there are
+  // threads), elements the rows
+  for (int c0 = 0; c0 < ng; c0 += BS) {
+    const int nc = min(BS, ng - c0);
+    stencil_seg<P>(T + ng + c0, nc, 1, ng, nr, max(1, min(BS / nc, 8)), Sb + c0, 1, ng, cstep, r0, ng);
+  }
   // solve along the rows
   const int nseg = max(1, min(BS / nr, 32));
   thomas_seg<P>(T + ng, nr, ng, 1, ng, nseg, W, cf);
