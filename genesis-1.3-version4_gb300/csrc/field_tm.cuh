@@ -126,6 +126,14 @@ __device__ __forceinline__ void solve_window(int b, int e, int nchunk, float cs,
   }
 }
 
+// Adds the carries over the ends of rows [b, e) of a line
+__device__ __forceinline__ void add_carries(float2 *L, const float2 *PW, int b, int e, int W, float2 lc, float2 rc) {
+  for (int j = 0; j < W; j++) {
+    L[b + j] = add_cmulf(L[b + j], PW[j], lc);
+    L[e - 1 - j] = add_cmulf(L[e - 1 - j], PW[j], rc);
+  }
+}
+
 // Prefetches [p, p + bytes) of an array into L2, rounded inwards to 16 bytes.
 __device__ __forceinline__ void l2_prefetch(const void *p, size_t bytes) {
   const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
@@ -151,6 +159,120 @@ __device__ __forceinline__ float warp_sums8(float (&v)[8]) {
   float s = v[0];
   s += __shfl_xor_sync(0xffffffffu, s, 2);
   return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
+
+// S1 = (I + c Dy) u of rows [b, e) of a column: into S (rows of st) and, eight rows at a
+// time, into this thread's tensor memory. u and S point at the band's first row; `above`: the
+// grid goes on above row b; `below`: rows of the grid from the band's first on. Rows outside
+// the grid are zeros, which gives the one-sided differences at its edges.
+__device__ __forceinline__ void tm_stencil_cols(const float2 *u, float2 *S, uint32_t tm, int ng, int st, int line,
+                                                bool act, int b, int e, int nq, bool above, int below, float cs) {
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 prev = above ? u[(b - 1) * ng + line] : zero;
+  float2 cur = act ? u[b * ng + line] : zero;
+#pragma unroll 1
+  for (int q = 0; q < nq; q++) {
+    float2 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int r = b + 8 * q + j;
+      v[j] = r < e && r + 1 < below ? u[(r + 1) * ng + line] : zero;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const float2 nx = v[j];
+      v[j] = stencil(cs, cur, make_float2(nx.x - 2.f * cur.x + prev.x, nx.y - 2.f * cur.y + prev.y));
+      prev = cur;
+      cur = nx;
+      const int r = b + 8 * q + j;
+      if (r < e) S[r * st + line] = v[j];
+    }
+    __syncwarp();
+    tm_put8(tm + 16 * q, v);
+  }
+}
+
+// The column solve of the second right-hand side 2 u' - S1 in place, zeros outside [b, e).
+template <int LA>
+__device__ __forceinline__ void tm_solve_cols(float2 *L, uint32_t tm, int st, int b, int e, int nq, int nchunk,
+                                              float cs, float2 cb, float2 kap) {
+  const float2 zero = make_float2(0.f, 0.f);
+  solve_window<LA>(
+      b, e, nchunk, cs, cb, kap,
+      [&](int r, float2 *v) {
+        const int q = (r - b) >> 3;
+        if (q < nq) {
+          float2 s1[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) v[j] = r + j < e ? L[(r + j) * st] : zero;
+          __syncwarp();
+          tm_get8(tm + 16 * q, s1);
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+            v[j] = r + j < e ? make_float2(2.f * v[j].x - s1[j].x, 2.f * v[j].y - s1[j].y) : zero;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; j++) v[j] = zero;
+        }
+      },
+      [&](int r, float2 x) { L[r * st] = x; });
+}
+
+// Writes rows [b, e) of a column with the carries lc and rc over its ends to u, and sums the
+// field record's terms (global row of row 0: r0).
+template <bool REC>
+__device__ __forceinline__ void tm_write_cols(float2 *u, const float2 *L, const float2 *PW, int ng, int st, int line,
+                                              int b, int e, int W, float2 lc, float2 rc, int r0, float (&f)[8]) {
+  const int lo = b + W, hi = e - W;  // [lo, hi): no carry
+  const float shift = -0.5f * (float)(ng - 1);
+  float dy = (float)(r0 + b) + shift;
+  auto put = [&](int r, float2 x) {
+    u[r * ng + line] = x;
+    if constexpr (REC) {
+      const float w = fmaf(x.x, x.x, x.y * x.y), t = dy * w;
+      f[0] += w;
+      f[3] += t;
+      f[4] = fmaf(dy, t, f[4]);
+      f[5] += x.x;
+      f[6] += x.y;
+      dy += 1.f;
+    }
+  };
+  const int mid = min(lo, e);
+#pragma unroll 4
+  for (int r = b; r < mid; r++) {
+    float2 x = add_cmulf(L[r * st], PW[r - b], lc);
+    if (r >= hi) x = add_cmulf(x, PW[e - 1 - r], rc);
+    put(r, x);
+  }
+#pragma unroll 4
+  for (int r = mid; r < hi; r++) put(r, L[r * st]);
+#pragma unroll 4
+  for (int r = max(mid, hi); r < e; r++) put(r, add_cmulf(L[r * st], PW[e - 1 - r], rc));
+  if constexpr (REC) {
+    const float dx = (float)line + shift;
+    f[1] = dx * f[0];
+    f[2] = dx * f[1];
+  }
+}
+
+// The CTA's totals of the threads' record terms: emit(q, total) from the last warp, which
+// folds the warps' sums in FP64, four lanes a value, while the others go on. One barrier.
+template <class EM>
+__device__ __forceinline__ void tm_fold_record(float (&f)[8], double *red, EM emit) {
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const float v = warp_sums8(f);
+  if ((tid & 3) == 0 && (tid & 31) < 4 * kFieldSums) red[warp * kFieldSums + ((tid & 31) >> 2)] = (double)v;
+  __syncthreads();
+  if (warp == (int)(blockDim.x >> 5) - 1) {
+    const int k2 = (tid & 31) >> 2;
+    double t = 0;
+    if (k2 < kFieldSums)
+      for (int w = tid & 3; w < (int)(blockDim.x >> 5); w += 4) t += red[w * kFieldSums + k2];
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    if ((tid & 3) == 0 && k2 < kFieldSums) emit(k2, t);
+  }
 }
 
 // REC: the field record of every slice (k_diag_field_f's sums) is formed too.
@@ -202,32 +324,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
     const bool vec = deposit && (np & 3) == 0 && !p.count;
     Quad quad{};
     if (vec && tid < (np >> 2)) quad = load_quad(p, base, tid);
-    // S1 of the thread's rows of its column, eight rows' loads at a time; rows outside the
-    // grid are zeros, which gives the one-sided differences at the edges
-    {
-      float2 prev = left ? u[(b - 1) * ng + line] : zero;
-      float2 cur = act ? u[b * ng + line] : zero;
-#pragma unroll 1
-      for (int q = 0; q < nq; q++) {
-        float2 v[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int r = b + 8 * q + j;
-          v[j] = r < e && r + 1 < ng ? u[(r + 1) * ng + line] : zero;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const float2 nx = v[j];
-          v[j] = stencil(cs, cur, make_float2(nx.x - 2.f * cur.x + prev.x, nx.y - 2.f * cur.y + prev.y));
-          prev = cur;
-          cur = nx;
-          const int r = b + 8 * q + j;
-          if (r < e) S[r * st + line] = v[j];
-        }
-        __syncwarp();
-        tm_put8(tm + 16 * q, v);
-      }
-    }
+    tm_stencil_cols(u, S, tm, ng, st, line, act, b, e, nq, left, ng, cs);
     __syncwarp();
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     __syncthreads();
@@ -273,37 +370,14 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
         rc = carry(right, right ? L[e] : zero, L[e - 1]);
       }
       __syncthreads();
-      if (act)
-        for (int j = 0; j < W; j++) {
-          L[b + j] = add_cmulf(L[b + j], PW[j], lc);
-          L[e - 1 - j] = add_cmulf(L[e - 1 - j], PW[j], rc);
-        }
+      if (act) add_carries(L, PW, b, e, W, lc, rc);
     }
     __syncthreads();
     // columns: the second right-hand side 2 u' - S1, solved, then written with the
     // neighbours' carries (writing the rows without carries from the solve itself: 631 against
     // 640 us for 4096 slices of 151^2, 257 against 250 us for 2000 of 117^2)
     float2 *L = S + line;
-    const int lo = b + W, hi = e - W;  // [lo, hi): no carry
-    solve_window<LA>(
-        b, e, nchunk, cs, cb, kap,
-        [&](int r, float2 *v) {
-          const int q = (r - b) >> 3;
-          if (q < nq) {
-            float2 s1[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = r + j < e ? L[(r + j) * st] : zero;
-            __syncwarp();
-            tm_get8(tm + 16 * q, s1);
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-              v[j] = r + j < e ? make_float2(2.f * v[j].x - s1[j].x, 2.f * v[j].y - s1[j].y) : zero;
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = zero;
-          }
-        },
-        [&](int r, float2 x) { L[r * st] = x; });
+    tm_solve_cols<LA>(L, tm, st, b, e, nq, nchunk, cs, cb, kap);
     __syncthreads();
     float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     {
@@ -312,36 +386,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
         lc = carry(left, left ? L[(b - 1) * st] : zero, L[b * st]);
         rc = carry(right, right ? L[e * st] : zero, L[(e - 1) * st]);
       }
-      const float shift = -0.5f * (float)(ng - 1);
-      float dy = (float)b + shift;
-      auto put = [&](int r, float2 x) {
-        u[r * ng + line] = x;
-        if constexpr (REC) {
-          const float w = fmaf(x.x, x.x, x.y * x.y), t = dy * w;
-          f[0] += w;
-          f[3] += t;
-          f[4] = fmaf(dy, t, f[4]);
-          f[5] += x.x;
-          f[6] += x.y;
-          dy += 1.f;
-        }
-      };
-      const int mid = min(lo, e);
-#pragma unroll 4
-      for (int r = b; r < mid; r++) {
-        float2 x = add_cmulf(L[r * st], PW[r - b], lc);
-        if (r >= hi) x = add_cmulf(x, PW[e - 1 - r], rc);
-        put(r, x);
-      }
-#pragma unroll 4
-      for (int r = mid; r < hi; r++) put(r, L[r * st]);
-#pragma unroll 4
-      for (int r = max(mid, hi); r < e; r++) put(r, add_cmulf(L[r * st], PW[e - 1 - r], rc));
-      if constexpr (REC) {
-        const float dx = (float)line + shift;
-        f[1] = dx * f[0];
-        f[2] = dx * f[1];
-      }
+      tm_write_cols<REC>(u, L, PW, ng, st, line, b, e, W, lc, rc, 0, f);
     }
     if constexpr (REC) {
       double *o = dfield + (size_t)i * (kFieldSums + 2);
@@ -350,21 +395,210 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
         o[7] = v.x;
         o[8] = v.y;
       }
-      const float v = warp_sums8(f);
-      if ((tid & 3) == 0 && (tid & 31) < 4 * kFieldSums) red[warp * kFieldSums + ((tid & 31) >> 2)] = (double)v;
-      __syncthreads();
-      // the last warp folds the warps' sums in FP64, four lanes a value, while the others go on
-      if (warp == (int)(blockDim.x >> 5) - 1) {
-        const int k2 = (tid & 31) >> 2;
-        double t = 0;
-        if (k2 < kFieldSums)
-          for (int w = tid & 3; w < (int)(blockDim.x >> 5); w += 4) t += red[w * kFieldSums + k2];
-        t += __shfl_xor_sync(0xffffffffu, t, 1);
-        t += __shfl_xor_sync(0xffffffffu, t, 2);
-        if ((tid & 3) == 0 && k2 < kFieldSums) o[k2] = t;
-      }
+      tm_fold_record(f, red, [&](int q, double t) { o[q] = t; });
     } else {
       __syncthreads();
+    }
+  }
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(cols) : "memory");
+}
+
+// ---- the same step with a slice's rows split between the CTAs of a cluster ---------------
+//
+// For slices that do not fit one CTA's shared memory, and for windows of so few slices that
+// one CTA a slice leaves most SMs idle. CTA q of CL holds rows [q ng / CL, (q + 1) ng / CL) of
+// the slice, and the phases are those of k_field_tm_f on this band:
+//  * the column segments end at the band's rows; a segment next to the band's edge finds the
+//    neighbour's row there in its shared memory (one row of the band above and one of the
+//    band below is all that crosses), and the rows next to the band's that S1 needs in
+//    global memory, which nobody writes before every CTA has passed a cluster barrier;
+//  * every CTA reads all the slice's particles and deposits into its own rows (adding to a
+//    peer's shared memory instead took 2.8 times as long as one CTA's whole deposition; a
+//    list of the particles with a row in the band, made first, gained nothing: what the
+//    deposition of a band takes is the latency of its atomics, not the lanes left idle);
+//  * rows are solved within the CTA, in more segments the fewer rows it has.
+// One slice a cluster: the hardware hands out the next, whose field and particles are
+// prefetched into L2. Two CTAs of clusters never share an SM (kClusterMinSmem): the second
+// would wait for tensor memory while its peers wait for it, and the first's peers likewise.
+// Measured against k_field_band_f and k_field_tm_f: at field_cluster (kernels_mixed.cu). Of a band's
+// 63 thousand cycles (255^2, CL 3) S1 takes 13, the deposition 5 to 19 (the middle band holds the
+// beam), the columns 11, the rows 10, the last pass 7; of the 32 of 151^2 with CL 4 the deposition
+// up to 10, S1, rows and columns 4 to 6 each.
+constexpr size_t kClusterMinSmem = 116u * 1024u;
+constexpr int kMaxCluster = 8;
+struct ClShape {
+  int cl, threads, nseg, words, cols;
+  size_t smem;
+};
+// The shape for clusters of cl CTAs (cl 0: it does not fit). Every segment is longer than W.
+inline ClShape cl_shape(int ng, int W, int cl) {
+  const int nmin = ng / cl, nmax = (ng + cl - 1) / cl;
+  const ClShape none{0, 0, 0, 0, 0, 0};
+  if (W < 1 || W > kTmLook + 1 || nmin < W + 1 || ng > kTmMaxThreads) return none;
+  ClShape t{cl, 0, std::max(1, std::min(std::min(kTmMaxThreads / ng, 8), nmin / (W + 1))), 0, 32, 0};
+  // as many threads as the tensor memory has words for
+  for (int need = 0;; t.nseg--) {
+    if (t.nseg < 1) return none;
+    const int len = (nmax + t.nseg - 1) / t.nseg, least = (ng * t.nseg + 31) / 32 * 32;
+    t.words = (len + 7) / 8 * 16;
+    t.threads = kTmMaxThreads;
+    auto fits = [&] { return (need = (t.threads / 32 + 3) / 4 * t.words) <= 512; };
+    while (!fits() && t.threads > least) t.threads -= 32;
+    if (t.threads < least || need > 512) continue;
+    while (t.cols < need) t.cols *= 2;
+    break;
+  }
+  t.smem = (((size_t)W + 1) / 2 * 2 + ((size_t)nmax * (ng | 1) + 1) / 2 * 2) * sizeof(float2) +
+           (size_t)(t.threads / 32 + 1 + kMaxCluster) * kFieldSums * sizeof(double);
+  if (t.smem > 227u * 1024u - 16) return none;
+  t.smem = std::max(t.smem, kClusterMinSmem);
+  return t;
+}
+
+template <int LA, bool REC>
+__global__ void __launch_bounds__(kTmMaxThreads, 1)
+    k_field_cl_f(StepConstF sc, int k, PtrsF p, float2 *__restrict__ field, const float2 *__restrict__ coef,
+                 const float2 *__restrict__ pows, int ns, int np, int ng, int deposit, int nseg, int W, int words,
+                 int cols, int ahead, double *dfield) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t tm_base;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int CL = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int tid = threadIdx.x, warp = tid >> 5, st = ng | 1;
+  const FieldStepF &fs = sc.f[k];
+  const int r0 = rank * ng / CL, nrow = (rank + 1) * ng / CL - r0, nmax = (ng + CL - 1) / CL;
+  float2 *PW = reinterpret_cast<float2 *>(smem_raw);  // kappa^{j+1}
+  float2 *S = PW + (W + 1) / 2 * 2;
+  double *red = reinterpret_cast<double *>(S + (nmax * st + 1) / 2 * 2);
+  double *parts = red + (size_t)(blockDim.x / 32 + 1) * kFieldSums;  // [CTA][kFieldSums], used in CTA 0
+  if (warp == 0) {
+    const uint32_t sadr = (uint32_t)__cvta_generic_to_shared(&tm_base);
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sadr), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  for (int t = tid; t < W; t += blockDim.x) PW[t] = pows[t];
+  const int is = blockIdx.x / CL, i = ring_slot(is, fs.first, ns);
+  float2 *u = field + (size_t)i * ng * ng + (size_t)r0 * ng;  // the band
+  const size_t base = (size_t)is * np;
+  const bool vec = deposit && (np & 3) == 0 && !p.count;
+  // the first particles' loads in flight while S1 is formed
+  Quad quad{};
+  if (vec && tid < (np >> 2)) quad = load_quad(p, base, tid);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tm = tm_base + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * words);
+
+  // column and segment of the thread
+  const int line = tid % ng, seg = tid / ng;
+  const bool act = seg < nseg;
+  const int b = act ? seg * nrow / nseg : 0, e = act ? (seg + 1) * nrow / nseg : 0;
+  const bool left = act && r0 + b > 0, right = act && r0 + e < ng;
+  const int nq = words >> 4;  // batches of eight rows
+  const float cs = fs.cstep;
+  const float2 cb = coef[2 * ng - 1], kap = PW[0], zero = make_float2(0.f, 0.f);
+  auto carry = [&](bool inner, float2 other, float2 own) { return inner ? other : cmulf(make_float2(-kap.x, -kap.y), own); };
+
+  const bool cols_on = __any_sync(0xffffffffu, act);  // warps without a column have nothing to issue
+  if (cols_on) {
+    tm_stencil_cols(u, S, tm, ng, st, line, act, b, e, nq, left, ng - r0, cs);
+    __syncwarp();
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  if (deposit) {
+    const Band g(ng, st, r0, nrow);
+    if (vec) {
+      const float scl = fs.dep_scl * (float)p.current[is];
+#pragma unroll 1
+      for (int q = tid; q < (np >> 2); q += blockDim.x) {
+        const Quad v = quad;
+        if (q + (int)blockDim.x < (np >> 2)) quad = load_quad(p, base, q + blockDim.x);
+        deposit_quad(sc, fs, scl, S, g, v);
+      }
+    } else {
+      deposit_smem(sc, fs, p, S, is, np, g);
+    }
+    __syncthreads();
+  }
+  // a later slice's field and particles on their way to L2
+  if (rank == 0 && tid < 5 && is + ahead < ns) {
+    const int nx = is + ahead;
+    const size_t o = (size_t)nx * np;
+    const size_t n = p.count ? min(p.count[nx], np) : np;
+    if (tid == 0) l2_prefetch(field + (size_t)ring_slot(nx, fs.first, ns) * ng * ng, (size_t)ng * ng * 8);
+    if (deposit && tid == 1) l2_prefetch(p.x + o, n * 4);
+    if (deposit && tid == 2) l2_prefetch(p.y + o, n * 4);
+    if (deposit && tid == 3) l2_prefetch(p.dg + o, n * 4);
+    if (deposit && tid == 4) l2_prefetch(p.theta + o, n * 8);
+  }
+  {  // the band's rows
+    const int nsr = min((int)blockDim.x / nrow, ng / (W + 1));
+    const int row = tid % nrow, sr = tid / nrow;
+    const bool on = sr < nsr;
+    const int rb = on ? sr * ng / nsr : 0, re = on ? (sr + 1) * ng / nsr : 0;
+    float2 *L = S + row * st;
+    if (__any_sync(0xffffffffu, on)) solve_window<LA>(
+        rb, re, ((ng + nsr - 1) / nsr + kTmChunk - 1) / kTmChunk, cs, cb, kap,
+        [&](int r, float2 *v) {
+#pragma unroll
+          for (int j = 0; j < kTmChunk; j++) v[j] = r + j < re ? L[r + j] : zero;
+        },
+        [&](int r, float2 x) { L[r] = x; });
+    __syncthreads();
+    float2 lc = zero, rc = zero;
+    if (on) {
+      const bool hl = sr > 0, hr = sr + 1 < nsr;
+      lc = carry(hl, hl ? L[rb - 1] : zero, L[rb]);
+      rc = carry(hr, hr ? L[re] : zero, L[re - 1]);
+    }
+    __syncthreads();
+    if (on) add_carries(L, PW, rb, re, W, lc, rc);
+  }
+  __syncthreads();
+  float2 *L = S + line;
+  if (cols_on) tm_solve_cols<LA>(L, tm, st, b, e, nq, ((nmax + nseg - 1) / nseg + kTmChunk - 1) / kTmChunk, cs, cb, kap);
+  cl.sync();  // the neighbours' edge rows are solved, and nobody reads u any more
+  float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  {
+    float2 lc = zero, rc = zero;
+    if (act) {
+      float2 above = zero, below = zero;
+      if (left) {
+        const int hi = (rank - 1) * ng / CL;  // first row of the band above
+        above = b > 0 ? L[(b - 1) * st] : cl.map_shared_rank(S, rank - 1)[(r0 - 1 - hi) * st + line];
+      }
+      if (right) below = e < nrow ? L[e * st] : cl.map_shared_rank(S, rank + 1)[line];
+      lc = carry(left, above, L[b * st]);
+      rc = carry(right, below, L[(e - 1) * st]);
+    }
+    // the peers' rows are read: the last barrier, which keeps a CTA's shared memory until then, does
+    // not wait for the field's writes (with the record it also brings the parts to CTA 0, below)
+    if constexpr (!REC) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    tm_write_cols<REC>(u, L, PW, ng, st, line, b, e, W, lc, rc, r0, f);
+  }
+  if constexpr (REC) {
+    double *o = dfield + (size_t)i * (kFieldSums + 2);
+    const int mid = ng / 2 - r0;
+    if (line == ng / 2 && b <= mid && mid < e) {  // the value on the axis
+      const float2 v = u[mid * ng + line];
+      o[7] = v.x;
+      o[8] = v.y;
+    }
+    double *to = cl.map_shared_rank(parts, 0) + rank * kFieldSums;
+    tm_fold_record(f, red, [&](int q, double t) { to[q] = t; });
+  }
+  if constexpr (!REC) {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  } else {
+    cl.sync();
+    if (rank == 0 && tid < kFieldSums) {
+      double t = 0;
+      for (int q = 0; q < CL; q++) t += parts[q * kFieldSums + tid];
+      dfield[(size_t)i * (kFieldSums + 2) + tid] = t;
     }
   }
   if (warp == 0)

@@ -1340,6 +1340,13 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       band_w = std::max(band_w, sc.f[k].tw);
     }
     const int band_cl = pair_ok ? g4::band_cluster(ng, band_w) : 0;
+    // a cluster a slice with its bands' S1 in tensor memory: grids too large for one CTA,
+    // windows of few slices, and a pair where one is asked for
+    int cluster = !pair_ok || h->field_kernel == 2 ? 0
+                  : h->field_kernel == 1 && fused  ? 2
+                                                   : g4::field_cluster(ng, ns * h->together, band_w);
+    for (int k = 0; k < c.nfield && cluster; k++)
+      if (!g4::field_cluster_fits(ng, sc.f[k].tw, cluster)) cluster = 0;
     bool pair = band_cl > 0 && (h->field_kernel == 1 || !fused);
     // the whole step in one kernel (push, deposition, ADI; one CTA per slice): chosen
     // by the autotuner (field_kernel 2) for one-field windows without space charge
@@ -1358,20 +1365,24 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       }
       if (isr.ctr) g4::launch_isr_advance(h->stream, h->isr_ctr);
       if (rec_ok) h->diag_fields_in_step = h->diag_beam_in_step = true;
-    } else if (fused || pair) {
+    } else if (fused || pair || cluster) {
       g4::StepConstF scf = scf_push;
       if (do_push) push(nullptr, 0);
       if (do_field) {
         // the diagnostic record of a step run by g4gpu_run_diag, formed by the fused
         // kernel itself when it holds the scratch for it
-        bool rec = h->diag_rec && !pair;
-        for (int k = 0; k < c.nfield && rec; k++)
+        bool rec = h->diag_rec && (!pair || cluster);
+        for (int k = 0; k < c.nfield && rec && !cluster; k++)
           rec = g4::field_record_fits(ng, field_threads(h, sc.f[k].tw), sc.f[k].tw, h->diag_nharm);
         const int bw = g4::beam_diag_width(h->diag_nharm), fw = g4::kFieldSums + 2;
         for (int k = 0; k < c.nfield; k++) {
           const char *cb = (const char *)h->coef + (size_t)sc.f[k].coef * 3 * ng * h->csize;
           Timed t(h, G4GPU_K_ADI_X);
-          if (pair)
+          if (cluster)
+            g4::launch_field_cluster_mixed(L, scf, k, h->beam, h->field[k], cb, seg_powers(h, sc.f[k].coef), ns, np, ng,
+                                           sc.f[k].dep_on, cluster,
+                                           rec ? h->diag_rec + (size_t)ns * bw + (size_t)k * ns * fw : nullptr);
+          else if (pair)
             g4::launch_field_band_mixed(L, scf, k, h->beam, h->field[k], cb, ns, np, ng, sc.f[k].dep_on,
                                         band_cl);
           else
@@ -2305,7 +2316,9 @@ extern "C" int g4gpu_batch_run(g4gpu_batch b, int istep0, int nsteps, int stages
       if (nm[i] <= 0) continue;
       cudaStreamWaitEvent(m->stream, b->fork, 0);
       m->capturing = true;
+      m->together = nrun;
       rc = enqueue_steps(m, istep0, nm[i], stages);
+      m->together = 1;
       m->capturing = false;
       cudaEventRecord(b->join[i], m->stream);
       cudaStreamWaitEvent(b->origin, b->join[i], 0);

@@ -125,6 +125,7 @@ struct g4gpu_ctx {
   // layout, set-up), so that a batch's ensemble graphs of this member are not reused
   long long graph_gen = 0;
   bool capturing = false;
+  int together = 1;  // windows stepped side by side (g4gpu_batch_run)
 
   // learned closure (g4gpu_learned.cpp)
   g4gpu_mlp_ctx *mlp = nullptr;

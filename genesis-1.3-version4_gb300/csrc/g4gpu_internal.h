@@ -183,6 +183,14 @@ void launch_field_band_mixed(const Launch &L, const StepConstF &sc, int k, const
 void launch_field_fused_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b,
                               void *field, const void *coef, const void *pow, int ns, int np, int ngrid, int deposit,
                               int threads, double *dbeam, double *dfield, int nharm, double gref);
+// The fused field step with a slice's rows split between the cl CTAs of a cluster
+// (k_field_cl_f): field_cluster gives the cluster size for a window of ns slices, 0 where one
+// CTA a slice is better or no size fits; dfield as launch_field_fused_mixed's.
+int field_cluster(int ngrid, int ns, int W);
+bool field_cluster_fits(int ngrid, int W, int cl);
+void launch_field_cluster_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b, void *field,
+                                const void *coef, const void *pow, int ns, int np, int ngrid, int deposit, int cl,
+                                double *dfield);
 // the CTA size of a handle without a set one, and whether the kernel that size and warm-up
 // length W select records the field's diagnostics
 int field_threads_auto(int ngrid, int ns, int W);

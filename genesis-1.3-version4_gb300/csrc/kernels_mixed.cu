@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -179,14 +180,28 @@ __device__ __forceinline__ void transverse_f(const StepConstF &sc, bool last, fl
 struct CellF {
   int i00, i10, i01, i11;
   float wx, wy;
+  int iy;
 };
 // ng x ng cells in rows of st elements
 struct Grid {
   int ng, st;
   __device__ __forceinline__ Grid(int n) : ng(n), st(n) {}
   __device__ __forceinline__ Grid(int n, int stride) : ng(n), st(stride) {}
+  // offset of row iy, whether cell offset i is held, whether none of rows iy, iy + 1 is
+  __device__ __forceinline__ int row(int iy) const { return iy * st; }
+  __device__ __forceinline__ bool holds(int) const { return true; }
+  __device__ __forceinline__ bool outside(int) const { return false; }
 };
-__device__ __forceinline__ bool ll_gridpoint_f(float gm, float dg, Grid g, float x, float y, CellF &c) {
+// The rows [r0, r0 + n) of a grid: deposits into other rows are left out.
+struct Band : Grid {
+  int r0, n;
+  __device__ __forceinline__ Band(int ng, int stride, int first, int rows) : Grid(ng, stride), r0(first), n(rows) {}
+  __device__ __forceinline__ int row(int iy) const { return (iy - r0) * st; }
+  __device__ __forceinline__ bool holds(int i) const { return (unsigned)i < (unsigned)(n * st); }
+  __device__ __forceinline__ bool outside(int iy) const { return iy + 1 < r0 || iy >= r0 + n; }
+};
+template <class G>
+__device__ __forceinline__ bool ll_gridpoint_f(float gm, float dg, G g, float x, float y, CellF &c) {
   const int ng = g.ng;
   if ((x > -gm) && (x < gm) && (y > -gm) && (y < gm)) {
     float wx = (x + gm) / dg, wy = (y + gm) / dg;
@@ -196,10 +211,11 @@ __device__ __forceinline__ bool ll_gridpoint_f(float gm, float dg, Grid g, float
     c.wy = 1.f + fy - wy;
     int ix1 = ix + 1 < ng ? ix + 1 : ix;
     int iy1 = iy + 1 < ng ? iy + 1 : iy;
-    c.i00 = ix + iy * g.st;
-    c.i10 = ix1 + iy * g.st;
-    c.i01 = ix + iy1 * g.st;
-    c.i11 = ix1 + iy1 * g.st;
+    c.iy = iy;
+    c.i00 = ix + g.row(iy);
+    c.i10 = ix1 + g.row(iy);
+    c.i01 = ix + g.row(iy1);
+    c.i11 = ix1 + g.row(iy1);
     return true;
   }
   return false;
@@ -298,7 +314,7 @@ __device__ __forceinline__ void deposit_f(const StepConstF &sc, const PtrsF &p, 
     const FieldStepF &fs = sc.f[k];
     if (!fs.dep_on) continue;
     CellF c;
-    const bool on = valid && ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c);
+    const bool on = valid && ll_gridpoint_f(fs.gridmax, fs.dgrid, Grid(ng), x, y, c);
     float2 cp = make_float2(0.f, 0.f);
     if (on) {
       float part = base * fs.dep_scl * cur;
@@ -351,7 +367,7 @@ __device__ __forceinline__ void push_rest_f(const StepConstF &sc, const PtrsF &p
     const FieldStepF &fs = sc.f[k];
     const float2 *f = fslice[k];
     CellF c;
-    if (ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c)) {
+    if (ll_gridpoint_f(fs.gridmax, fs.dgrid, Grid(ng), x, y, c)) {
       float2 v00 = f[c.i00], v10 = f[c.i10], v01 = f[c.i01], v11 = f[c.i11];
       float w00 = c.wx * c.wy, w10 = (1.f - c.wx) * c.wy, w01 = c.wx * (1.f - c.wy),
             w11 = (1.f - c.wx) * (1.f - c.wy);
@@ -772,11 +788,13 @@ __device__ __forceinline__ void r2_cols_seg(float2 *S, const float2 *__restrict_
 // of its 15 thousand cycles). Measured and slower: one 64-bit compare-and-swap loop per cell
 // for both parts, in turn or the four side by side (field step of 4096 slices 709 -> 712 and
 // 737 us).
-__device__ __forceinline__ void add_to_cells(float2 *S, int i00, int i10, int i01, int i11, const float2 *v) {
+template <class G>
+__device__ __forceinline__ void add_to_cells(float2 *S, G g, int i00, int i10, int i01, int i11, const float2 *v) {
   const int i[4] = {i00, i10, i01, i11};
   const bool odd = threadIdx.x & 1u;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
+    if (!g.holds(i[q])) continue;
     float *c = reinterpret_cast<float *>(S + i[q]);
     atomicAdd(c + (odd ? 1 : 0), odd ? v[q].y : v[q].x);
     atomicAdd(c + (odd ? 0 : 1), odd ? v[q].x : v[q].y);
@@ -791,11 +809,12 @@ __device__ __forceinline__ void add_to_cells(float2 *S, int i00, int i10, int i0
 // runs of equal cells; only the first lane of each run issues the atomics. This cuts
 // the atomics (and their same-address conflicts) by the run length and keeps the
 // result exact up to FP32 summation order. Every lane of the warp must call it.
+template <class G>
 __device__ __forceinline__ void deposit_lanes(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                              Grid ng, float x, float y, long long th, float dgam) {
+                                              G ng, float x, float y, long long th, float dgam) {
   const unsigned lane = threadIdx.x & 31u;
   CellF c;
-  bool on = ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c);
+  bool on = ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c) && !ng.outside(c.iy);
   float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (on) {
     float g = (float)sc.gammaref + dgam;
@@ -812,7 +831,7 @@ __device__ __forceinline__ void deposit_lanes(const StepConstF &sc, const FieldS
   }
   // runs of equal lower-left cells among adjacent lanes (off-grid lanes carry
   // zeros and key -1; they issue no atomics)
-  int key = on ? c.i00 : -1;
+  int key = on ? c.i00 : INT_MIN;
   bool run_head;
   // both shuffles run on every lane (a short-circuit && would leave some lanes out
   // of a full-mask shuffle)
@@ -846,14 +865,15 @@ __device__ __forceinline__ void deposit_lanes(const StepConstF &sc, const FieldS
   if (on && run_head) {
     const float2 w[4] = {make_float2(v[0], v[1]), make_float2(v[2], v[3]), make_float2(v[4], v[5]),
                          make_float2(v[6], v[7])};
-    add_to_cells(S, c.i00, c.i10, c.i01, c.i11, w);
+    add_to_cells(S, ng, c.i00, c.i10, c.i01, c.i11, w);
   }
 }
 
 // Adds the deposited source of beam slice `is` to S, the particles read from global
 // memory (used when no staging buffer fits beside the slice).
+template <class G>
 __device__ __forceinline__ void deposit_smem(const StepConstF &sc, const FieldStepF &fs,
-                                             const PtrsF &p, float2 *S, int is, int np, Grid ng) {
+                                             const PtrsF &p, float2 *S, int is, int np, G ng) {
   const float scl = fs.dep_scl * slice_cur_f(p, is, np);
   const size_t base = (size_t)is * np;
   const int n = slice_np_f(p, is, np);
@@ -878,10 +898,11 @@ __device__ __forceinline__ void deposit_smem(const StepConstF &sc, const FieldSt
 }
 
 // The contribution of one particle to the four cells around it (no aggregation).
+template <class G>
 __device__ __forceinline__ void deposit_one(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                            Grid ng, float x, float y, long long th, float dgam) {
+                                            G ng, float x, float y, long long th, float dgam) {
   CellF c;
-  if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c)) return;
+  if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c) || ng.outside(c.iy)) return;
   float dx = x - sc.ax, dy = y - sc.ay;
   float faw2 = 1.f + sc.kx * dx * dx + sc.ky * dy * dy + 2.f * (sc.gradx * dx + sc.grady * dy);
   float part = sqrtf(faw2) * scl / ((float)sc.gammaref + dgam);
@@ -891,16 +912,16 @@ __device__ __forceinline__ void deposit_one(const StepConstF &sc, const FieldSte
   float w00 = c.wx * c.wy, w10 = (1.f - c.wx) * c.wy, w01 = c.wx * (1.f - c.wy), w11 = (1.f - c.wx) * (1.f - c.wy);
   const float2 v[4] = {make_float2(w00 * cpx, w00 * cpy), make_float2(w10 * cpx, w10 * cpy),
                        make_float2(w01 * cpx, w01 * cpy), make_float2(w11 * cpx, w11 * cpy)};
-  add_to_cells(S, c.i00, c.i10, c.i01, c.i11, v);
+  add_to_cells(S, ng, c.i00, c.i10, c.i01, c.i11, v);
 }
 
 // The summed contribution of n particles that share x and y (one cell, one set of
 // weights, one undulator factor), n = 2 or 4.
-template <int N>
+template <int N, class G>
 __device__ __forceinline__ void deposit_group(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                              Grid ng, float x, float y, const long long *th, const float *dgam) {
+                                              G ng, float x, float y, const long long *th, const float *dgam) {
   CellF c;
-  if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c)) return;
+  if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c) || ng.outside(c.iy)) return;
   float dx = x - sc.ax, dy = y - sc.ay;
   float faw2 = 1.f + sc.kx * dx * dx + sc.ky * dy * dy + 2.f * (sc.gradx * dx + sc.grady * dy);
   float a = sqrtf(faw2) * scl;
@@ -916,7 +937,7 @@ __device__ __forceinline__ void deposit_group(const StepConstF &sc, const FieldS
   float w00 = c.wx * c.wy, w10 = (1.f - c.wx) * c.wy, w01 = c.wx * (1.f - c.wy), w11 = (1.f - c.wx) * (1.f - c.wy);
   const float2 v[4] = {make_float2(w00 * cpx, w00 * cpy), make_float2(w10 * cpx, w10 * cpy),
                        make_float2(w01 * cpx, w01 * cpy), make_float2(w11 * cpx, w11 * cpy)};
-  add_to_cells(S, c.i00, c.i10, c.i01, c.i11, v);
+  add_to_cells(S, ng, c.i00, c.i10, c.i01, c.i11, v);
 }
 
 __device__ __forceinline__ float sqrt_approx(float a) {
@@ -937,8 +958,9 @@ __device__ __forceinline__ float rcp_approx(float a) {
 // deposited nothing, unless all four lie inside the grid in the same cell. The cells are
 // compared as floats and converted once; dx, dy and the gradients drop out of a centred
 // undulator's factor.
+template <class G>
 __device__ __forceinline__ bool deposit_cell4(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S,
-                                              Grid ng, const float *x, const float *y, const long long *th,
+                                              G ng, const float *x, const float *y, const long long *th,
                                               const float *dgam) {
   const float gm = fs.gridmax, dg = fs.dgrid;
   float wx[4], wy[4];
@@ -952,6 +974,8 @@ __device__ __forceinline__ bool deposit_cell4(const StepConstF &sc, const FieldS
     wy[m] = 1.f + fy - ty;
   }
   if (!same) return false;
+  const int ix = min((int)fx, ng.ng - 1), iy = min((int)fy, ng.ng - 1);
+  if (ng.outside(iy)) return true;  // the rows are another band's
   const float g0 = (float)sc.gammaref;
   float2 v00 = make_float2(0.f, 0.f), v10 = v00, v01 = v00, v11 = v00;
 #pragma unroll
@@ -974,10 +998,9 @@ __device__ __forceinline__ bool deposit_cell4(const StepConstF &sc, const FieldS
     v01 = make_float2(fmaf(wx[m], b.x, v01.x), fmaf(wx[m], b.y, v01.y));
     v11 = make_float2(fmaf(ux, b.x, v11.x), fmaf(ux, b.y, v11.y));
   }
-  const int ix = min((int)fx, ng.ng - 1), iy = min((int)fy, ng.ng - 1);
-  const int i = ix + iy * ng.st, ex = ix + 1 < ng.ng ? 1 : 0, ey = iy + 1 < ng.ng ? ng.st : 0;
+  const int i = ix + ng.row(iy), ex = ix + 1 < ng.ng ? 1 : 0, ey = iy + 1 < ng.ng ? ng.st : 0;
   const float2 v[4] = {v00, v10, v01, v11};
-  add_to_cells(S, i, i + ex, i + ey, i + ey + ex, v);
+  add_to_cells(S, ng, i, i + ex, i + ey, i + ey + ex, v);
   return true;
 }
 
@@ -999,7 +1022,8 @@ __device__ __forceinline__ Quad load_quad(const PtrsF &p, size_t base, int q) {
   return Quad{reinterpret_cast<const float4 *>(p.x + base)[q], reinterpret_cast<const float4 *>(p.y + base)[q],
               reinterpret_cast<const float4 *>(p.dg + base)[q], T[2 * q], T[2 * q + 1]};
 }
-__device__ __forceinline__ void deposit_quad(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S, Grid ng,
+template <class G>
+__device__ __forceinline__ void deposit_quad(const StepConstF &sc, const FieldStepF &fs, float scl, float2 *S, G ng,
                                              const Quad &v) {
   const float4 &x = v.x, &y = v.y, &g = v.g;
   const long long th[4] = {v.t01.x, v.t01.y, v.t23.x, v.t23.y};
@@ -1076,21 +1100,21 @@ __global__ void __launch_bounds__(128) k_source_f(StepConstF sc, PtrsF p, const 
   const float dg[4] = {g.x, g.y, g.z, g.w};
   const bool p01 = x[0] == x[1] && y[0] == y[1], p23 = x[2] == x[3] && y[2] == y[3];
   if (p01 && p23 && x[0] == x[2] && y[0] == y[2]) {
-    deposit_group<4>(sc, fs, scl, S, ng, x[0], y[0], th, dg);
+    deposit_group<4>(sc, fs, scl, S, Grid(ng), x[0], y[0], th, dg);
     return;
   }
-  if (deposit_cell4(sc, fs, scl, S, ng, x, y, th, dg)) return;
+  if (deposit_cell4(sc, fs, scl, S, Grid(ng), x, y, th, dg)) return;
   if (p01) {
-    deposit_group<2>(sc, fs, scl, S, ng, x[0], y[0], th, dg);
+    deposit_group<2>(sc, fs, scl, S, Grid(ng), x[0], y[0], th, dg);
   } else {
-    deposit_one(sc, fs, scl, S, ng, x[0], y[0], th[0], dg[0]);
-    deposit_one(sc, fs, scl, S, ng, x[1], y[1], th[1], dg[1]);
+    deposit_one(sc, fs, scl, S, Grid(ng), x[0], y[0], th[0], dg[0]);
+    deposit_one(sc, fs, scl, S, Grid(ng), x[1], y[1], th[1], dg[1]);
   }
   if (p23) {
-    deposit_group<2>(sc, fs, scl, S, ng, x[2], y[2], th + 2, dg + 2);
+    deposit_group<2>(sc, fs, scl, S, Grid(ng), x[2], y[2], th + 2, dg + 2);
   } else {
-    deposit_one(sc, fs, scl, S, ng, x[2], y[2], th[2], dg[2]);
-    deposit_one(sc, fs, scl, S, ng, x[3], y[3], th[3], dg[3]);
+    deposit_one(sc, fs, scl, S, Grid(ng), x[2], y[2], th[2], dg[2]);
+    deposit_one(sc, fs, scl, S, Grid(ng), x[3], y[3], th[3], dg[3]);
   }
 }
 
@@ -1368,9 +1392,9 @@ __global__ void __launch_bounds__(kFusedMaxThreads, 1)
   if (deposit) {  // S = S1 + src
     // full slices of a multiple of 4 particles take the 16-byte vector loads
     if ((np & 3) == 0 && !p.count)
-      deposit_quads(sc, fs, p, S, is, np, ng);
+      deposit_quads(sc, fs, p, S, is, np, Grid(ng));
     else
-      deposit_smem(sc, fs, p, S, is, np, ng);
+      deposit_smem(sc, fs, p, S, is, np, Grid(ng));
     __syncthreads();
   }
   const float2 invden = K[0];
@@ -1519,7 +1543,7 @@ __global__ void __launch_bounds__(MAXT, 1)
           p.py[o] = py[v];
         }
         if (deposit)
-          deposit_lanes(sc, fs, scl, S, ng, in ? x[v] : 1e30f, in ? y[v] : 1e30f, th[v], dg[v]);
+          deposit_lanes(sc, fs, scl, S, Grid(ng), in ? x[v] : 1e30f, in ? y[v] : 1e30f, th[v], dg[v]);
       }
     }
   }
@@ -1822,6 +1846,10 @@ PtrsF make_ptrs_f(const DeviceBeam &b, void *const *field, void *const *src, int
 }
 
 // ---- fused field step on a cluster of CTAs (2, 3 or 4 per slice) ---------------
+//
+// For the clusters that k_field_cl_f (field_tm.cuh) does not take: warm-ups W of more than
+// kTmLook + 1 rows (large steps), and step factors that differ between the fields so that
+// one of them is such.
 //
 // The slice's rows are split between the CL CTAs of a thread-block cluster: CTA q
 // holds the band of rows [q h, min((q + 1) h, ng)), h = ceil(ng / CL). A band is a
@@ -2556,6 +2584,100 @@ int field_threads_auto(int ngrid, int ns, int W) {
   if (two && ns > field_sms() && field_tm_fits(ngrid, two, W) && field_tm_per_sm(tm_smem_bytes(ngrid, W, two), two) == 2)
     return two;
   return kTmMaxThreads;
+}
+namespace {
+template <int LA, bool REC>
+void launch_field_cl(const Launch &L, const StepConstF &sc, int k, const PtrsF &p, void *field, const void *coef,
+                     const void *pow, int ns, int np, int ngrid, int deposit, int cl, double *dfield) {
+  static std::atomic<unsigned long long> configured{0};  // one bit per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !(configured.load() & (1ull << dev))) {
+    cudaFuncSetAttribute(k_field_cl_f<LA, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 16);
+    if (dev < 64) configured.fetch_or(1ull << dev);
+  }
+  const int W = sc.f[k].tw;
+  const ClShape t = cl_shape(ngrid, W, cl);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {(unsigned)cl, 1, 1};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cl * ns);
+  cfg.blockDim = dim3(t.threads);
+  cfg.dynamicSmemBytes = t.smem;
+  cfg.stream = (cudaStream_t)L.stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_field_cl_f<LA, REC>, sc, k, p, (float2 *)field, (const float2 *)coef, (const float2 *)pow,
+                     ns, np, ngrid, deposit, t.nseg, W, t.words, t.cols, field_sms() / cl, dfield);
+}
+}  // namespace
+
+// Clusters of cl CTAs of k_field_cl_f that run at once (one CTA an SM)
+static int cluster_slots(int cl) {
+  static std::atomic<int> slots[64][kMaxCluster + 1];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int n = dev < 64 ? slots[dev][cl].load() : 0;
+  if (n) return n;
+  cudaFuncSetAttribute(k_field_cl_f<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 16);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {(unsigned)cl, 1, 1};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(cl * 64);
+  cfg.blockDim = dim3(kTmMaxThreads);
+  cfg.dynamicSmemBytes = 227 * 1024 - 16;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, k_field_cl_f<8, false>, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = std::max(1, field_sms() / cl);
+  }
+  if (dev < 64) slots[dev][cl].store(n);
+  return n;
+}
+
+// The cluster whose rounds over the window's slices take the least time. One round takes 17 us
+// of latencies and 36 us / CL for a slice of 255^2 (measured, one round, 8192 particles: 255^2
+// with CL 3, 4, 6, 8 29, 27, 23, 22 us; 151^2 with CL 1, 2, 4, 8 28.6, 23.1, 20.5, 19.7); a grid
+// that fits one CTA but not with its odd stride and tensor memory (ngrid 166 to 168) takes a
+// quarter more there. So a window of few slices is spread over idle SMs (1 to 36 slices of
+// 151^2 28.6 -> 20.5 us, 75 24.5) and one that fills the chip takes the smallest cluster that
+// fits (300 slices: 255^2 272 us with k_field_band_f -> 184 with CL 3, 201 with 4; 180^2 191 ->
+// 104; 300^2 439 -> 245). Grids whose bands do not fit four CTAs (ngrid above 333) stay with the
+// tiled path and its two passes in the kernel statistics.
+int field_cluster(int ngrid, int ns, int W) {
+  const double cells = (double)ngrid * ngrid / (255. * 255.);
+  const bool tm = field_tm_fits(ngrid, kTmMaxThreads, W);
+  double best = 1e30;
+  int cl = 0;
+  if (tm || ngrid <= fused_max_ngrid()) {
+    if (ns > field_sms() && tm) return 0;
+    best = (17 + 36 * cells) * (tm ? 1 : 1.25) * ((ns + field_sms() - 1) / field_sms());
+  } else if (!band_cluster(ngrid, W)) {
+    return 0;
+  }
+  for (int c = 2; c <= kMaxCluster; c++) {
+    if (!cl_shape(ngrid, W, c).cl) continue;
+    const int n = cluster_slots(c);
+    const double t = (17 + 36 * cells / c) * ((ns + n - 1) / n);
+    if (t < 0.95 * best) {
+      best = t;
+      cl = c;
+    }
+  }
+  return cl;
+}
+bool field_cluster_fits(int ngrid, int W, int cl) { return cl_shape(ngrid, W, cl).cl > 0; }
+
+void launch_field_cluster_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b, void *field,
+                                const void *coef, const void *pow, int ns, int np, int ngrid, int deposit, int cl,
+                                double *dfield) {
+  PtrsF p = make_ptrs_f(b, nullptr, nullptr, 0);
+  const auto launch = sc.f[k].tw <= 9 ? (dfield ? launch_field_cl<8, true> : launch_field_cl<8, false>)
+                                      : (dfield ? launch_field_cl<kTmLook, true> : launch_field_cl<kTmLook, false>);
+  launch(L, sc, k, p, field, coef, pow, ns, np, ngrid, deposit, cl, dfield);
 }
 bool field_record_fits(int ngrid, int threads, int W, int nharm) {
   return field_tm_fits(ngrid, fused_threads(ngrid, threads), W) || fused_diag_fits(ngrid, threads, nharm);
