@@ -299,6 +299,8 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tm = tm_base + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * words);
+  chain_next();
+  chain_wait();
 
   // line (a column in the column phases, a row in the row solve) and segment of the thread
   const int line = tid % ng, seg = tid / ng;
@@ -484,13 +486,15 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   float2 *u = field + (size_t)i * ng * ng + (size_t)r0 * ng;  // the band
   const size_t base = (size_t)is * np;
   const bool vec = deposit && (np & 3) == 0 && !p.count;
-  // the first particles' loads in flight while S1 is formed
-  Quad quad{};
-  if (vec && tid < (np >> 2)) quad = load_quad(p, base, tid);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tm = tm_base + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * words);
+  chain_next();
+  chain_wait();
+  // the first particles' loads in flight while S1 is formed
+  Quad quad{};
+  if (vec && tid < (np >> 2)) quad = load_quad(p, base, tid);
 
   // column and segment of the thread
   const int line = tid % ng, seg = tid / ng;

@@ -34,6 +34,7 @@
 #include <string>
 
 #include "g4gpu_internal.h"
+#include "launch_chain.cuh"
 #include "philox.cuh"
 
 // Scratch of g4gpu_adi_advance_noalloc: 32 MiB, shared by every call on a device and
@@ -407,6 +408,8 @@ __device__ __forceinline__ void push_rest_f(const StepConstF &sc, const PtrsF &p
 template <int NF>
 __global__ void __launch_bounds__(512) k_push_f(StepConstF sc, PtrsF p, int ns, int np, int ng,
                                                 int deposit) {
+  chain_next();
+  chain_wait();
   int is = blockIdx.y;
   int ip = blockIdx.x * blockDim.x + threadIdx.x;
   // lanes past the slice's particles stay for the deposition's warp shuffles
@@ -1708,6 +1711,8 @@ __global__ void __launch_bounds__(BS) k_diag_beam_f(PtrsF p, double gref, int np
   // place once the last group has been read
   constexpr int kStages = kDiagAhead + 1, kRed = (BS / 32) * (NSUM + 10);
   static_assert(kRed * sizeof(double) <= sizeof(float4) * kStages * 7 * BS, "");
+  chain_next();
+  chain_wait();
   __shared__ float4 ring[kStages][7][BS];
   __shared__ double res[NSUM + 10];
   double *sh = reinterpret_cast<double *>(ring);
@@ -2442,10 +2447,10 @@ void launch_push_mixed_sc(const Launch &L, const StepConstF &sc, const DeviceBea
   dim3 grid((np + block - 1) / block, ns);
   cudaStream_t s = (cudaStream_t)L.stream;
   switch (sc.nfld) {
-    case 1: k_push_f<1><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
-    case 2: k_push_f<2><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
-    case 3: k_push_f<3><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
-    default: k_push_f<G4GPU_MAX_FIELDS><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
+    case 1: chain_launch(k_push_f<1>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
+    case 2: chain_launch(k_push_f<2>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
+    case 3: chain_launch(k_push_f<3>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
+    default: chain_launch(k_push_f<G4GPU_MAX_FIELDS>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
   }
 }
 
@@ -2505,13 +2510,13 @@ void launch_diag_beam_mixed(const Launch &L, const DeviceBeam &b, double gammare
   PtrsF p = make_ptrs_f(b, nullptr, nullptr, 0);
   cudaStream_t s = (cudaStream_t)L.stream;
   if (nharm <= 1)
-    k_diag_beam_f<kDiagBlock, 1><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
+    chain_launch(k_diag_beam_f<kDiagBlock, 1>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
   else if (nharm <= 3)
-    k_diag_beam_f<kDiagBlock, 3><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
+    chain_launch(k_diag_beam_f<kDiagBlock, 3>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
   else if (nharm <= 5)
-    k_diag_beam_f<kDiagBlock, 5><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
+    chain_launch(k_diag_beam_f<kDiagBlock, 5>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
   else
-    k_diag_beam_f<kDiagBlock, G4GPU_MAX_HARM><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
+    chain_launch(k_diag_beam_f<kDiagBlock, G4GPU_MAX_HARM>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
 }
 
 void launch_diag_field_mixed(const Launch &L, const void *field, int ns, int ngrid, double *out) {
@@ -2568,9 +2573,9 @@ void launch_field_tm(const Launch &L, const StepConstF &sc, int k, const PtrsF &
   const TmShape t = tm_shape(ngrid, threads, W);
   threads = t.threads;
   const size_t smem = tm_smem_bytes(ngrid, W, threads);
-  k_field_tm_f<LA, REC><<<std::min(ns, field_sms() * field_tm_per_sm(smem, threads)), threads, smem,
-                          (cudaStream_t)L.stream>>>(sc, k, p, (float2 *)field, (const float2 *)coef, (const float2 *)pow,
-                                                    ns, np, ngrid, deposit, t.nseg, W, t.words, t.cols, dfield);
+  chain_launch(k_field_tm_f<LA, REC>, std::min(ns, field_sms() * field_tm_per_sm(smem, threads)), threads, smem,
+               (cudaStream_t)L.stream, 0, sc, k, p, (float2 *)field, (const float2 *)coef, (const float2 *)pow, ns, np,
+               ngrid, deposit, t.nseg, W, t.words, t.cols, dfield);
 }
 }  // namespace
 
@@ -2598,18 +2603,9 @@ void launch_field_cl(const Launch &L, const StepConstF &sc, int k, const PtrsF &
   }
   const int W = sc.f[k].tw;
   const ClShape t = cl_shape(ngrid, W, cl);
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim = {(unsigned)cl, 1, 1};
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(cl * ns);
-  cfg.blockDim = dim3(t.threads);
-  cfg.dynamicSmemBytes = t.smem;
-  cfg.stream = (cudaStream_t)L.stream;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_field_cl_f<LA, REC>, sc, k, p, (float2 *)field, (const float2 *)coef, (const float2 *)pow,
-                     ns, np, ngrid, deposit, t.nseg, W, t.words, t.cols, field_sms() / cl, dfield);
+  chain_launch(k_field_cl_f<LA, REC>, cl * ns, t.threads, t.smem, (cudaStream_t)L.stream, cl, sc, k, p, (float2 *)field,
+               (const float2 *)coef, (const float2 *)pow, ns, np, ngrid, deposit, t.nseg, W, t.words, t.cols,
+               field_sms() / cl, dfield);
 }
 }  // namespace
 
