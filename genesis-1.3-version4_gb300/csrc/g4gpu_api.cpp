@@ -1225,6 +1225,34 @@ static int enqueue_coarse_step(g4gpu_handle h, int istep, int cnt) {
   return G4GPU_OK;
 }
 
+namespace {
+void enqueue_diag(g4gpu_handle h, cudaStream_t stream, int nharm, double *rec, bool beam, bool field);
+
+// The order of a step against the records formed beside it (g4gpu_ctx::SideRecord)
+int side_before_push(g4gpu_handle h) {
+  if (!h->side || !h->side->beam_wait) return G4GPU_OK;
+  G4_CUDA(h, cudaStreamWaitEvent(h->stream, h->side->beam_read, 0));
+  h->side->beam_wait = false;
+  return G4GPU_OK;
+}
+int side_after_push(g4gpu_handle h) {
+  g4gpu_ctx::SideRecord *r = h->side;
+  if (!r || !r->beam) return G4GPU_OK;
+  G4_CUDA(h, cudaEventRecord(r->moved, h->stream));
+  G4_CUDA(h, cudaStreamWaitEvent(r->stream, r->moved, 0));
+  enqueue_diag(h, r->stream, h->diag_nharm, h->diag_rec, true, false);
+  G4_CUDA(h, cudaEventRecord(r->beam_read, r->stream));
+  r->beam_wait = h->diag_beam_in_step = true;
+  return G4GPU_OK;
+}
+int side_before_field(g4gpu_handle h) {
+  if (!h->side || !h->side->field_wait) return G4GPU_OK;
+  G4_CUDA(h, cudaStreamWaitEvent(h->stream, h->side->field_read, 0));
+  h->side->field_wait = false;
+  return G4GPU_OK;
+}
+}  // namespace
+
 static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
   const g4gpu_config &c = h->cfg;
   int ns = c.nslice, np = c.npart, ng = c.ngrid;
@@ -1271,7 +1299,7 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
     // the push the rest of the step.
     // Collective::apply after the integration (Beam.cpp:108)
     const void *wake = !h->wake_on ? nullptr : h->mixed ? (const void *)h->wake_lossf : (const void *)h->wake_loss;
-    auto push = [&](void *const *src, int deposit) -> int {
+    auto push_kernels = [&](void *const *src, int deposit) -> int {
       if (!h->sc_on) {
         Timed t(h, G4GPU_K_PUSH);
         if (h->mixed)
@@ -1326,6 +1354,11 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       if (isr.ctr) g4::launch_isr_advance(h->stream, h->isr_ctr);
       return G4GPU_OK;
     };
+    auto push = [&](void *const *src, int deposit) -> int {
+      int rc = side_before_push(h);
+      if (rc || (rc = push_kernels(src, deposit))) return rc;
+      return side_after_push(h);
+    };
     bool any_dep = false;
     for (int k = 0; k < c.nfield; k++) any_dep = any_dep || sc.f[k].dep_on;
     // mixed form with the slice in shared memory: deposition and ADI in one kernel,
@@ -1367,7 +1400,9 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       if (rec_ok) h->diag_fields_in_step = h->diag_beam_in_step = true;
     } else if (fused || pair || cluster) {
       g4::StepConstF scf = scf_push;
-      if (do_push) push(nullptr, 0);
+      if (do_push)
+        if (int rc = push(nullptr, 0)) return rc;
+      if (int rc = do_field ? side_before_field(h) : G4GPU_OK) return rc;
       if (do_field) {
         // the diagnostic record of a step run by g4gpu_run_diag, formed by the fused
         // kernel itself when it holds the scratch for it
@@ -1400,7 +1435,7 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
     g4::StepConstF scf{};
     if (h->mixed) scf = g4::to_float(sc, np);
     if (do_push) {
-      push(h->src, do_field && any_dep);
+      if (int rc = push(h->src, do_field && any_dep)) return rc;
     } else if (do_field && any_dep) {
       Timed t(h, G4GPU_K_PUSH);
       if (h->mixed)
@@ -1408,6 +1443,7 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
       else
         g4::launch_deposit_plain(L, sc, h->beam, h->src, ns, np, ng);
     }
+    if (int rc = do_field ? side_before_field(h) : G4GPU_OK) return rc;
     if (do_field && c.solver == G4GPU_SOLVER_FFT) {
       for (int k = 0; k < c.nfield; k++) {
         const void *srck = any_dep ? h->src[k] : nullptr;
@@ -1575,11 +1611,11 @@ int diag_scratch(g4gpu_handle h, int nharm) {
 }
 
 // Queues the kernels of one diagnostic record of the current state into `rec`.
-void enqueue_diag(g4gpu_handle h, int nharm, double *rec, bool beam, bool field) {
+void enqueue_diag(g4gpu_handle h, cudaStream_t stream, int nharm, double *rec, bool beam, bool field) {
   const g4gpu_config &c = h->cfg;
   int ns = c.nslice, np = c.npart, ng = c.ngrid;
   int bw = g4::beam_diag_width(nharm), fw = g4::kFieldSums + 2;
-  g4::Launch L{h->stream, h->derr};
+  g4::Launch L{stream, h->derr};
   double *db = rec, *dfd = rec + (size_t)ns * bw;
   if (!h->mixed) {
     if (!beam && !field) return;
@@ -1699,7 +1735,7 @@ int g4gpu_diag(g4gpu_handle h, int nharm, double *beam_out, double *field_out) {
   const size_t need = diag_record_doubles(h->cfg, nharm) * sizeof(double);
   int rc = diag_buffers(h, need);
   if (rc || (rc = diag_scratch(h, nharm))) return rc;
-  enqueue_diag(h, nharm, h->ddiag, beam_out != nullptr, field_out != nullptr);
+  enqueue_diag(h, h->stream, nharm, h->ddiag, beam_out != nullptr, field_out != nullptr);
   G4_CUDA(h, cudaGetLastError());
   G4_CUDA(h, cudaMemcpyAsync(h->hdiag, h->ddiag, need, cudaMemcpyDeviceToHost, h->stream));
   rc = check_device_flag(h);
@@ -1844,6 +1880,30 @@ int g4gpu_diag_fft(g4gpu_handle h, double *out) {
   return G4GPU_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// Whether g4gpu_run_diag forms the records beside the steps: not where a step's kernel forms
+// them itself, moves the beam outside the push (coarse steps), or is being timed. Windows that
+// leave SMs idle and windows of several rounds of CTAs gain; between them the record's CTAs
+// take the place and the pipes of CTAs of the step that would all have run at once. In line /
+// beside, us a step: mixed 1 x 8192 particles, 151^2 40 / 29, 22 x 4096 37 / 30, 75 x 8192
+// 53 / 62, 300 x 8192, 101^2 98 / 102, 300 x 8192, 255^2 297 / 279, 700 x 4096 212 / 196,
+// 2048 x 8192 596 / 567; FP64 1 x 8192, 255^2 91 / 78, 2 x 8192 106 / 108, 22 x 2052 98 / 121,
+// 64 x 4096 312 / 304, 150 x 2048 357 / 337, 320 x 8192 1974 / 1935.
+bool records_beside(g4gpu_handle h, int istep0, int nsteps) {
+  const g4gpu_config &c = h->cfg;
+  if (h->prof || h->field_kernel == 2) return false;
+  for (int s = istep0; s < istep0 + nsteps && s < (int)h->substeps.size(); s++)
+    if (h->substeps[s] > 1) return false;
+  if (!h->mixed) return c.nslice == 1 || c.nslice >= 64;
+  const int cluster = c.solver == G4GPU_SOLVER_ADI ? g4::field_cluster(c.ngrid, c.nslice, h->steps[istep0].f[0].tw) : 0;
+  return c.nslice <= 38 || c.nslice * std::max(cluster, 1) >= 608;  // a quarter of, or four times the SMs
+}
+}  // namespace
+
+extern "C" {
+
 int g4gpu_run_diag(g4gpu_handle h, int istep0, int nsteps, int nharm, double *beam_out, double *field_out) {
   if (!h) return fail(nullptr, G4GPU_ERR_ARG, "null handle");
   if (nharm < 1 || nharm > G4GPU_MAX_HARM) return fail(h, G4GPU_ERR_ARG, "nharm must be 1..16");
@@ -1868,9 +1928,13 @@ int g4gpu_run_diag(g4gpu_handle h, int istep0, int nsteps, int nharm, double *be
     std::vector<cudaEvent_t> ev;
     cudaEvent_t formed = nullptr;
     cudaStream_t copy = nullptr;
+    g4gpu_handle h = nullptr;
+    g4gpu_ctx::SideRecord side{};
     ~Events() {
+      if (h) h->side = nullptr;
       for (cudaEvent_t e : ev) cudaEventDestroy(e);
-      if (formed) cudaEventDestroy(formed);
+      for (cudaEvent_t e : {formed, side.moved, side.beam_read, side.field_read})
+        if (e) cudaEventDestroy(e);
       if (copy) {
         cudaStreamSynchronize(copy);
         cudaStreamDestroy(copy);
@@ -1880,6 +1944,14 @@ int g4gpu_run_diag(g4gpu_handle h, int istep0, int nsteps, int nharm, double *be
   done.ev.reserve(nsteps);
   G4_CUDA(h, cudaStreamCreateWithFlags(&done.copy, cudaStreamNonBlocking));
   G4_CUDA(h, cudaEventCreateWithFlags(&done.formed, cudaEventDisableTiming));
+  if (records_beside(h, istep0, nsteps)) {
+    for (cudaEvent_t *e : {&done.side.moved, &done.side.beam_read, &done.side.field_read})
+      G4_CUDA(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    done.side.stream = done.copy;
+    done.side.beam = beam_out != nullptr;
+    done.h = h;
+    h->side = &done.side;
+  }
   for (int s = 0; s < nsteps; s++) {
     // the fused field kernel forms the fields' record during the step where it can
     // (the slice is in its shared memory); the beam's, and the fields' elsewhere, come
@@ -1893,11 +1965,17 @@ int g4gpu_run_diag(g4gpu_handle h, int istep0, int nsteps, int nharm, double *be
     h->diag_fields_in_step = h->diag_beam_in_step = false;
     if (rc) return rc;
     for (int k = 0; k < c.nfield; k++) firsts[(size_t)s * G4GPU_MAX_FIELDS + k] = h->first[k];
-    enqueue_diag(h, nharm, h->ddiag + (size_t)s * rec, beam_out != nullptr && !beam_done,
-                 field_out != nullptr && !fields_done);
+    const bool beam_left = beam_out != nullptr && !beam_done, field_left = field_out != nullptr && !fields_done;
+    if (!h->side) enqueue_diag(h, h->stream, nharm, h->ddiag + (size_t)s * rec, beam_left, field_left);
     G4_CUDA(h, cudaGetLastError());
     G4_CUDA(h, cudaEventRecord(done.formed, h->stream));
     G4_CUDA(h, cudaStreamWaitEvent(done.copy, done.formed, 0));
+    if (h->side && field_left) {
+      enqueue_diag(h, done.copy, nharm, h->ddiag + (size_t)s * rec, false, true);
+      G4_CUDA(h, cudaGetLastError());
+      G4_CUDA(h, cudaEventRecord(done.side.field_read, done.copy));
+      done.side.field_wait = true;
+    }
     G4_CUDA(h, cudaMemcpyAsync(h->hdiag + (size_t)s * rec, h->ddiag + (size_t)s * rec, rec * sizeof(double),
                                cudaMemcpyDeviceToHost, done.copy));
     cudaEvent_t e;

@@ -126,6 +126,15 @@ struct g4gpu_ctx {
   long long graph_gen = 0;
   bool capturing = false;
   int together = 1;  // windows stepped side by side (g4gpu_batch_run)
+  // g4gpu_run_diag's records formed on a stream of their own, beside the step's later kernels
+  // (null: in line): the beam's once the push has moved it, the fields' after the step. The
+  // next push waits until the beam has been read, the next field solve until the fields have.
+  struct SideRecord {
+    cudaStream_t stream;
+    cudaEvent_t moved, beam_read, field_read;
+    bool beam, beam_wait = false, field_wait = false;
+  };
+  SideRecord *side = nullptr;
 
   // learned closure (g4gpu_learned.cpp)
   g4gpu_mlp_ctx *mlp = nullptr;

@@ -1711,8 +1711,6 @@ __global__ void __launch_bounds__(BS) k_diag_beam_f(PtrsF p, double gref, int np
   // place once the last group has been read
   constexpr int kStages = kDiagAhead + 1, kRed = (BS / 32) * (NSUM + 10);
   static_assert(kRed * sizeof(double) <= sizeof(float4) * kStages * 7 * BS, "");
-  chain_next();
-  chain_wait();
   __shared__ float4 ring[kStages][7][BS];
   __shared__ double res[NSUM + 10];
   double *sh = reinterpret_cast<double *>(ring);
@@ -2510,13 +2508,13 @@ void launch_diag_beam_mixed(const Launch &L, const DeviceBeam &b, double gammare
   PtrsF p = make_ptrs_f(b, nullptr, nullptr, 0);
   cudaStream_t s = (cudaStream_t)L.stream;
   if (nharm <= 1)
-    chain_launch(k_diag_beam_f<kDiagBlock, 1>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, 1><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
   else if (nharm <= 3)
-    chain_launch(k_diag_beam_f<kDiagBlock, 3>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, 3><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
   else if (nharm <= 5)
-    chain_launch(k_diag_beam_f<kDiagBlock, 5>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, 5><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
   else
-    chain_launch(k_diag_beam_f<kDiagBlock, G4GPU_MAX_HARM>, ns, kDiagBlock, 0, s, 0, p, gammaref, np, nharm, out);
+    k_diag_beam_f<kDiagBlock, G4GPU_MAX_HARM><<<ns, kDiagBlock, 0, s>>>(p, gammaref, np, nharm, out);
 }
 
 void launch_diag_field_mixed(const Launch &L, const void *field, int ns, int ngrid, double *out) {

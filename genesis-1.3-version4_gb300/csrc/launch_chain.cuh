@@ -8,7 +8,7 @@
 // allocation). All CTAs of a kernel have started before the next one's appear, so no CTA can
 // wait for one that has no room. Kernels launched in the ordinary way wait for all of it.
 //
-// Used by the mixed form's push, field step and beam record: 221 steps of one slice of 151^2
+// Used by the mixed form's push and field step: 221 steps of one slice of 151^2
 // 4.50 -> 4.16 ms, 48 steps of 150 slices of 117^2 with its copies 4.95 -> 4.66 ms, windows that
 // fill the chip unchanged. Not by the FP64 kernels, which it slowed down (111 steps of one
 // slice 8.65 -> 9.24 ms, 60 of 22 slices 6.46 -> 8.16): CTAs that are placed while the kernel
