@@ -212,6 +212,7 @@ int fft_tables(g4gpu_handle h) {
       m /= p;
     }
   if (m > 1) pl.radix[pl.nstage++] = m;
+  g4::fft_tile_layout(pl);
   // the n roots exp(-2 pi i m / n), then per stage the twiddles exp(-2 pi i q k / (ns R))
   const double two_pi = 2.0 * 3.14159265358979323846;
   std::vector<double> roots(2 * (2 * n - 1));

@@ -293,8 +293,12 @@ struct FFTPlan {
   // kernels divide small integers x (x d < 2^32) by them as one multiply-high
   unsigned mnb[32], mns[32];
   unsigned mn;  // ceil(2^32 / n)
+  // place of element i of line l in a tile: l ls + i + (i >> sh), see kernels_fft.cu
+  int ls, sh;
 };
+constexpr int kFftFlat = 31;  // sh of tiles without gaps (ls = n)
 int fft_max_ngrid(int mixed);
+void fft_tile_layout(FFTPlan &pl);  // ls and sh of a plan with its radices
 // lines of a slice one CTA transforms at a time in a pass with `bufs` tile buffers
 // and `per_sm` CTAs on an SM (es: bytes of a complex element; at most maxL)
 int fft_lines_per_cta(const FFTPlan &pl, int es, int bufs, int maxL, int per_sm, size_t table = 0);

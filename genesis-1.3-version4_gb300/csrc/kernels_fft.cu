@@ -275,10 +275,35 @@ __device__ __forceinline__ int fdiv(int x, int d, unsigned m) {
 // butterfly lives in one register array of the largest radix for every stage, so
 // that the stages' code paths share the registers held across the barrier.
 constexpr int MAX_RADIX = 17;
-template <int R, typename T2>
-__device__ __forceinline__ void stage_load(T2 *x, const T2 *src, int nb, int ns, int k, const T2 *tw) {
+//
+// Tiles of n divisible by 4 have gaps: one element after every 2^sh (2^sh the first radix), and an odd
+// line stride. Without them the first stage's stores, R elements from lane to lane, and the
+// transposed copies of the column pass, n from lane to lane, all fell into one pair of banks.
+// Past the first stage the strides are multiples of 2^sh, so that they only grow by the gaps;
+// its loads place every element. Three passes over 512 slices in FP32: n = 256 1056 -> 568 us,
+// 128 285 -> 175, 200 710 -> 695; odd n is not touched.
+// Kernels for tiles with gaps (GAP) are compiled beside those without.
+template <bool GAP>
+__device__ __forceinline__ int gaps(int i, int sh) { return GAP ? i >> sh : 0; }
+template <int R, bool GAP, typename T2>
+__device__ __forceinline__ void stage_load(T2 *x, const T2 *src, int j, int nb, int ns, int k, int sh, const T2 *tw) {
+  bool placed = false;
+  if constexpr (GAP && (R == 4 || R == 8 || R == 16)) {
+    if (ns == 1) {
+      placed = true;
 #pragma unroll
-  for (int q = 0; q < R; q++) x[q] = src[q * nb];
+      for (int q = 0; q < R; q++) {
+        const int i = j + q * nb;
+        x[q] = src[i + (i >> sh)];
+      }
+    }
+  }
+  if (!placed) {
+    const T2 *at = src + j + gaps<GAP>(j, sh);
+    const int step = nb + gaps<GAP>(nb, sh);
+#pragma unroll
+    for (int q = 0; q < R; q++) x[q] = at[q * step];
+  }
   if (ns > 1) {
 #pragma unroll
     for (int q = 1; q < R; q++) x[q] = cm(x[q], tw[(q - 1) * ns + k]);
@@ -290,6 +315,7 @@ __device__ __forceinline__ void stage_load(T2 *x, const T2 *src, int nb, int ns,
 // most STAGE_ANY_OUT outputs (lines n <= STAGE_ANY_OUT blockDim.x) in registers
 // before the CTA synchronises and they are written.
 constexpr int STAGE_ANY_OUT = 8;
+// (plans with such a stage have tiles without gaps)
 template <typename T2>
 __device__ __forceinline__ void any_load(T2 *acc, const T2 *A, int ls, int lines, int n, int ns, int r,
                                          const T2 *W) {
@@ -336,30 +362,30 @@ __host__ __device__ constexpr bool register_radix(int r) {
          r == 16 || r == 17;
 }
 
-// One 1-D Stockham FFT of length n, in place over `lines` lines of A stored with
-// line stride `ls`, the stages of the plan's radices in turn. W: the n roots exp(-2 pi i m / n), followed by the
+// One 1-D Stockham FFT of length n, in place over `lines` lines of the tile A, the stages of the plan's radices in turn. W: the n roots exp(-2 pi i m / n), followed by the
 // stage twiddle table (stage s's at W + n + plan.tw_off[s]).
-template <typename T2, int EXCH = 0>
-__device__ __forceinline__ void fft_lines(T2 *A, int ls, int lines, const FFTPlan &pl, const T2 *W,
+template <bool GAP, typename T2, int EXCH = 0>
+__device__ __forceinline__ void fft_lines(T2 *A, int lines, const FFTPlan &pl, const T2 *W,
                                           T2 *gout = nullptr,
                                           const Epilogue<T2, EXCH> &epi = Epilogue<T2, EXCH>{},
                                           bool wait_epi_copy = false) {
   int ns = 1;
   for (int s = 0; s < pl.nstage; s++) {
-    // the last stage of a pass with a global output writes it there (line stride ls)
+    // the last stage of a pass with a global output writes it there (line stride n)
     const bool to_global = gout && s == pl.nstage - 1;
     const int r = pl.radix[s], nb = pl.nb[s];
     const T2 *tw = W + pl.n + pl.tw_off[s];
     const bool act = (int)threadIdx.x < lines * nb;
     const int line = fdiv(threadIdx.x, nb, pl.mnb[s]), j = threadIdx.x - line * nb;
     const int k = j - fdiv(j, ns, pl.mns[s]) * ns;
-    const T2 *src = A + line * ls + j;
-    T2 *dst = A + line * ls + (j - k) * r + k;
+    const int ls = GAP ? pl.ls : pl.n, sh = pl.sh, oe = (j - k) * r + k, dstep = ns + gaps<GAP>(ns, sh);
+    const T2 *src = A + line * ls;
+    T2 *dst = A + line * ls + oe + gaps<GAP>(oe, sh);
     T2 x[MAX_RADIX];
     switch (r) {
 #define G4_LOAD(R) \
   case R:          \
-    if (act) stage_load<R>(x, src, nb, ns, k, tw); \
+    if (act) stage_load<R, GAP>(x, src, j, nb, ns, k, sh, tw); \
     break;
       G4_LOAD(2) G4_LOAD(3) G4_LOAD(4) G4_LOAD(5) G4_LOAD(7) G4_LOAD(8) G4_LOAD(9) G4_LOAD(11) G4_LOAD(13)
       G4_LOAD(15) G4_LOAD(16) G4_LOAD(17)
@@ -371,7 +397,7 @@ __device__ __forceinline__ void fft_lines(T2 *A, int ls, int lines, const FFTPla
     // copy group of this thread)
     if (to_global && wait_epi_copy) cp_wait<1>();
     __syncthreads();
-    const int o = line * ls + (j - k) * r + k;
+    const int o = line * pl.n + oe;
     Epilogue<T2, EXCH> e = epi;
     if (e.src) e.src += o;
     switch (r) {
@@ -381,7 +407,7 @@ __device__ __forceinline__ void fft_lines(T2 *A, int ls, int lines, const FFTPla
       if (to_global)                                     \
         dft<R, 2>(x, gout + o, ns, e);                   \
       else                                               \
-        dft<R, 1>(x, dst, ns);                           \
+        dft<R, 1>(x, dst, dstep);                        \
     }                                                    \
     break;
       G4_STORE(2) G4_STORE(3) G4_STORE(4) G4_STORE(5) G4_STORE(7) G4_STORE(8) G4_STORE(9) G4_STORE(11)
@@ -408,7 +434,7 @@ constexpr int FFT_CTAS_FP32 = 3, FFT_CTAS_FP64 = 2;
 // and imaginary parts are exchanged, exchanged back (the inverse transform), times `scale`,
 // plus 2 src (slice ii) when src is given, into `out`, with the source rows in a third tile buffer and one CTA per SM fewer.
 // in == out transforms in place.
-template <typename T2, int MODE>
+template <typename T2, int MODE, bool GAP>
 __global__ void __launch_bounds__(256, (sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64) - MODE)
     k_fft_rows(const T2 *in, T2 *out, const T2 *__restrict__ src, const T2 *__restrict__ roots, FFTPlan pl,
                int ns, int first, double scale, int L) {
@@ -416,20 +442,39 @@ __global__ void __launch_bounds__(256, (sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CT
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T2 *W = reinterpret_cast<T2 *>(smem_raw);
   const int n = pl.n;
-  T2 *Abuf = W + 2 * n;      // two tile buffers
-  T2 *S = Abuf + 2 * L * n;  // MODE 1: the tile's source rows
+  const int ls = GAP ? pl.ls : n, tn = L * ls;
+  T2 *Abuf = W + 2 * n;    // two tile buffers
+  T2 *S = Abuf + 2 * tn;   // MODE 1: the tile's source rows
   const int nblk = (n + L - 1) / L, ntiles = ns * nblk;
   const size_t ncell = (size_t)n * n;
   for (int t = threadIdx.x; t < 2 * n - 1; t += blockDim.x) cp_elem(W + t, roots + t);
+  // element t of a tile: row t / n, column t mod n, advanced by the CTA's stride
+  const int c_init = fdiv(threadIdx.x, n, pl.mn), e_init = threadIdx.x - c_init * n;
+  const int dc = fdiv(blockDim.x, n, pl.mn), de = blockDim.x - dc * n;
+  auto load_rows = [&](T2 *dst, const T2 *g, int cnt) {
+    if constexpr (!GAP) {
+      for (int t = threadIdx.x; t < cnt; t += blockDim.x) cp_elem(dst + t, g + t);
+      return;
+    }
+    int c = c_init, e = e_init;
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
+      cp_elem(dst + c * ls + e + gaps<GAP>(e, pl.sh), g + t);
+      c += dc;
+      e += de;
+      if (e >= n) {
+        e -= n;
+        c++;
+      }
+    }
+  };
   int tile = blockIdx.x;
   if (tile < ntiles) {
     const int ii = tile / nblk, r0 = (tile - ii * nblk) * L, cnt = min(L, n - r0) * n;
-    const T2 *g = in + (size_t)((ii + first) % ns) * ncell + (size_t)r0 * n;
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) cp_elem(Abuf + t, g + t);
+    load_rows(Abuf, in + (size_t)((ii + first) % ns) * ncell + (size_t)r0 * n, cnt);
   }
   cp_commit();
   for (int it = 0; tile < ntiles; tile += gridDim.x, it++) {
-    T2 *A = Abuf + (it & 1) * L * n;
+    T2 *A = Abuf + (it & 1) * tn;
     const int ii = tile / nblk, r0 = (tile - ii * nblk) * L, lines = min(L, n - r0), cnt = lines * n;
     const T2 *sb = (MODE == 1 && src) ? src + (size_t)ii * ncell + (size_t)r0 * n : nullptr;
     // the source rows of the epilogue: copied while the rows are transformed
@@ -439,16 +484,14 @@ __global__ void __launch_bounds__(256, (sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CT
     const int nx = tile + gridDim.x;
     if (nx < ntiles) {
       const int jj = nx / nblk, q0 = (nx - jj * nblk) * L, qc = min(L, n - q0) * n;
-      const T2 *g = in + (size_t)((jj + first) % ns) * ncell + (size_t)q0 * n;
-      T2 *dst = Abuf + ((it + 1) & 1) * L * n;
-      for (int t = threadIdx.x; t < qc; t += blockDim.x) cp_elem(dst + t, g + t);
+      load_rows(Abuf + ((it + 1) & 1) * tn, in + (size_t)((jj + first) % ns) * ncell + (size_t)q0 * n, qc);
     }
     cp_commit();
     cp_wait<2>();  // this tile's rows (committed one iteration earlier)
     __syncthreads();
     // the last stage writes the rows to global memory, scaled and with 2 src (MODE 1)
     T2 *o = out + (size_t)((ii + first) % ns) * ncell + (size_t)r0 * n;
-    fft_lines(A, n, lines, pl, W, o, Epilogue<T2, MODE>{(R)scale, sb ? S : nullptr}, sb != nullptr);
+    fft_lines<GAP>(A, lines, pl, W, o, Epilogue<T2, MODE>{(R)scale, sb ? S : nullptr}, sb != nullptr);
     __syncthreads();  // A is free for the copies of the next iteration
   }
   cp_wait<0>();
@@ -466,12 +509,12 @@ __device__ __forceinline__ void phase_sincos(float a, float *sn, float *cs) {
 // Transposed load of columns c0 .. c0 + lines - 1 of slice `g` (rows of n) into
 // lines of `dst` (line c = column c0 + c): thread t takes column t mod 16 of rows
 // t / 16, t / 16 + blockDim / 16, ... (lines <= 16)
-template <typename T2>
-__device__ __forceinline__ void load_cols(T2 *dst, const T2 *g, int n, int c0, int lines) {
-  const int tc = threadIdx.x & 15;
+template <bool GAP, typename T2>
+__device__ __forceinline__ void load_cols(T2 *dst, const T2 *g, const FFTPlan &pl, int c0, int lines) {
+  const int tc = threadIdx.x & 15, n = pl.n;
   if (tc < lines)
     for (int row = threadIdx.x >> 4; row < n; row += blockDim.x >> 4)
-      cp_elem(dst + tc * n + row, g + (size_t)row * n + c0 + tc);
+      cp_elem(dst + tc * (GAP ? pl.ls : n) + row + gaps<GAP>(row, pl.sh), g + (size_t)row * n + c0 + tc);
 }
 
 // Column pass over tiles of L (<= 16) columns: FFT of the columns, the propagator exp(K2
@@ -485,7 +528,7 @@ __device__ __forceinline__ void load_cols(T2 *dst, const T2 *g, int n, int c0, i
 // product of a row and a column factor, exp(i dx^2 k2dz) exp(i dy^2 k2dz), from a table of n
 // entries a CTA forms once (both frequency maps are the same): a sincos per cell, about 35
 // FP64 instructions with its phase, would be a fifth of the pass.
-template <typename T2>
+template <typename T2, bool GAP>
 __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64)
     k_fft_cols(T2 *__restrict__ field, const T2 *__restrict__ srcf, const T2 *__restrict__ roots, double k2dz,
                const typename Real<T2>::T *__restrict__ sigt, FFTPlan pl, int ns, int first, int L) {
@@ -493,9 +536,10 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T2 *W = reinterpret_cast<T2 *>(smem_raw);
   const int n = pl.n;
+  const int ls = GAP ? pl.ls : n, tn = L * ls;
   T2 *Abuf = W + 2 * n;
-  T2 *SA = Abuf + 2 * L * n;  // filtered source columns (only with srcf)
-  T2 *E = SA + (srcf ? L * n : 0);  // FP64: exp(i dx^2 k2dz) by FFT index
+  T2 *SA = Abuf + 2 * tn;         // filtered source columns (only with srcf)
+  T2 *E = SA + (srcf ? tn : 0);   // FP64: exp(i dx^2 k2dz) by FFT index
   const int nblk = (n + L - 1) / L, ntiles = ns * nblk;
   const size_t ncell = (size_t)n * n;
   const R kdz = (R)k2dz, half = (R)(0.5 * (n - 1));
@@ -517,19 +561,19 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
   int tile = blockIdx.x;
   if (tile < ntiles) {
     const int ii = tile / nblk, c0 = (tile - ii * nblk) * L;
-    load_cols(Abuf, field + (size_t)((ii + first) % ns) * ncell, n, c0, min(L, n - c0));
+    load_cols<GAP>(Abuf, field + (size_t)((ii + first) % ns) * ncell, pl, c0, min(L, n - c0));
   }
   cp_commit();
   for (int it = 0; tile < ntiles; tile += gridDim.x, it++) {
-    T2 *A = Abuf + (it & 1) * L * n;
+    T2 *A = Abuf + (it & 1) * tn;
     const int ii = tile / nblk, c0 = (tile - ii * nblk) * L, lines = min(L, n - c0);
     T2 *u = field + (size_t)((ii + first) % ns) * ncell;
-    if (srcf) load_cols(SA, srcf + (size_t)ii * ncell, n, c0, lines);
+    if (srcf) load_cols<GAP>(SA, srcf + (size_t)ii * ncell, pl, c0, lines);
     cp_commit();
     const int nx = tile + gridDim.x;
     if (nx < ntiles) {
       const int jj = nx / nblk, q0 = (nx - jj * nblk) * L;
-      load_cols(Abuf + ((it + 1) & 1) * L * n, field + (size_t)((jj + first) % ns) * ncell, n, q0,
+      load_cols<GAP>(Abuf + ((it + 1) & 1) * tn, field + (size_t)((jj + first) % ns) * ncell, pl, q0,
                 min(L, n - q0));
     }
     cp_commit();
@@ -548,8 +592,9 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
         int c = c_init, ky = ky_init;
         for (int t = threadIdx.x; t < lines * n; t += blockDim.x) {
           T2 v;
+          const int at = GAP ? c * ls + ky + gaps<GAP>(ky, pl.sh) : t;
           if constexpr (sizeof(T2) == 16) {
-            v = cm(cm(A[t], E[c0 + c]), E[ky]);
+            v = cm(cm(A[at], E[c0 + c]), E[ky]);
           } else {
             int ix = c0 + c + off, iy = ky + off;
             ix -= ix >= n ? n : 0;
@@ -557,10 +602,10 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
             const R dx = (R)ix - half, dy = (R)iy - half;
             R sn, cs;
             phase_sincos((dx * dx + dy * dy) * kdz, &sn, &cs);
-            v = cm(A[t], mk<T2>(cs, sn));
+            v = cm(A[at], mk<T2>(cs, sn));
           }
-          if (srcf) v = axpy((R)2 * st[t], SA[t], v);
-          A[t] = mk<T2>(v.y, v.x);
+          if (srcf) v = axpy((R)2 * st[t], SA[at], v);
+          A[at] = mk<T2>(v.y, v.x);
           c += dc;
           ky += dky;
           if (ky >= n) {
@@ -570,12 +615,12 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
         }
         __syncthreads();
       }
-      fft_lines(job == 1 && srcf ? SA : A, n, lines, pl, W);
+      fft_lines<GAP>(job == 1 && srcf ? SA : A, lines, pl, W);
     }
     const int tc = threadIdx.x & 15;
     if (tc < lines)
       for (int row = threadIdx.x >> 4; row < n; row += blockDim.x >> 4)
-        u[(size_t)row * n + c0 + tc] = A[tc * n + row];
+        u[(size_t)row * n + c0 + tc] = A[tc * ls + row + gaps<GAP>(row, pl.sh)];
     __syncthreads();
   }
   cp_wait<0>();
@@ -587,7 +632,7 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
 // power-weighted moments of the tile's elements on the shifted frequency map (dx, dy
 // as in k_fft_cols' propagator). One partial per tile, deterministic:
 // part[(ii nblk + blk) 5 + k] = sum |F|^2, dx |F|^2, dx^2 |F|^2, dy |F|^2, dy^2 |F|^2.
-template <typename T2>
+template <typename T2, bool GAP>
 __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64)
     k_fft_cols_moments(const T2 *__restrict__ work, const T2 *__restrict__ roots, FFTPlan pl, int ns, int first,
                        int L, double *__restrict__ part) {
@@ -596,6 +641,7 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
   __shared__ double red[8][5];
   T2 *W = reinterpret_cast<T2 *>(smem_raw);
   const int n = pl.n;
+  const int ls = GAP ? pl.ls : n, tn = L * ls;
   T2 *Abuf = W + 2 * n;
   const int nblk = (n + L - 1) / L, ntiles = ns * nblk;
   const size_t ncell = (size_t)n * n;
@@ -608,22 +654,22 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
   int tile = blockIdx.x;
   if (tile < ntiles) {
     const int ii = tile / nblk, c0 = (tile - ii * nblk) * L;
-    load_cols(Abuf, work + (size_t)((ii + first) % ns) * ncell, n, c0, min(L, n - c0));
+    load_cols<GAP>(Abuf, work + (size_t)((ii + first) % ns) * ncell, pl, c0, min(L, n - c0));
   }
   cp_commit();
   for (int it = 0; tile < ntiles; tile += gridDim.x, it++) {
-    T2 *A = Abuf + (it & 1) * L * n;
+    T2 *A = Abuf + (it & 1) * tn;
     const int ii = tile / nblk, blk = tile - ii * nblk, c0 = blk * L, lines = min(L, n - c0);
     const int nx = tile + gridDim.x;
     if (nx < ntiles) {
       const int jj = nx / nblk, q0 = (nx - jj * nblk) * L;
-      load_cols(Abuf + ((it + 1) & 1) * L * n, work + (size_t)((jj + first) % ns) * ncell, n, q0,
+      load_cols<GAP>(Abuf + ((it + 1) & 1) * tn, work + (size_t)((jj + first) % ns) * ncell, pl, q0,
                 min(L, n - q0));
     }
     cp_commit();
     cp_wait<1>();
     __syncthreads();
-    fft_lines(A, n, lines, pl, W);
+    fft_lines<GAP>(A, lines, pl, W);
     R m[5] = {0, 0, 0, 0, 0};
     int c = c_init, ky = ky_init;
     for (int t = threadIdx.x; t < lines * n; t += blockDim.x) {
@@ -631,7 +677,7 @@ __global__ void __launch_bounds__(256, sizeof(T2) == 8 ? FFT_CTAS_FP32 : FFT_CTA
       ix -= ix >= n ? n : 0;
       iy -= iy >= n ? n : 0;
       const R dx = (R)ix - half, dy = (R)iy - half;
-      const T2 v = A[t];
+      const T2 v = A[GAP ? c * ls + ky + gaps<GAP>(ky, pl.sh) : t];
       const R w = v.x * v.x + v.y * v.y;
       m[0] += w;
       m[1] += dx * w;
@@ -667,7 +713,9 @@ constexpr int FFT_THREADS = 256;
 
 // Shared memory of a pass with `bufs` tile buffers of L lines and the roots and
 // twiddles (2 n elements).
-size_t fft_smem(int n, int L, int bufs, size_t es) { return (size_t)(2 * n + bufs * L * n) * es; }
+size_t fft_smem(const FFTPlan &pl, int L, int bufs, size_t es) {
+  return (size_t)(2 * pl.n + bufs * L * pl.ls) * es;
+}
 
 // CTAs of a pass resident on one SM: the register bound of its launch bounds,
 // fewer where the shared memory does not allow them.
@@ -691,7 +739,7 @@ int sm_count() {
   return cached[dev];
 }
 
-template <typename T2>
+template <typename T2, bool GAP>
 void launch_fft(void *stream, void *field, const void *src, void *work, const void *roots, double k2c,
                 const void *sig, int filtered, double delz, const FFTPlan &pl, int ns, int first) {
   cudaStream_t s = (cudaStream_t)stream;
@@ -701,9 +749,9 @@ void launch_fft(void *stream, void *field, const void *src, void *work, const vo
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(configured.load() & (1ull << dev))) {
-    cudaFuncSetAttribute(k_fft_rows<T2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(k_fft_rows<T2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaFuncSetAttribute(k_fft_cols<T2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_fft_rows<T2, 0, GAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_fft_rows<T2, 1, GAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_fft_cols<T2, GAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     configured.fetch_or(1ull << dev);
   }
   const int nsm = sm_count();
@@ -720,28 +768,28 @@ void launch_fft(void *stream, void *field, const void *src, void *work, const vo
   typedef typename Real<T2>::T R;
   // forward rows of the field (and, filtered, of the source into the work array)
   const int Lr = fft_lines_per_cta(pl, es, 2, 32, rows_ctas);
-  const size_t mr = fft_smem(n, Lr, 2, (size_t)es);
+  const size_t mr = fft_smem(pl, Lr, 2, (size_t)es);
   const unsigned gr = grid(Lr, mr, rows_ctas);
-  k_fft_rows<T2, 0><<<gr, FFT_THREADS, mr, s>>>(f, f, nullptr, rt, pl, ns, first, 1.0, Lr);
-  if (sfw) k_fft_rows<T2, 0><<<gr, FFT_THREADS, mr, s>>>(sr, sfw, nullptr, rt, pl, ns, 0, 1.0, Lr);
+  k_fft_rows<T2, 0, GAP><<<gr, FFT_THREADS, mr, s>>>(f, f, nullptr, rt, pl, ns, first, 1.0, Lr);
+  if (sfw) k_fft_rows<T2, 0, GAP><<<gr, FFT_THREADS, mr, s>>>(sr, sfw, nullptr, rt, pl, ns, 0, 1.0, Lr);
   // columns
   const int bc = sfw ? 3 : 2;
   const size_t table = es == 16 ? (size_t)n * es : 0;  // the propagator's factors
   const int Lc = fft_lines_per_cta(pl, es, bc, 16, cols_ctas, table);
-  const size_t mc = fft_smem(n, Lc, bc, (size_t)es) + table;
-  k_fft_cols<T2><<<grid(Lc, mc, cols_ctas), FFT_THREADS, mc, s>>>(f, sfw, rt, k2c * delz, (const R *)sig, pl,
+  const size_t mc = fft_smem(pl, Lc, bc, (size_t)es) + table;
+  k_fft_cols<T2, GAP><<<grid(Lc, mc, cols_ctas), FFT_THREADS, mc, s>>>(f, sfw, rt, k2c * delz, (const R *)sig, pl,
                                                                  ns, first, Lc);
   // inverse rows, 1/n^2, + 2 src when unfiltered (the source rows in a third tile
   // buffer, at one CTA per SM fewer)
   const T2 *s1 = filtered ? nullptr : sr;
   const int c1 = rows_ctas - 1;
   const int L1 = fft_lines_per_cta(pl, es, s1 ? 3 : 2, 32, c1);
-  const size_t m1 = fft_smem(n, L1, s1 ? 3 : 2, (size_t)es);
-  k_fft_rows<T2, 1><<<grid(L1, m1, c1), FFT_THREADS, m1, s>>>(f, f, s1, rt, pl, ns, first, 1.0 / ((double)n * n),
+  const size_t m1 = fft_smem(pl, L1, s1 ? 3 : 2, (size_t)es);
+  k_fft_rows<T2, 1, GAP><<<grid(L1, m1, c1), FFT_THREADS, m1, s>>>(f, f, s1, rt, pl, ns, first, 1.0 / ((double)n * n),
                                                               L1);
 }
 
-template <typename T2>
+template <typename T2, bool GAP>
 void launch_fft_diag_t(void *stream, const void *field, void *work, const void *roots, const FFTPlan &pl, int ns,
                        int first, double *part, int L) {
   cudaStream_t s = (cudaStream_t)stream;
@@ -751,9 +799,9 @@ void launch_fft_diag_t(void *stream, const void *field, void *work, const void *
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(configured.load() & (1ull << dev))) {
-    cudaFuncSetAttribute(k_fft_rows<T2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(k_fft_rows<T2, 0, GAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     // (the kernel's static reduction array counts against the 227 KB too)
-    cudaFuncSetAttribute(k_fft_cols_moments<T2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+    cudaFuncSetAttribute(k_fft_cols_moments<T2, GAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
     configured.fetch_or(1ull << dev);
   }
   const int ctas = es == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64;
@@ -764,11 +812,11 @@ void launch_fft_diag_t(void *stream, const void *field, void *work, const void *
     return (unsigned)(tiles < cap ? tiles : cap);
   };
   const int Lr = fft_lines_per_cta(pl, es, 2, 32, ctas);
-  const size_t mr = fft_smem(n, Lr, 2, (size_t)es);
-  k_fft_rows<T2, 0><<<grid(Lr, mr), FFT_THREADS, mr, s>>>((const T2 *)field, (T2 *)work, nullptr, (const T2 *)roots,
+  const size_t mr = fft_smem(pl, Lr, 2, (size_t)es);
+  k_fft_rows<T2, 0, GAP><<<grid(Lr, mr), FFT_THREADS, mr, s>>>((const T2 *)field, (T2 *)work, nullptr, (const T2 *)roots,
                                                           pl, ns, first, 1.0, Lr);
-  const size_t mc = fft_smem(n, L, 2, (size_t)es);
-  k_fft_cols_moments<T2><<<grid(L, mc), FFT_THREADS, mc, s>>>((const T2 *)work, (const T2 *)roots, pl, ns, first, L,
+  const size_t mc = fft_smem(pl, L, 2, (size_t)es);
+  k_fft_cols_moments<T2, GAP><<<grid(L, mc), FFT_THREADS, mc, s>>>((const T2 *)work, (const T2 *)roots, pl, ns, first, L,
                                                               part);
 }
 
@@ -789,8 +837,20 @@ int fft_lines_per_cta(const FFTPlan &pl, int es, int bufs, int maxL, int per_sm,
   }
   if (L < 1) L = 1;
   const size_t cap = 228u * 1024u / per_sm - 1024;
-  while (L > 1 && fft_smem(n, L, bufs, es) + table > cap) L--;
+  while (L > 1 && fft_smem(pl, L, bufs, es) + table > cap) L--;
   return L;
+}
+
+// Gaps where the first radix is 4, 8 or 16 and every stage has a register radix, while a line
+// with them is small against shared memory. (Radix 2 first, n = 250: 2190 us without, 2360 with.)
+void fft_tile_layout(FFTPlan &pl) {
+  pl.ls = pl.n;
+  pl.sh = kFftFlat;
+  if (pl.n % 4 || pl.n > 1024) return;
+  for (int s = 0; s < pl.nstage; s++)
+    if (!register_radix(pl.radix[s])) return;
+  pl.sh = pl.radix[0] == 16 ? 4 : pl.radix[0] == 8 ? 3 : 2;
+  pl.ls = (pl.n + (pl.n >> pl.sh)) | 1;
 }
 
 int fft_max_ngrid(int mixed) {
@@ -821,19 +881,21 @@ int fft_diag_lines(const FFTPlan &pl, int mixed) {
 void launch_fft_diag(void *stream, int mixed, const void *field, void *work, const void *roots, const FFTPlan &pl,
                      int ns, int first, double *part) {
   const int L = fft_diag_lines(pl, mixed);
+  const bool gap = pl.sh != kFftFlat;
   if (mixed)
-    launch_fft_diag_t<float2>(stream, field, work, roots, pl, ns, first, part, L);
+    (gap ? launch_fft_diag_t<float2, true> : launch_fft_diag_t<float2, false>)(stream, field, work, roots, pl, ns, first, part, L);
   else
-    launch_fft_diag_t<double2>(stream, field, work, roots, pl, ns, first, part, L);
+    (gap ? launch_fft_diag_t<double2, true> : launch_fft_diag_t<double2, false>)(stream, field, work, roots, pl, ns, first, part, L);
 }
 
 void launch_fft_solve(void *stream, int mixed, void *field, const void *src, void *work, const void *roots,
                       double k2c, const void *sig, int filtered, double delz, const FFTPlan &pl, int ns,
                       int first) {
+  const bool gap = pl.sh != kFftFlat;
   if (mixed)
-    launch_fft<float2>(stream, field, src, work, roots, k2c, sig, filtered, delz, pl, ns, first);
+    (gap ? launch_fft<float2, true> : launch_fft<float2, false>)(stream, field, src, work, roots, k2c, sig, filtered, delz, pl, ns, first);
   else
-    launch_fft<double2>(stream, field, src, work, roots, k2c, sig, filtered, delz, pl, ns, first);
+    (gap ? launch_fft<double2, true> : launch_fft<double2, false>)(stream, field, src, work, roots, k2c, sig, filtered, delz, pl, ns, first);
 }
 
 }  // namespace g4
