@@ -190,17 +190,17 @@ def job_value(ws, slices_per_rank, steps, ms_max):
 
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per slice of one launch,
-# from the ncu --set full capture of a 608-slice window of the same workload
-# (profiles/ncu_full_k_push_f_k_field_fused_f_sase608.md); the traffic of these kernels
+# from ncu captures of a 608-slice window of the same workload
+# (profiles/ncu_step_kernels.md); the traffic of these kernels
 # grows in proportion to the slices of a launch, so a full launch's is the per-slice
 # figure times the slices.
-TRAFFIC_PER_SLICE = {"field": 447986.0, "push": 431960.0}
+TRAFFIC_PER_SLICE = {"field": 450200.0, "push": 428300.0}
 TRAFFIC_SOURCE = "ncu capture of a 608-slice window, scaled to the launch's slices"
 # FP64 instructions (DFMA + DMUL + DADD, thread level) per particle of the plain push and
-# per cell of each plain ADI sweep, from ncu captures of a 152-slice window
-# (profiles/ncu_fp64_k_push_k_adi_plain_sase152.md); nominal GB300 FP64 rate: 1.25 TFLOP/s
+# per cell of the plain ADI's row and column pass, from ncu captures of a 152-slice window
+# (profiles/ncu_step_kernels.md); nominal GB300 FP64 rate: 1.25 TFLOP/s
 # with FMA counted as two operations, i.e. 625 G FP64 instructions/s.
-FP64_INSTR = {"push_per_particle": 414.1, "adi_per_cell": 17.9}
+FP64_INSTR = {"push_per_particle": 222.1, "rows_per_cell": 20.7, "cols_per_cell": 14.7}
 FP64_NOMINAL_GINSTR = 625.0
 
 
@@ -222,8 +222,8 @@ def fp64_roofline(kernels_plain, peak_ginstr, peak_source):
     out = {"bound": "fp64", "peak_ginstr_s": peak_ginstr, "peak_source": peak_source,
            "instr_source": "ncu dfma+dmul+dadd counts of a 152-slice capture"}
     for k, n in (("push", NS * NPART * FP64_INSTR["push_per_particle"]),
-                 ("adi_x", NS * NGRID * NGRID * FP64_INSTR["adi_per_cell"]),
-                 ("adi_y", NS * NGRID * NGRID * FP64_INSTR["adi_per_cell"])):
+                 ("adi_x", NS * NGRID * NGRID * FP64_INSTR["rows_per_cell"]),
+                 ("adi_y", NS * NGRID * NGRID * FP64_INSTR["cols_per_cell"])):
         if k in kernels_plain:
             g = n / (kernels_plain[k]["ms_avg"] / 1e3) / 1e9
             out[k] = {"ginstr_s": g, "frac": g / peak_ginstr}

@@ -100,8 +100,8 @@ struct g4gpu_ctx {
   // launch shapes (chosen by g4gpu_autotune, defaults otherwise; 0: by the window's size)
   int push_block = 0;
   int field_threads = 0;
-  // mixed ADI with the slice in shared memory: 0 one CTA per slice (k_field_fused_f),
-  // 1 a cluster pair (k_field_band_f<2>), 2 the whole step per CTA (k_step_fused_f)
+  // mixed ADI with the slice on chip: 0 one CTA per slice or a cluster by the window's size
+  // (k_field_tm_f, k_field_cl_f), 1 a cluster pair, 2 the whole step per CTA (k_step_fused_f)
   int field_kernel = 0;
 
   // captured step sequences, keyed by the step range and the ring state they start from

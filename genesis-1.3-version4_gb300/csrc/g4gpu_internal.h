@@ -168,7 +168,8 @@ void launch_diag_field_mixed(const Launch &L, const void *field, int ns, int ngr
 // for ngrid <= fused_max_ngrid() (168: the FP32 slice must fit in 227 KB).
 int fused_max_ngrid();
 // The same step on a thread-block cluster of cl CTAs per slice (2 <= cl <=
-// kMaxBandCluster), each holding a band of the rows; usable when the step's segmented
+// kMaxBandCluster), each holding a band of the rows (where launch_field_cluster_mixed does
+// not fit: long warm-ups); usable when the step's segmented
 // solves apply (FieldStep::tw > 0). band_cluster(ngrid, W) gives the smallest cluster
 // whose bands fit shared memory with the last band at least W rows (the segments'
 // warm-up), or 0 if none does.

@@ -401,11 +401,12 @@ int g4gpu_set_graph_mode(g4gpu_handle h, int on);
 int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_threads, int *field_kernel);
 /* Sets the launch shapes g4gpu_autotune would choose: push_block a multiple of 32 in
  * [32, 512], field_threads a multiple of 32 in [2 ngrid, 1024] (mixed ADI form; the kernel
- * that keeps a slice's stencil term in tensor memory takes at most 768 of them), and
- * field_kernel 0, 1 or 2; other values are rejected with G4GPU_ERR_ARG. The pair kernel
- * runs only where its segmented solves apply, the whole-step kernel only on one-field
- * windows without space charge; elsewhere the single-CTA field kernel does. No
- * reference counterpart. */
+ * that keeps a slice's stencil term in tensor memory takes at most 768 of them, and its
+ * cluster form, for windows of few slices and large grids, a size of its own), and
+ * field_kernel 0, 1 (a pair of CTAs a slice) or 2 (the whole step in one kernel); other
+ * values are rejected with G4GPU_ERR_ARG. The pair runs only where its segmented solves
+ * apply, the whole-step kernel only on one-field windows without space charge; elsewhere
+ * field_kernel 0 does. No reference counterpart. */
 int g4gpu_set_launch_shapes(g4gpu_handle h, int push_block, int field_threads, int field_kernel);
 
 /* A batch owns nrun independent handles (one time window each, with its own
