@@ -74,6 +74,7 @@ StepConstF to_float(const StepConst &s, int npart) {
   f.autophase = s.autophase;
   f.autophase_q = (long long)llrint(s.autophase * (4294967296.0 / kTwoPiHost));
   f.gammaref = s.gammaref;
+  f.g0 = (float)s.gammaref;
   f.chic = s.chic;
   for (int i = 0; i < 8; i++) f.cm[i] = (float)s.cm[i];
   f.r56 = (float)s.r56;
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(256) k_deposit_f(StepConstF sc, PtrsF p, int n
   const bool valid = ip < slice_np_f(p, is, np);
   size_t o = (size_t)is * np + (valid ? ip : 0);
   deposit_f<NF>(sc, p, (size_t)is * (size_t)ng * ng, ng, slice_cur_f(p, is, np),
-                (float)sc.gammaref + p.dg[o], p.theta[o], p.x[o], p.y[o], valid);
+                sc.g0 + p.dg[o], p.theta[o], p.x[o], p.y[o], valid);
 }
 
 struct CoefF {
@@ -820,7 +821,7 @@ __device__ __forceinline__ void deposit_lanes(const StepConstF &sc, const FieldS
   bool on = ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c) && !ng.outside(c.iy);
   float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (on) {
-    float g = (float)sc.gammaref + dgam;
+    float g = sc.g0 + dgam;
     float dx = x - sc.ax, dy = y - sc.ay;
     float faw2 = 1.f + sc.kx * dx * dx + sc.ky * dy * dy + 2.f * (sc.gradx * dx + sc.grady * dy);
     float part = sqrtf(faw2) * scl / g;
@@ -908,7 +909,7 @@ __device__ __forceinline__ void deposit_one(const StepConstF &sc, const FieldSte
   if (!ll_gridpoint_f(fs.gridmax, fs.dgrid, ng, x, y, c) || ng.outside(c.iy)) return;
   float dx = x - sc.ax, dy = y - sc.ay;
   float faw2 = 1.f + sc.kx * dx * dx + sc.ky * dy * dy + 2.f * (sc.gradx * dx + sc.grady * dy);
-  float part = sqrtf(faw2) * scl / ((float)sc.gammaref + dgam);
+  float part = sqrtf(faw2) * scl / (sc.g0 + dgam);
   float sn, co;
   __sincosf(phase_of(th, (unsigned)fs.harm), &sn, &co);
   float cpx = sn * part, cpy = co * part;
@@ -931,7 +932,7 @@ __device__ __forceinline__ void deposit_group(const StepConstF &sc, const FieldS
   float cpx = 0.f, cpy = 0.f;
 #pragma unroll
   for (int m = 0; m < N; m++) {
-    float part = a / ((float)sc.gammaref + dgam[m]);
+    float part = a / (sc.g0 + dgam[m]);
     float sn, co;
     __sincosf(phase_of(th[m], (unsigned)fs.harm), &sn, &co);
     cpx += sn * part;
@@ -979,7 +980,7 @@ __device__ __forceinline__ bool deposit_cell4(const StepConstF &sc, const FieldS
   if (!same) return false;
   const int ix = min((int)fx, ng.ng - 1), iy = min((int)fy, ng.ng - 1);
   if (ng.outside(iy)) return true;  // the rows are another band's
-  const float g0 = (float)sc.gammaref;
+  const float g0 = sc.g0;
   float2 v00 = make_float2(0.f, 0.f), v10 = v00, v01 = v00, v11 = v00;
 #pragma unroll
   for (int m = 0; m < 4; m++) {
@@ -1512,7 +1513,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     const float2 *fslice[1] = {u};
     const size_t base = (size_t)is * np;
     const int lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
-    const float g0 = (float)sc.gammaref;
+    const float g0 = sc.g0;
     const float ez = p.eloss ? (float)p.eloss[is] : 0.f;
     for (int w0 = warp * 32 * U; w0 < n; w0 += nwarp * 32 * U) {
       float dg[U], x[U], y[U], px[U], py[U];
@@ -2063,7 +2064,7 @@ __device__ __forceinline__ void pair_group(const StepConstF &sc, const FieldStep
   float a = sqrtf(faw2) * scl;
   float cpx = 0.f, cpy = 0.f;
   for (int m = 0; m < n; m++) {
-    float part = a / ((float)sc.gammaref + dgam[m]);
+    float part = a / (sc.g0 + dgam[m]);
     float sn, co;
     __sincosf(phase_of(th[m], (unsigned)fs.harm), &sn, &co);
     cpx += sn * part;
@@ -2096,7 +2097,7 @@ __device__ __forceinline__ bool pair_cell4(const StepConstF &sc, const FieldStep
     cell_rc(fs.gridmax, fs.dgrid, ng, x[m], y[m], cm);
     const float dx = x[m] - sc.ax, dy = y[m] - sc.ay;
     const float faw2 = 1.f + sc.kx * dx * dx + sc.ky * dy * dy + 2.f * (sc.gradx * dx + sc.grady * dy);
-    const float part = sqrtf(faw2) * scl / ((float)sc.gammaref + dgam[m]);
+    const float part = sqrtf(faw2) * scl / (sc.g0 + dgam[m]);
     float sn, co;
     __sincosf(phase_of(th[m], (unsigned)fs.harm), &sn, &co);
     const float cpx = sn * part, cpy = co * part;
