@@ -108,12 +108,13 @@ __device__ __forceinline__ void solve_lines(const Lines &s, int nline, int lstri
 // Tile T [L][ng | 1]: an odd row stride, so that the lanes of a warp, which walk L rows
 // at once, read 16-byte elements of different banks.
 template <int L>
-__global__ void k_adi_rows(const double2 *__restrict__ field, double2 *__restrict__ src, double2 *__restrict__ tmp,
+__global__ void k_adi_rows(const double2 *field, double2 *src, double2 *tmp,
                            Coef cf, double c, int ns, int ng, int first, int nband, int nseg, int nco, int W,
                            int has_src) {
   extern __shared__ __align__(16) unsigned char adi_smem[];
   const int st1 = ng | 1;
-  const Lines ln = lines_setup(adi_smem, L, nseg, nco, W, ng, cf);
+  const Lines ln = lines_setup(adi_smem, L, nseg, nco, W, ng, cf);  // tables: no kernel writes them
+  chain_wait();
   C2 *T = ln.T;
   const int ii = blockIdx.x / nband, r0 = (blockIdx.x - ii * nband) * L, nr = min(L, ng - r0);
   const size_t ncell = (size_t)ng * ng;
@@ -149,11 +150,11 @@ __global__ void k_adi_rows(const double2 *__restrict__ field, double2 *__restric
 
 // Tile T [ng][L].
 template <int L>
-__global__ void k_adi_cols(double2 *__restrict__ field, const double2 *__restrict__ s1,
-                           const double2 *__restrict__ tmp, Coef cf, double c, int ns, int ng, int first, int nband,
+__global__ void k_adi_cols(double2 *field, const double2 *s1, const double2 *tmp, Coef cf, double c, int ns, int ng, int first, int nband,
                            int nseg, int nco, int W) {
   extern __shared__ __align__(16) unsigned char adi_smem[];
-  const Lines ln = lines_setup(adi_smem, L, nseg, nco, W, ng, cf);
+  const Lines ln = lines_setup(adi_smem, L, nseg, nco, W, ng, cf);  // tables: no kernel writes them
+  chain_wait();
   C2 *T = ln.T;
   const int ii = blockIdx.x / nband, c0 = (blockIdx.x - ii * nband) * L, nc = min(L, ng - c0);
   const size_t ncell = (size_t)ng * ng;

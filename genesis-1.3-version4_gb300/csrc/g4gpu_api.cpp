@@ -1890,14 +1890,15 @@ namespace {
 // take the place and the pipes of CTAs of the step that would all have run at once. In line /
 // beside, us a step: mixed 1 x 8192 particles, 151^2 40 / 29, 22 x 4096 37 / 30, 75 x 8192
 // 53 / 62, 300 x 8192, 101^2 98 / 102, 300 x 8192, 255^2 297 / 279, 700 x 4096 212 / 196,
-// 2048 x 8192 596 / 567; FP64 1 x 8192, 255^2 91 / 78, 2 x 8192 106 / 108, 22 x 2052 98 / 121,
-// 64 x 4096 312 / 304, 150 x 2048 357 / 337, 320 x 8192 1974 / 1935.
+// 2048 x 8192 596 / 567; FP64 1 x 8192, 255^2 87 / 77, 2 x 8192, 151^2 70 / 62, 255^2 106 / 108,
+// 22 x 2052, 101^2 94 / 119, 64 x 4096 243 / 252, 64 x 4096, 151^2 310 / 303, 150 x 2048, 101^2
+// 354 / 338, 320 x 8192, 151^2 1969 / 1933.
 bool records_beside(g4gpu_handle h, int istep0, int nsteps) {
   const g4gpu_config &c = h->cfg;
   if (h->prof || h->field_kernel == 2) return false;
   for (int s = istep0; s < istep0 + nsteps && s < (int)h->substeps.size(); s++)
     if (h->substeps[s] > 1) return false;
-  if (!h->mixed) return c.nslice == 1 || c.nslice >= 64;
+  if (!h->mixed) return c.nslice * c.ngrid <= 304 || c.nslice >= 64;  // lines: two a SM
   const int cluster = c.solver == G4GPU_SOLVER_ADI ? g4::field_cluster(c.ngrid, c.nslice, h->steps[istep0].f[0].tw) : 0;
   return c.nslice <= 38 || c.nslice * std::max(cluster, 1) >= 608;  // a quarter of, or four times the SMs
 }

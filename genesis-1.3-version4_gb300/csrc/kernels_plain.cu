@@ -16,6 +16,7 @@
 #include <atomic>
 
 #include "g4gpu_internal.h"
+#include "launch_chain.cuh"
 #include "philox.cuh"
 
 namespace g4 {
@@ -453,6 +454,7 @@ __device__ __forceinline__ int slice_np(const Ptrs &p, int is, int np) {
 template <int NF>
 __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int np, int ng,
                                               int deposit) {
+  chain_wait();
   int is = blockIdx.y;
   int ip = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = slice_np(p, is, np);
@@ -876,10 +878,10 @@ void launch_push_plain_sc(const Launch &L, const StepConst &sc, const DeviceBeam
   dim3 grid((np + block - 1) / block, ns);
   cudaStream_t s = (cudaStream_t)L.stream;
   switch (sc.nfld) {
-    case 1: k_push<1><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
-    case 2: k_push<2><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
-    case 3: k_push<3><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
-    default: k_push<G4GPU_MAX_FIELDS><<<grid, block, 0, s>>>(sc, p, ns, np, ngrid, deposit); break;
+    case 1: chain_launch(k_push<1>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
+    case 2: chain_launch(k_push<2>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
+    case 3: chain_launch(k_push<3>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
+    default: chain_launch(k_push<G4GPU_MAX_FIELDS>, grid, block, 0, s, 0, sc, p, ns, np, ngrid, deposit); break;
   }
   // every particle's phasor now matches its phase (bytes of 1: a nonzero flag)
   if (p.phasor) cudaMemsetAsync((void *)p.phasor_ok, 1, sizeof(int), s);
@@ -953,11 +955,11 @@ void launch_adi_lines(cudaStream_t st, int phase, const AdiShape &a, double2 *fi
   const size_t smem = adi64::lines_bytes(L, L * (phase == 0 ? ng | 1 : ng), a.nseg, nco, W);
   const unsigned blocks = (unsigned)ns * (unsigned)nband;
   if (phase == 0)
-    adi64::k_adi_rows<L><<<blocks, a.threads, smem, st>>>(field, src, tmp, cf, c, ns, ng, first, nband, a.nseg, nco,
-                                                          W, has_src);
+    chain_launch(adi64::k_adi_rows<L>, blocks, a.threads, smem, st, 0, field, src, tmp, cf, c, ns, ng, first, nband, a.nseg,
+                 nco, W, has_src);
   else
-    adi64::k_adi_cols<L><<<blocks, a.threads, smem, st>>>(field, src, tmp, cf, c, ns, ng, first, nband, a.nseg, nco,
-                                                          W);
+    chain_launch(adi64::k_adi_cols<L>, blocks, a.threads, smem, st, 0, field, src, tmp, cf, c, ns, ng, first, nband, a.nseg,
+                 nco, W);
 }
 }  // namespace
 

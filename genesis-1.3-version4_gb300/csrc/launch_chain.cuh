@@ -8,11 +8,13 @@
 // allocation). All CTAs of a kernel have started before the next one's appear, so no CTA can
 // wait for one that has no room. Kernels launched in the ordinary way wait for all of it.
 //
-// Used by the mixed form's push and field step: 221 steps of one slice of 151^2
-// 4.50 -> 4.16 ms, 48 steps of 150 slices of 117^2 with its copies 4.95 -> 4.66 ms, windows that
-// fill the chip unchanged. Not by the FP64 kernels, which it slowed down (111 steps of one
-// slice 8.65 -> 9.24 ms, 60 of 22 slices 6.46 -> 8.16): CTAs that are placed while the kernel
-// before runs share an SM, and its FP64 pipe, where they would have had one each.
+// Used by the mixed form's push and field step: 221 steps of one slice of 151^2 4.50 -> 4.16 ms,
+// 48 steps of 150 slices of 117^2 with its copies 4.95 -> 4.66 ms, windows that fill the chip
+// unchanged. The FP64 push and segmented ADI wait likewise but never call chain_next: their
+// successors appear when the last CTA has ended, without the launch in between (a step without
+// records of 1 x 8192 particles, 255^2 67.4 -> 60.5 us, 22 x 2052, 101^2 70.5 -> 66.3). With
+// chain_next at their start CTAs placed beside the running kernel's shared an SM's FP64 pipe
+// where they would have had one each: 60 steps of 22 slices with records 6.46 -> 8.16 ms.
 #pragma once
 #include <cuda_runtime.h>
 
