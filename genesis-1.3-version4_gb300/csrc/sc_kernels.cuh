@@ -41,7 +41,6 @@ namespace {
 
 constexpr int kScThreads = 256;
 constexpr int kScScanChunk = 2048;
-constexpr int kScBatch = 4;
 
 template <typename T>
 __device__ __forceinline__ T sc_warp_sum(T v) {
@@ -414,7 +413,7 @@ __global__ void __launch_bounds__(kScThreads) k_sc_moments(ScBeam<F> b, typename
 
 // Long-range loss and short-range field of one slice. ez: [ns][np] (may be null when
 // the short-range part is off); smem: modes_per_pass * ng * (R2 + R).
-template <class F>
+template <class F, int kScBatch>
 __global__ void __launch_bounds__(kScThreads) k_sc_field(ScBeam<F> b, double *st, typename F::R *ez, ScConst c) {
   using R = typename F::R;
   using R2 = typename F::R2;
@@ -589,7 +588,8 @@ void sc_launch(const Launch &L, const ScConst &c, const typename F::Step &step, 
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(configured.load() & (1ull << dev))) {
-    cudaFuncSetAttribute(k_sc_field<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_max_smem());
+    cudaFuncSetAttribute(k_sc_field<F, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_max_smem());
+    cudaFuncSetAttribute(k_sc_field<F, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_max_smem());
     configured.fetch_or(1ull << dev);
   }
   cudaStream_t s = (cudaStream_t)L.stream;
@@ -598,7 +598,11 @@ void sc_launch(const Launch &L, const ScConst &c, const typename F::Step &step, 
     return;
   }
   const size_t smem = c.shortrange ? (size_t)c.modes_per_pass * sc_bytes_per_mode(c.ng, !F::kPlain) : 0;
-  k_sc_field<F><<<c.ns, kScThreads, smem, s>>>(sb, buf.st, (typename F::R *)buf.ez, c);
+  // particles' loads issued together: four with one or two modes, two with more, where the
+  // modes' arithmetic hides them and four cost registers (4096 x 8192, FP32: 1, 6, 15 modes 397,
+  // 953, 1834 us by fours, 402, 890, 1660 by twos)
+  const bool few = (2 * c.nphi + 1) * c.nz <= 2;
+  (few ? k_sc_field<F, 4> : k_sc_field<F, 2>)<<<c.ns, kScThreads, smem, s>>>(sb, buf.st, (typename F::R *)buf.ez, c);
 }
 
 }  // namespace
