@@ -162,15 +162,25 @@ __global__ void k_adi_cols(double2 *field, const double2 *s1, const double2 *tmp
   const double2 *a = s1 + (size_t)ii * ncell + c0;
   const double2 *w = tmp + (size_t)ii * ncell + c0;
   const int line = threadIdx.x % L, row0 = threadIdx.x / L, dr = blockDim.x / L;
+  // with `edge` also the term of the columns whose cbet in the row solve has not settled
+  // (column_tables)
+  const C2 fix = c0 + line < nco ? ld(cf.pw + 3 * kSegPow + c0 + line) : C2{0, 0};
+  auto fill = [&](bool edge) {
 #pragma unroll 4
-  for (int r = row0; r < ng; r += dr) {
-    C2 v = {0, 0};
-    if (line < nc) {
-      const C2 wv = ld(w + (size_t)r * ng + line), av = ld(a + (size_t)r * ng + line);
-      v = C2{fma(2., wv.x, -av.x), fma(2., wv.y, -av.y)};
+    for (int r = row0; r < ng; r += dr) {
+      C2 v = {0, 0};
+      if (line < nc) {
+        const C2 wv = ld(w + (size_t)r * ng + line), av = ld(a + (size_t)r * ng + line);
+        v = C2{fma(2., wv.x, -av.x), fma(2., wv.y, -av.y)};
+        if (edge) v = sub_cmul(v, C2{-fix.x, -fix.y}, wv);
+      }
+      T[r * L + line] = v;
     }
-    T[r * L + line] = v;
-  }
+  };
+  if (c0 < nco)
+    fill(true);
+  else
+    fill(false);
   __syncthreads();
   solve_lines(ln, L, 1, L, ng, nseg, nco, W, c);
   if (line < nc)

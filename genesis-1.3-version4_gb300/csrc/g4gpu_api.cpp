@@ -163,6 +163,60 @@ void adi_coefficients(double delz, double dgrid, double xks, int ngrid, std::vec
   }
 }
 
+// Two tables of kSegPow entries for the steps whose second right-hand side is 2 u' - S1
+// (adi_plain.cuh, field_tm.cuh): cbet of the column solve, whose last entry is the settled
+// value, and what the first columns add to 2 u' - S1, as a multiple of u'. A rounded cbet
+// scales every solution by 1 + e, the same e in every step, which outgrows the random
+// roundings; 2 u' - S1 carries the row solve's e twice. The column solve's cbet is therefore
+// the rounded (1 - 2 e) beta: what is left of a step's 3 e is the rounding of one number.
+// Before it settles, cbet has another e in every entry, so the FP64 solve's first columns add
+// their 2 (e - e_j) u'. Field of 151^2 after 100 FP64 steps of factor 0.034, rms error against
+// extended precision 1.25e-14 -> 3.1e-15 (8.2e-15 with the stencil's second right-hand side and
+// cbet for both); after 60 mixed steps, against FP64, 4.0e-6 -> 1.2e-6 (3.9e-6).
+// The exact beta_i = 1 / (w2 - c cwet_i) = 1 / (1 + 2 i r + r^2 beta_{i-1}) is cbet[i] + low[i]:
+// one Newton step from the residual, formed with exact products.
+std::vector<std::complex<double>> column_tables(const std::vector<std::complex<double>> &cbet, double r, bool mixed) {
+  typedef std::complex<double> cd;
+  struct Two {
+    double hi, lo;
+  };
+  auto prod = [](double a, double b) { return Two{a * b, std::fma(a, b, -a * b)}; };
+  auto sum = [](double a, double b) {
+    const double s = a + b, t = s - a;
+    return Two{s, (a - (s - t)) + (b - t)};
+  };
+  const int n = (int)cbet.size();
+  const Two r2 = prod(r, r);
+  std::vector<cd> low(n);
+  for (int i = 0; i < n; i++) {
+    Two tr{1, 0}, ti{2 * r, 0};
+    if (i > 0) {
+      const cd b = cbet[i - 1], l = low[i - 1];
+      const Two pr = prod(r2.hi, b.real()), pi = prod(r2.hi, b.imag());
+      tr = sum(1, pr.hi);
+      tr.lo += pr.lo + r2.lo * b.real() + r2.hi * l.real();
+      ti = sum(2 * r, pi.hi);
+      ti.lo += pi.lo + r2.lo * b.imag() + r2.hi * l.imag();
+    }
+    const cd b = cbet[i];
+    const Two rr = prod(tr.hi, b.real()), ii = prod(ti.hi, b.imag()), ri = prod(tr.hi, b.imag()),
+              ir = prod(ti.hi, b.real());
+    const cd e((((1 - rr.hi) + ii.hi) - rr.lo) + ii.lo - tr.lo * b.real() + ti.lo * b.imag(),
+               -(((ri.hi + ir.hi) + ri.lo) + ir.lo + tr.lo * b.imag() + ti.lo * b.real()));
+    low[i] = b * e;
+  }
+  // the row solve's settled cbet, as its kernel holds it, relative to beta
+  const cd bs = cbet[n - 1], held = mixed ? cd((float)bs.real(), (float)bs.imag()) : bs;
+  const cd e = ((held - bs) - low[n - 1]) / bs;
+  std::vector<cd> out(2 * g4::kSegPow);
+  for (int j = 0; j < g4::kSegPow; j++) {
+    const int i = std::min(j, n - 1);
+    out[j] = cbet[i] + (low[i] - 2. * e * cbet[i]);
+    out[g4::kSegPow + j] = 2. * (e + low[i] / cbet[i]);
+  }
+  return out;
+}
+
 // Warm-up length of the segmented tridiagonal solve for one coefficient set. Both
 // recurrences of the Thomas algorithm, d_k = (r_k - c_k d_{k-1}) cbet_k forward and
 // x_k = d_k - cwet_{k+1} x_{k+1} backward, forget their starting value by the factor
@@ -439,7 +493,7 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
   typedef std::complex<double> cd;
   std::map<std::pair<int, double>, int> sets;  // (field, delz) -> set
   std::vector<cd> coefs;                       // [nset][3][ng]
-  std::vector<cd> pows;                        // [nset][2][kSegPow]
+  std::vector<cd> pows;                        // [nset][4][kSegPow]
   std::vector<int> set_tw;                     // warm-up length per coefficient set
   for (int i = 0; i < nsteps; i++) {
     const double *r = tab + (size_t)i * G4GPU_LAT_NCOL;
@@ -535,6 +589,8 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
           }
           pows.insert(pows.end(), pw.begin(), pw.end());
           for (const cd &v : pw) pows.push_back(v * q);
+          pw = column_tables(cb, cs, h->mixed);
+          pows.insert(pows.end(), pw.begin(), pw.end());
         }
         it = sets.find(key);
       }
@@ -942,9 +998,9 @@ int g4gpu_get_field(g4gpu_handle h, int ifld, double *field, int *first, double 
   return check_device_flag(h);
 }
 
-// The powers of a coefficient set's segmented solves.
+// The tables of a coefficient set's segmented solves (kSegPow).
 static const void *seg_powers(g4gpu_handle h, int set) {
-  return (const char *)h->seg_pow + (size_t)set * 2 * g4::kSegPow * h->csize;
+  return (const char *)h->seg_pow + (size_t)set * 4 * g4::kSegPow * h->csize;
 }
 // Threads a CTA of the fused field kernel: as set, else by the grid and the window.
 static int field_threads(g4gpu_handle h, int W) {

@@ -29,7 +29,7 @@ struct g4gpu_ctx {
   void *diag_work = nullptr;  // g4gpu_diag_fft's scratch where tmp is absent
   void *coef = nullptr;      // [nset][3][ngrid] complex of the field type
   size_t coef_bytes = 0;
-  void *seg_pow = nullptr;   // [nset][2][kSegPow] powers (complex of the field type) of the segmented solves
+  void *seg_pow = nullptr;   // [nset][4][kSegPow] tables (complex of the field type) of the segmented solves
   size_t seg_pow_bytes = 0;
   // FFT solver tables per field: roots of unity [n], Im(K2) and the sigmoid [n^2]
   void *fft_roots[G4GPU_MAX_FIELDS] = {};

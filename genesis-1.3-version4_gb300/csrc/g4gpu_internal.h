@@ -16,8 +16,9 @@ constexpr double kVacimp = 376.73;
 constexpr double kEev = 510998.95069;
 constexpr double kCe = 4.8032045e-11;
 
-// Entries of a coefficient set's powers for the FP64 segmented solves: the largest
-// warm-up length segment_warmup returns for 62 bits
+// Entries of a coefficient set's four tables for the segmented solves: kappa^{j+1},
+// kappa^{j+1} / (1 - kappa^2), cbet of the column solve and the first columns' factors
+// (column_tables, g4gpu_api.cpp): the largest warm-up length segment_warmup returns for 62 bits
 constexpr int kSegPow = 41;
 
 // Per field, per integration step constants.
@@ -145,7 +146,7 @@ void launch_deposit_plain(const Launch &L, const StepConst &sc, const DeviceBeam
                           void *const *src, int ns, int np, int ngrid);
 // phase 0: implicit along x into tmp; phase 1: implicit along y back into the field.
 // src: the deposited source (has_src), overwritten as scratch between the two phases;
-// pow: the coefficient set's [2][kSegPow] powers
+// pow: the coefficient set's [4][kSegPow] tables
 void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, void *field, void *src, void *tmp,
                       const void *coef, const void *pow, int ns, int ngrid, int has_src);
 // One diagnostic record (beam [nslice][beam_diag_width(nharm)], then per field
@@ -184,7 +185,7 @@ void launch_field_band_mixed(const Launch &L, const StepConstF &sc, int k, const
 // threads: CTA size, a multiple of 32 in [2 ngrid, 1024]. dbeam / dfield (may be
 // null): the step's diagnostic record, beam [nslice][beam_diag_width(nharm)] (formed by
 // the launch of field 0) and this field's [nslice][kFieldSums + 2] in storage order.
-// pow: the coefficient set's [2][kSegPow] powers.
+// pow: the coefficient set's [4][kSegPow] tables.
 void launch_field_fused_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b,
                               void *field, const void *coef, const void *pow, int ns, int np, int ngrid, int deposit,
                               int threads, double *dbeam, double *dfield, int nharm, double gref);
