@@ -142,9 +142,16 @@ __device__ __forceinline__ void l2_prefetch(const void *p, size_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(z - a)) : "memory");
 }
 
-// Sums of v[0..8) over a warp: lane 4 k holds the sum of v[k] (nine shuffles: each step
-// halves the values a lane carries).
-__device__ __forceinline__ float warp_sums8(float (&v)[8]) {
+// Sums of v[0..8) over a warp: lane 4 k holds the sum of v[k], as a pair hi + lo (each step
+// halves the values a lane carries; the additions' errors go to lo).
+__device__ __forceinline__ float2 add_pairs(float2 a, float2 b) {
+  const float t = a.x + b.x, bp = t - a.x;
+  return make_float2(t, a.y + b.y + ((a.x - (t - bp)) + (b.x - bp)));
+}
+__device__ __forceinline__ float2 shfl_xor2(float2 v, int o) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+__device__ __forceinline__ float2 warp_sums8(float2 (&v)[8]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int o = 16, n = 4; o >= 4; o >>= 1, n >>= 1) {
@@ -152,13 +159,13 @@ __device__ __forceinline__ float warp_sums8(float (&v)[8]) {
 #pragma unroll
     for (int j = 0; j < 4; j++)
       if (j < n) {
-        const float send = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
-        v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        const float2 send = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
+        v[j] = add_pairs(keep, shfl_xor2(send, o));
       }
   }
-  float s = v[0];
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  return s + __shfl_xor_sync(0xffffffffu, s, 1);
+  float2 s = v[0];
+  s = add_pairs(s, shfl_xor2(s, 2));
+  return add_pairs(s, shfl_xor2(s, 1));
 }
 
 // S1 = (I + c Dy) u of rows [b, e) of a column: into S (rows of st) and, eight rows at a
@@ -219,22 +226,25 @@ __device__ __forceinline__ void tm_solve_cols(float2 *L, uint32_t tm, int st, in
 }
 
 // Writes rows [b, e) of a column with the carries lc and rc over its ends to u, and sums the
-// field record's terms (global row of row 0: r0).
+// field record's terms (global row of row 0: r0), compensated like k_diag_field_f's, so that a
+// record formed in the step is the one formed after it: plain FP32 sums here and over the warp
+// erred by 3e-8 to 7e-8 of the sums of a 151^2 field, these by 2e-9 (a step with its record:
+// 300 slices of 255^2 270 -> 283 us, 4096 of 151^2 1332 -> 1357, one 23.3 -> 24.2).
 template <bool REC>
 __device__ __forceinline__ void tm_write_cols(float2 *u, const float2 *L, const float2 *PW, int ng, int st, int line,
-                                              int b, int e, int W, float2 lc, float2 rc, int r0, float (&f)[8]) {
+                                              int b, int e, int W, float2 lc, float2 rc, int r0, float2 (&f)[8]) {
   const int lo = b + W, hi = e - W;  // [lo, hi): no carry
   const float shift = -0.5f * (float)(ng - 1);
   float dy = (float)(r0 + b) + shift;
+  KahanF2 su, sw;  // the field itself; w and dy w
+  KahanF s2;       // dy^2 w
   auto put = [&](int r, float2 x) {
     u[r * ng + line] = x;
     if constexpr (REC) {
       const float w = fmaf(x.x, x.x, x.y * x.y), t = dy * w;
-      f[0] += w;
-      f[3] += t;
-      f[4] = fmaf(dy, t, f[4]);
-      f[5] += x.x;
-      f[6] += x.y;
+      sw.add(make_float2(w, t));
+      s2.add(dy * t);
+      su.add(x);
       dy += 1.f;
     }
   };
@@ -251,26 +261,36 @@ __device__ __forceinline__ void tm_write_cols(float2 *u, const float2 *L, const 
   for (int r = max(mid, hi); r < e; r++) put(r, add_cmulf(L[r * st], PW[e - 1 - r], rc));
   if constexpr (REC) {
     const float dx = (float)line + shift;
-    f[1] = dx * f[0];
-    f[2] = dx * f[1];
+    auto times_dx = [&](float2 v) {
+      const float h = dx * v.x;
+      return make_float2(h, fmaf(dx, v.y, fmaf(dx, v.x, -h)));
+    };
+    f[0] = make_float2(sw.s.x, -sw.c.x);
+    f[1] = times_dx(f[0]);
+    f[2] = times_dx(f[1]);
+    f[3] = make_float2(sw.s.y, -sw.c.y);
+    f[4] = make_float2(s2.s, -s2.c);
+    f[5] = make_float2(su.s.x, -su.c.x);
+    f[6] = make_float2(su.s.y, -su.c.y);
+    f[7] = make_float2(0.f, 0.f);
   }
 }
 
-// The CTA's totals of the threads' record terms: emit(q, total) from the last warp, which
-// folds the warps' sums in FP64, four lanes a value, while the others go on. One barrier.
+// The CTA's totals of the threads' record terms: emit(q, pair) from the last warp, which
+// folds the warps' pairs, four lanes a value, while the others go on. One barrier.
 template <class EM>
-__device__ __forceinline__ void tm_fold_record(float (&f)[8], double *red, EM emit) {
+__device__ __forceinline__ void tm_fold_record(float2 (&f)[8], float2 *red, EM emit) {
   const int tid = threadIdx.x, warp = tid >> 5;
-  const float v = warp_sums8(f);
-  if ((tid & 3) == 0 && (tid & 31) < 4 * kFieldSums) red[warp * kFieldSums + ((tid & 31) >> 2)] = (double)v;
+  const float2 v = warp_sums8(f);
+  if ((tid & 3) == 0 && (tid & 31) < 4 * kFieldSums) red[warp * kFieldSums + ((tid & 31) >> 2)] = v;
   __syncthreads();
   if (warp == (int)(blockDim.x >> 5) - 1) {
     const int k2 = (tid & 31) >> 2;
-    double t = 0;
+    float2 t = make_float2(0.f, 0.f);
     if (k2 < kFieldSums)
-      for (int w = tid & 3; w < (int)(blockDim.x >> 5); w += 4) t += red[w * kFieldSums + k2];
-    t += __shfl_xor_sync(0xffffffffu, t, 1);
-    t += __shfl_xor_sync(0xffffffffu, t, 2);
+      for (int w = tid & 3; w < (int)(blockDim.x >> 5); w += 4) t = add_pairs(t, red[w * kFieldSums + k2]);
+    t = add_pairs(t, shfl_xor2(t, 1));
+    t = add_pairs(t, shfl_xor2(t, 2));
     if ((tid & 3) == 0 && k2 < kFieldSums) emit(k2, t);
   }
 }
@@ -287,7 +307,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   const FieldStepF &fs = sc.f[k];
   float2 *PW = reinterpret_cast<float2 *>(smem_raw);  // kappa^{j+1}
   float2 *S = PW + (W + 1) / 2 * 2;
-  double *red = reinterpret_cast<double *>(S + (ng * st + 1) / 2 * 2);
+  float2 *red = S + (ng * st + 1) / 2 * 2;  // [warp][kFieldSums]
   if (warp == 0) {
     const uint32_t sadr = (uint32_t)__cvta_generic_to_shared(&tm_base);
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sadr), "r"(cols)
@@ -382,7 +402,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
     float2 *L = S + line;
     tm_solve_cols<LA>(L, tm, st, b, e, nq, nchunk, cs, cbc, kap);
     __syncthreads();
-    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float2 f[8];
     {
       float2 lc = zero, rc = zero;
       if (act) {
@@ -398,7 +418,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
         o[7] = v.x;
         o[8] = v.y;
       }
-      tm_fold_record(f, red, [&](int q, double t) { o[q] = t; });
+      tm_fold_record(f, red, [&](int q, float2 t) { o[q] = (double)t.x + (double)t.y; });
     } else {
       __syncthreads();
     }
@@ -474,8 +494,8 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   const int r0 = rank * ng / CL, nrow = (rank + 1) * ng / CL - r0, nmax = (ng + CL - 1) / CL;
   float2 *PW = reinterpret_cast<float2 *>(smem_raw);  // kappa^{j+1}
   float2 *S = PW + (W + 1) / 2 * 2;
-  double *red = reinterpret_cast<double *>(S + (nmax * st + 1) / 2 * 2);
-  double *parts = red + (size_t)(blockDim.x / 32 + 1) * kFieldSums;  // [CTA][kFieldSums], used in CTA 0
+  float2 *red = S + (nmax * st + 1) / 2 * 2;  // [warp][kFieldSums]
+  float2 *parts = red + (size_t)(blockDim.x / 32 + 1) * kFieldSums;  // [CTA][kFieldSums], used in CTA 0
   if (warp == 0) {
     const uint32_t sadr = (uint32_t)__cvta_generic_to_shared(&tm_base);
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sadr), "r"(cols)
@@ -568,7 +588,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   float2 *L = S + line;
   if (cols_on) tm_solve_cols<LA>(L, tm, st, b, e, nq, ((nmax + nseg - 1) / nseg + kTmChunk - 1) / kTmChunk, cs, cbc, kap);
   cl.sync();  // the neighbours' edge rows are solved, and nobody reads u any more
-  float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  float2 f[8];
   {
     float2 lc = zero, rc = zero;
     if (act) {
@@ -594,17 +614,17 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
       o[7] = v.x;
       o[8] = v.y;
     }
-    double *to = cl.map_shared_rank(parts, 0) + rank * kFieldSums;
-    tm_fold_record(f, red, [&](int q, double t) { to[q] = t; });
+    float2 *to = cl.map_shared_rank(parts, 0) + rank * kFieldSums;
+    tm_fold_record(f, red, [&](int q, float2 t) { to[q] = t; });
   }
   if constexpr (!REC) {
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   } else {
     cl.sync();
     if (rank == 0 && tid < kFieldSums) {
-      double t = 0;
-      for (int q = 0; q < CL; q++) t += parts[q * kFieldSums + tid];
-      dfield[(size_t)i * (kFieldSums + 2) + tid] = t;
+      float2 t = parts[tid];
+      for (int q = 1; q < CL; q++) t = add_pairs(t, parts[q * kFieldSums + tid]);
+      dfield[(size_t)i * (kFieldSums + 2) + tid] = (double)t.x + (double)t.y;
     }
   }
   if (warp == 0)

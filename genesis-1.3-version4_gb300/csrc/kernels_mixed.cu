@@ -1438,6 +1438,32 @@ __global__ void __launch_bounds__(kFusedMaxThreads, 1)
   if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
+// Compensated (Kahan) FP32 sum: a thread's partial sum of a slice quantity keeps
+// ~FP32 relative accuracy however many terms it takes, so it can be folded into the
+// FP64 slice total once (GB300's FP64 rate is 1/64 of FP32; per-term FP64 adds would
+// bound the diagnostics).
+struct KahanF {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float v) {
+    const float y = v - c;
+    const float t = s + y;
+    c = (t - s) - y;
+    s = t;
+  }
+};
+// Two of them side by side, in packed instructions
+struct KahanF2 {
+  float2 s = {0.f, 0.f}, c = {0.f, 0.f};
+  static __device__ __forceinline__ float2 minus(float2 a, float2 b) {
+    return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+  }
+  __device__ __forceinline__ void add(float2 v) {
+    const float2 y = minus(v, c), t = __fadd2_rn(s, y);
+    c = minus(minus(t, s), y);
+    s = t;
+  }
+};
+
 #include "field_tm.cuh"
 
 // ---- the whole step of one slice in one CTA: push, deposition and ADI -----------
@@ -1584,20 +1610,6 @@ __global__ void __launch_bounds__(MAXT, 1)
 }
 
 // DiagBeam sums with FP64 accumulation (Diagnostic.cpp:415-456); one block per slice
-// Compensated (Kahan) FP32 sum: a thread's partial sum of a slice quantity keeps
-// ~FP32 relative accuracy however many terms it takes, so it can be folded into the
-// FP64 slice total once (GB300's FP64 rate is 1/64 of FP32; per-term FP64 adds would
-// bound the diagnostics).
-struct KahanF {
-  float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add(float v) {
-    const float y = v - c;
-    const float t = s + y;
-    c = (t - s) - y;
-    s = t;
-  }
-};
-
 // All NS sums and NX min/max pairs of a block in one pass: every warp reduces its
 // lanes' values with shuffles, lane 0 stores them, and after one barrier thread k
 // combines value k over the warps (sums in FP64) into out[k]. The lanes' compensated
