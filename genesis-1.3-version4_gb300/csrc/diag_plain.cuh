@@ -20,6 +20,7 @@ struct Args {
   Ptrs p;
   const double2 *ph1;  // e^{i theta} of every particle while *p.phasor_ok, null: none
   int ns, np, nharm, ng;
+  double gref;  // gammaref: the record's gamma sums are about it
   int nbc, chunk;  // CTAs and particles of a CTA per beam slice
   int nfc, rows;   // CTAs and rows of a CTA per field slice
   double *rec;     // the record: beam [ns][beam_diag_width], fields [nfield][ns][kFieldSums + 2]
@@ -61,12 +62,15 @@ __device__ __forceinline__ void fold(const long long (&v)[NV], int nsum, int nmi
     int i = (k + 8 * q) % n4;
     long long a = r[i];
     if (k < nsum) {
-      double s = __longlong_as_double(a);
-      for (int j = 1; j < n4; j++) {
-        i = i + 1 < n4 ? i + 1 : 0;
-        s += __longlong_as_double(r[i]);
-      }
-      a = __double_as_longlong(s);
+      // four partial sums: shorter chains of roundings and of latencies (n4 is a multiple of 8)
+      double s[4] = {0, 0, 0, 0};
+      for (int j = 0; j < n4; j += 4)
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+          s[w] += __longlong_as_double(r[i]);
+          i = i + 1 < n4 ? i + 1 : 0;
+        }
+      a = __double_as_longlong((s[0] + s[1]) + (s[2] + s[3]));
     } else {
       const bool lo = k < nsum + nmin;
       for (int j = 1; j < n4; j++) {
@@ -150,8 +154,10 @@ __device__ __forceinline__ void beam_chunk(const Args &a, int is, int c, long lo
       sincos(p.theta[o], &sn, &cs);
       z = C2{cs, sn};
     }
-    s[0] += g;
-    s[1] = fma(g, g, s[1]);
+    // gamma about gammaref: the difference is exact, and the spread does not cancel
+    const double dg = g - a.gref;
+    s[0] += dg;
+    s[1] = fma(dg, dg, s[1]);
     s[2] += x;
     s[3] = fma(x, x, s[3]);
     s[4] += y;
@@ -204,9 +210,8 @@ __device__ __forceinline__ void field_rows(const Args &a, int k, int i, int c, l
   __syncthreads();
   double s[NV] = {0};
   for (int col = tid; col < ng; col += blockDim.x) {
-    double sw = 0;
-#pragma unroll 4
-    for (int r = 0; r < nr; r++) {
+    double s2[2] = {0, 0};
+    auto row = [&](int r, double &sw) {
       const double2 u = f[(size_t)(r0 + r) * ng + col], d = dy[r];
       const double w = fma(u.x, u.x, u.y * u.y);
       sw += w;
@@ -214,7 +219,15 @@ __device__ __forceinline__ void field_rows(const Args &a, int k, int i, int c, l
       s[4] = fma(d.y, w, s[4]);
       s[5] += u.x;
       s[6] += u.y;
+    };
+    int r = 0;
+#pragma unroll 2
+    for (; r + 1 < nr; r += 2) {
+      row(r, s2[0]);
+      row(r + 1, s2[1]);
     }
+    if (r < nr) row(r, s2[0]);
+    const double sw = s2[0] + s2[1];
     const double dx = (double)col + shift, t = dx * sw;
     s[0] += sw;
     s[1] += t;

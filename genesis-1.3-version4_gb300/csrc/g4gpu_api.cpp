@@ -1680,7 +1680,7 @@ void enqueue_diag(g4gpu_handle h, cudaStream_t stream, int nharm, double *rec, b
     for (int k = 0; k < c.nfield && h1 < 0; k++)
       if (c.harm[k] == 1) h1 = k;
     Timed t(h, G4GPU_K_DIAG);
-    g4::launch_diag_plain(L, h->beam, h->field, c.nfield, h1, ns, np, ng, nharm, beam, field, rec, h->diag_part,
+    g4::launch_diag_plain(L, h->beam, h->field, c.nfield, h1, ns, np, ng, nharm, c.gammaref, beam, field, rec, h->diag_part,
                           h->diag_count);
     return;
   }
@@ -1713,12 +1713,13 @@ void finish_diag(g4gpu_handle h, const double *raw, int nharm, const int *first,
       const int n = h->beam.count ? h->hcount[is] : np;
       double norm = n > 0 ? 1. / static_cast<double>(n) : 1.;
       const double *s = raw + (size_t)is * bw;
-      double g1 = s[0] * norm, g2 = s[1] * norm, x1 = s[2] * norm, x2 = s[3] * norm;
+      // gamma's sums are about gammaref, so that the spread keeps its digits
+      double d1 = s[0] * norm, d2 = s[1] * norm, g1 = n > 0 ? c.gammaref + d1 : 0., x1 = s[2] * norm, x2 = s[3] * norm;
       double y1 = s[4] * norm, y2 = s[5] * norm, px1 = s[6] * norm, px2 = s[7] * norm;
       double py1 = s[8] * norm, py2 = s[9] * norm, xpx = s[10] * norm, ypy = s[11] * norm;
       double *o = beam_out + (size_t)is * ow;
       o[G4GPU_DB_ENERGY] = g1;
-      o[G4GPU_DB_ENERGYSPREAD] = std::sqrt(std::fabs(g2 - g1 * g1));
+      o[G4GPU_DB_ENERGYSPREAD] = std::sqrt(std::fabs(d2 - d1 * d1));
       o[G4GPU_DB_XPOS] = x1;
       o[G4GPU_DB_XSIZE] = std::sqrt(std::fabs(x2 - x1 * x1));
       o[G4GPU_DB_YPOS] = y1;

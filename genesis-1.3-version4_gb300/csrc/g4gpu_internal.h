@@ -155,7 +155,8 @@ void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, vo
 // count: diag_plain_scratch's doubles and counters (zeroed once, left zero).
 size_t diag_plain_scratch(int ns, int np, int nharm, int ng, int nfield, size_t *counters);
 void launch_diag_plain(const Launch &L, const DeviceBeam &b, void *const *field, int nfield, int h1, int ns, int np,
-                       int ngrid, int nharm, bool beam, bool fields, double *rec, double *scratch, unsigned *count);
+                       int ngrid, int nharm, double gref, bool beam, bool fields, double *rec, double *scratch,
+                       unsigned *count);
 
 // kernels_mixed.cu (FP32 field, FP64 phase)
 void launch_push_mixed(const Launch &L, const StepConstF &sc, const DeviceBeam &b,
@@ -362,7 +363,7 @@ void closure_denormalize(void *stream, const float *y, const float *scale, const
                          int rows, int n, int ld);
 
 // number of raw sums per slice written by the diagnostic kernels
-constexpr int kBeamSums = 12;   // g1 g2 x1 x2 y1 y2 px1 px2 py1 py2 xpx ypy
+constexpr int kBeamSums = 12;   // g1 g2 (of gamma - gammaref) x1 x2 y1 y2 px1 px2 py1 py2 xpx ypy
 constexpr int kBeamMinMax = 10; // xmin xmax pxmin pxmax ymin ymax pymin pymax gmin gmax
 #ifdef __CUDACC__
 __host__ __device__

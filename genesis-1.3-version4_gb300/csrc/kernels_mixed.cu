@@ -1294,10 +1294,7 @@ __device__ __forceinline__ void slice_beam_sums(const PtrsF &p, double gref, int
   }
   cta_reduce<NSUM, 5>(c, mn, mx, sh, res);
   const int k = threadIdx.x;
-  const double n = (double)cnt;
-  if (k == 0) o[0] = n * gref + res[0];
-  if (k == 1) o[1] = n * gref * gref + 2.0 * gref * res[0] + res[1];
-  if (k >= 2 && k < kBeamSums) o[k] = res[k];
+  if (k < kBeamSums) o[k] = res[k];
   if (k >= kBeamSums && k < kBeamSums + 2 * nharm) o[kBeamMinMax + k] = res[k];
   if (k < 10) o[kBeamSums + k] = (k >= 8 ? gref : 0.0) + res[NSUM + k];
 }
@@ -1674,10 +1671,9 @@ __device__ __forceinline__ void block_reduce_all(const KahanF *s, const float *m
 // compensated FP32 sums, folded into FP64 once, and the slice totals are FP64 sums
 // over the threads (the per-slice reductions, bunching and energy included, stay
 // FP64; GB300 runs FP64 at 1/64 of the FP32 rate, so per-particle FP64 arithmetic
-// would bound the kernel). The energy moments are
-// taken about gammaref: sum g = N gref + sum dg and sum g^2 = N gref^2 + 2 gref sum dg
-// + sum dg^2, without the cancellation of squaring g itself. NH: compile-time bound on
-// the number of harmonics (the arrays stay in registers).
+// would bound the kernel). The energy moments are those of dg, about gammaref: no
+// cancellation, as squaring g itself would bring. NH: compile-time bound on the number of
+// harmonics (the arrays stay in registers).
 //
 // Memory bounds it (28 bytes a particle against ~100 instructions), so what matters is
 // how many bytes are on their way. Four particles at a time are copied to shared memory in
@@ -1771,11 +1767,8 @@ __global__ void __launch_bounds__(BS) k_diag_beam_f(PtrsF p, double gref, int np
   __syncthreads();
   const int w = beam_diag_width(nharm);
   double *o = out + (size_t)is * w;
-  const double n = (double)cnt;
   for (int k = tid; k < NSUM || k < 10; k += BS) {
-    if (k == 0) o[0] = n * gref + res[0];
-    if (k == 1) o[1] = n * gref * gref + 2.0 * gref * res[0] + res[1];
-    if (k >= 2 && k < kBeamSums) o[k] = res[k];
+    if (k < kBeamSums) o[k] = res[k];
     if (k >= kBeamSums && k < kBeamSums + 2 * nh) o[kBeamMinMax + k] = res[k];  // bunching after min/max
     if (k < 10) o[kBeamSums + k] = (k >= 8 ? gref : 0.0) + res[NSUM + k];
   }

@@ -1032,7 +1032,8 @@ size_t diag_plain_scratch(int ns, int np, int nharm, int ng, int nfield, size_t 
 }
 
 void launch_diag_plain(const Launch &L, const DeviceBeam &b, void *const *field, int nfield, int h1, int ns, int np,
-                       int ngrid, int nharm, bool beam, bool fields, double *rec, double *scratch, unsigned *count) {
+                       int ngrid, int nharm, double gref, bool beam, bool fields, double *rec, double *scratch,
+                       unsigned *count) {
   diag64::Args a{};
   a.p = make_ptrs(b, field, nullptr, nfield);
   const int nt = diag_threads(ngrid);
@@ -1040,6 +1041,7 @@ void launch_diag_plain(const Launch &L, const DeviceBeam &b, void *const *field,
   a.np = np;
   a.nharm = nharm;
   a.ng = ngrid;
+  a.gref = gref;
   a.chunk = diag_chunk(ns, np, nt);
   a.nbc = beam ? (np + a.chunk - 1) / a.chunk : 0;
   a.rows = diag_rows(ns * nfield, ngrid);
