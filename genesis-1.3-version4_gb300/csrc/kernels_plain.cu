@@ -516,7 +516,10 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
     C2 cs;
     if (cached) {
       cs = ld(p.phasor + k * p.pstride + o);
-      if (sc.autophase != 0.) cs = cmul_fma(cs, C2{fs.rot_auto[0], fs.rot_auto[1]});
+      if (sc.autophase != 0.) {  // and by the rounding of theta0
+        cs = cmul_fma(cs, C2{fs.rot_auto[0], fs.rot_auto[1]});
+        cs = add_imul(cs, fs.rharm * ((theta0 - th) - sc.autophase), cs);
+      }
     } else {
       double sn, co;
       sincos(fs.rharm * theta0, &sn, &co);
@@ -567,13 +570,15 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
   gamma = fma(stpz, fma(k2gg, kSixth, k3gg), gamma);
   dth = fma(stpz, fma(k2pp, kSixth, k3pp), dth);
   double theta = theta0 + dth;
-  // the deposition's phasors, kept for the next push
+  // the deposition's phasors, kept for the next push and the records: turned by the advance of
+  // the phase as it is stored (the rounding of a phase of thousands of radians, step after step,
+  // would part them from it: 1e-11 after 600 steps of 8 rad)
   C2 cs[NF];
   if (deposit || p.phasor) {
+    const double d = (theta - theta0) - sc.dnom_full;
 #pragma unroll
     for (int k = 0; k < NF; k++) {
       if (k >= sc.nfld) break;
-      const double d = dth - sc.dnom_full;
       cs[k] = cmul_fma(bfull[k], expi(sc.f[k].rharm == 1. ? d : sc.f[k].rharm * d));
     }
   }
@@ -587,8 +592,9 @@ __global__ void __launch_bounds__(512) k_push(StepConst sc, Ptrs p, int ns, int 
   if (p.wake) gamma += p.wake[is] * sc.delz / kEev;
   // TrackBeam::applyR56 (TrackBeam.cpp:260-277)
   if (sc.chic) {
-    const double r = sc.r56 * (gamma - sc.gammaref);
-    theta += r;
+    const double th0 = theta;
+    theta += sc.r56 * (gamma - sc.gammaref);
+    const double r = theta - th0;
     if (deposit || p.phasor) {
 #pragma unroll
       for (int k = 0; k < NF; k++) {
