@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   float2 *S = PW + (W + 1) / 2 * 2;
   float2 *red = S + (ng * st + 1) / 2 * 2;  // [warp][kFieldSums]
   if (warp == 0) {
+    __syncwarp();
     const uint32_t sadr = (uint32_t)__cvta_generic_to_shared(&tm_base);
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sadr), "r"(cols)
                  : "memory");
@@ -352,17 +353,10 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     __syncthreads();
     if (deposit) {  // S = S1 + src
-      if (vec) {
-        const float scl = fs.dep_scl * (float)p.current[is];
-#pragma unroll 1
-        for (int q = tid; q < (np >> 2); q += blockDim.x) {
-          const Quad v = quad;
-          if (q + (int)blockDim.x < (np >> 2)) quad = load_quad(p, base, q + blockDim.x);
-          deposit_quad(sc, fs, scl, S, Grid(ng, st), v);
-        }
-      } else {
+      if (vec)
+        deposit_quads(sc, fs, p, S, is, np, Grid(ng, st), quad);
+      else
         deposit_smem(sc, fs, p, S, is, np, Grid(ng, st));
-      }
       __syncthreads();
     }
     // the next slice's field and particles on their way to L2 while this one is solved
@@ -423,6 +417,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
       __syncthreads();
     }
   }
+  __syncwarp();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(cols) : "memory");
 }
@@ -497,6 +492,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   float2 *red = S + (nmax * st + 1) / 2 * 2;  // [warp][kFieldSums]
   float2 *parts = red + (size_t)(blockDim.x / 32 + 1) * kFieldSums;  // [CTA][kFieldSums], used in CTA 0
   if (warp == 0) {
+    __syncwarp();
     const uint32_t sadr = (uint32_t)__cvta_generic_to_shared(&tm_base);
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sadr), "r"(cols)
                  : "memory");
@@ -537,17 +533,10 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   __syncthreads();
   if (deposit) {
     const Band g(ng, st, r0, nrow);
-    if (vec) {
-      const float scl = fs.dep_scl * (float)p.current[is];
-#pragma unroll 1
-      for (int q = tid; q < (np >> 2); q += blockDim.x) {
-        const Quad v = quad;
-        if (q + (int)blockDim.x < (np >> 2)) quad = load_quad(p, base, q + blockDim.x);
-        deposit_quad(sc, fs, scl, S, g, v);
-      }
-    } else {
+    if (vec)
+      deposit_quads(sc, fs, p, S, is, np, g, quad);
+    else
       deposit_smem(sc, fs, p, S, is, np, g);
-    }
     __syncthreads();
   }
   // a later slice's field and particles on their way to L2
@@ -587,6 +576,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   __syncthreads();
   float2 *L = S + line;
   if (cols_on) tm_solve_cols<LA>(L, tm, st, b, e, nq, ((nmax + nseg - 1) / nseg + kTmChunk - 1) / kTmChunk, cs, cbc, kap);
+  __syncwarp();
   cl.sync();  // the neighbours' edge rows are solved, and nobody reads u any more
   float2 f[8];
   {
@@ -603,7 +593,10 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
     }
     // the peers' rows are read: the last barrier, which keeps a CTA's shared memory until then, does
     // not wait for the field's writes (with the record it also brings the parts to CTA 0, below)
-    if constexpr (!REC) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if constexpr (!REC) {
+      __syncwarp();  // the carries above and the rows below part a warp's lanes
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
     tm_write_cols<REC>(u, L, PW, ng, st, line, b, e, W, lc, rc, r0, f);
   }
   if constexpr (REC) {
@@ -617,6 +610,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
     float2 *to = cl.map_shared_rank(parts, 0) + rank * kFieldSums;
     tm_fold_record(f, red, [&](int q, float2 t) { to[q] = t; });
   }
+  __syncwarp();
   if constexpr (!REC) {
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   } else {
@@ -627,6 +621,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
       dfield[(size_t)i * (kFieldSums + 2) + tid] = (double)t.x + (double)t.y;
     }
   }
+  __syncwarp();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(cols) : "memory");
 }
