@@ -47,6 +47,10 @@ __device__ __forceinline__ Lines lines_setup(unsigned char *smem, int nline, int
   return s;
 }
 
+__device__ __forceinline__ bool finite(C2 v) {
+  return (__double2hiint(v.x) & 0x7ff00000) != 0x7ff00000 && (__double2hiint(v.y) & 0x7ff00000) != 0x7ff00000;
+}
+
 // Solves (I - i c D) x = r in place on the nline lines of the tile (element k of line l
 // at T[l * lstride + k * estride]), nseg threads per line. The Thomas recurrences
 // (tridagx / tridagy, FieldSolverADI.cpp:94-122)
@@ -58,6 +62,8 @@ __device__ __forceinline__ Lines lines_setup(unsigned char *smem, int nline, int
 // with D the last d of the segment before (its own zero start is forgotten there) and x_e
 // the first x of the segment after. Only the W elements next to a segment's ends need the
 // terms; the CTA's threads share them out. With nseg = 1 the sweeps are the reference's.
+// A value that is not finite runs through a whole line in the reference's sweeps, and so it
+// does here (`bad`, by the barrier that is there anyway).
 // Why segments: the FP64 pipe takes 64 cycles for a warp's instruction, so one thread per
 // line is a chain of 10 ng of them, and a window of few slices leaves most SMs idle.
 // Every thread calls it, after a barrier; a barrier has passed when it returns.
@@ -65,8 +71,9 @@ __device__ __forceinline__ void solve_lines(const Lines &s, int nline, int lstri
                                             int nco, int W, double c) {
   const int tid = threadIdx.x;
   const int line = tid % nline, seg = tid / nline;
+  const int b = seg * ng / nseg, e = (seg + 1) * ng / nseg;
+  bool bad = false;
   if (seg < nseg) {
-    const int b = seg * ng / nseg, e = (seg + 1) * ng / nseg;
     C2 *L = s.T + (size_t)line * lstride;
     // one loop for all segments (the tables' last entry is their constant): lanes of
     // different segments stay together, and a warp's FP64 instruction costs the same for
@@ -84,8 +91,18 @@ __device__ __forceinline__ void solve_lines(const Lines &s, int nline, int lstri
       L[k * estride] = x;
     }
     s.edge_x[seg * nline + line] = x;
+    bad = !finite(x);
   }
-  __syncthreads();
+  if (__syncthreads_or(bad)) {
+    if (seg < nseg) {
+      bad = false;
+      for (int q = 0; q < nseg; q++) bad = bad || !finite(s.edge_x[q * nline + line]);
+      const double nan = __longlong_as_double(0x7ff8000000000000LL);
+      if (bad)
+        for (int k = b; k < e; k++) s.T[(size_t)line * lstride + k * estride] = C2{nan, nan};
+    }
+    __syncthreads();
+  }
   if (nseg == 1) return;
   const int ntask = (nseg - 1) * W * nline;
   for (int t = tid; t < ntask; t += blockDim.x) {
