@@ -2093,16 +2093,19 @@ size_t g4gpu_device_bytes(g4gpu_handle h) { return h ? h->bytes : 0; }
 // ---- launch-shape tuning -----------------------------------------------------
 
 namespace {
+// nslice: what is best depends on the window (4 and 300 slices of 151^2: a cluster a slice,
+// one CTA a slice; the first's CTA size made the second's step 79 us instead of 68)
 struct TuneKey {
-  int device, precision, npart, ngrid, nfield, solver;
+  int device, precision, nslice, npart, ngrid, nfield, solver;
   bool operator<(const TuneKey &o) const {
-    return std::tie(device, precision, npart, ngrid, nfield, solver) <
-           std::tie(o.device, o.precision, o.npart, o.ngrid, o.nfield, o.solver);
+    return std::tie(device, precision, nslice, npart, ngrid, nfield, solver) <
+           std::tie(o.device, o.precision, o.nslice, o.npart, o.ngrid, o.nfield, o.solver);
   }
 };
 std::mutex g_tune_mu;
+// the fastest set shapes, and those of the handle (0: automatic, where that is no slower)
 struct TuneVal {
-  int push_block, field_threads, field_kernel;
+  int push_block, field_threads, field_kernel, own_push, own_threads;
 };
 std::map<TuneKey, TuneVal> g_tune;
 
@@ -2159,17 +2162,20 @@ extern "C" int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_thread
     if (!h->field_loaded[k]) return fail(h, G4GPU_ERR_STATE, "a field is not loaded");
   cudaSetDevice(h->cfg.device);
   const g4gpu_config &c = h->cfg;
-  TuneKey key{c.device, c.precision, c.npart, c.ngrid, c.nfield, c.solver};
+  TuneKey key{c.device, c.precision, c.nslice, c.npart, c.ngrid, c.nfield, c.solver};
+  auto take = [&](const TuneVal &v) {
+    h->push_block = v.own_push;
+    h->field_threads = v.own_threads;
+    h->field_kernel = v.field_kernel;
+    if (push_block) *push_block = v.push_block;
+    if (field_threads) *field_threads = v.field_threads;
+    if (field_kernel) *field_kernel = v.field_kernel;
+  };
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
-      h->push_block = it->second.push_block;
-      h->field_threads = it->second.field_threads;
-      h->field_kernel = it->second.field_kernel;
-      if (push_block) *push_block = h->push_block;
-      if (field_threads) *field_threads = h->field_threads;
-      if (field_kernel) *field_kernel = h->field_kernel;
+      take(it->second);
       return G4GPU_OK;
     }
   }
@@ -2189,7 +2195,7 @@ extern "C" int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_thread
   if (fused) {
     fields.clear();
     int lo = (2 * c.ngrid + 31) / 32 * 32;
-    for (int t : {lo, 512, 768, 1024})
+    for (int t : {lo, 384, 512, 768, 1024})
       if (t >= lo && std::find(fields.begin(), fields.end(), t) == fields.end()) fields.push_back(t);
   }
   bool saved_graph = h->graph_mode, saved_prof = h->prof;
@@ -2217,26 +2223,35 @@ extern "C" int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_thread
     *ms = best;
     return G4GPU_OK;
   };
-  int best_pb = 256, best_ft = fields[0];
-  float best_ms = 1e30f;
+  // the fastest of the set sizes, and what the handle takes: that size where it beats the
+  // automatic one by more than two timings of a step differ
+  const float kGain = 0.97f;
+  int best_pb = 256, best_ft = fields[0], own_pb = 0, own_ft = 0;
+  float best_ms = 1e30f, auto_ms = 1e30f;
+  if (!rc) rc = time_step(0, 0, &auto_ms);
   for (int pb : pushes) {
     float ms;
-    if ((rc = time_step(pb, best_ft, &ms))) break;
+    if (rc || (rc = time_step(pb, 0, &ms))) break;
     if (ms < best_ms) {
       best_ms = ms;
       best_pb = pb;
     }
   }
+  if (best_ms < kGain * auto_ms) {
+    own_pb = best_pb;
+    auto_ms = best_ms;
+  }
   if (!rc && fields.size() > 1) {
     best_ms = 1e30f;
     for (int ft : fields) {
       float ms;
-      if ((rc = time_step(best_pb, ft, &ms))) break;
+      if ((rc = time_step(own_pb, ft, &ms))) break;
       if (ms < best_ms) {
         best_ms = ms;
         best_ft = ft;
       }
     }
+    if (best_ms < kGain * auto_ms) own_ft = best_ft;
   }
   // the cluster-pair field kernel, where the step's segmented solves apply
   int best_fk = 0;
@@ -2249,7 +2264,7 @@ extern "C" int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_thread
   pairable = pairable && g4::band_cluster(c.ngrid, band_w) == 2;
   if (!rc && pairable) {
     float ms;
-    if (!(rc = time_step(best_pb, best_ft, &ms))) {
+    if (!(rc = time_step(own_pb, own_ft, &ms))) {
       float single = ms;
       h->field_kernel = 1;
       float pms = 1e30f;
@@ -2264,28 +2279,28 @@ extern "C" int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_thread
         if (rep > 0 && t < pms) pms = t;
       }
       h->field_kernel = 0;
-      if (!rc && pms < single) best_fk = 1;
+      if (!rc && pms < kGain * single) best_fk = 1;
     }
   }
   // the whole step in one kernel, over its CTA sizes (each with its own particles per
   // lane), against the best of the above
   if (!rc && fused && c.nfield == 1 && !h->sc_on) {
     float cur = 1e30f;
-    if (!(rc = time_step(best_pb, best_ft, &cur, best_fk))) {
+    if (!(rc = time_step(own_pb, own_ft, &cur, best_fk))) {
       int step_ft = 0;
       float step_ms = 1e30f;
       for (int ft : fields) {
         if (ft != (2 * c.ngrid + 31) / 32 * 32 && ft < 512) continue;
         float ms;
-        if ((rc = time_step(best_pb, ft, &ms, 2))) break;
+        if ((rc = time_step(own_pb, ft, &ms, 2))) break;
         if (ms < step_ms) {
           step_ms = ms;
           step_ft = ft;
         }
       }
-      if (!rc && step_ms < cur) {
+      if (!rc && step_ms < kGain * cur) {
         best_fk = 2;
-        best_ft = step_ft;
+        best_ft = own_ft = step_ft;
       }
     }
   }
@@ -2296,16 +2311,12 @@ extern "C" int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_thread
   h->prof = saved_prof;
   std::memset(h->launches, 0, sizeof(h->launches));
   if (rc) return rc;
-  h->push_block = best_pb;
-  h->field_threads = best_ft;
-  h->field_kernel = best_fk;
+  const TuneVal val{best_pb, best_ft, best_fk, own_pb, own_ft};
+  take(val);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[key] = {best_pb, best_ft, best_fk};
+    g_tune[key] = val;
   }
-  if (push_block) *push_block = best_pb;
-  if (field_threads) *field_threads = best_ft;
-  if (field_kernel) *field_kernel = best_fk;
   return check_device_flag(h);
 }
 

@@ -387,19 +387,20 @@ int g4gpu_measure_fp64_rate(int device, double *instr_per_s);
 int g4gpu_set_graph_mode(g4gpu_handle h, int on);
 
 /* Times the candidate launch shapes of the step kernels on the handle's own data
- * (one step per candidate; beam and field are restored afterwards) and keeps the
- * fastest: threads per block of the push, threads per CTA of the fused field
- * kernel, and the fused field kernel itself (0: one CTA per slice, 1: a cluster of
- * two CTAs per slice, each holding half the rows, 2: the whole step of a slice in
- * one CTA, push, deposition and ADI, for one-field windows without space charge;
- * steps it does not apply to run kernel 0). Grids too large for one CTA (ngrid > 168)
- * run on the smallest cluster of 2 to 4 CTAs whose bands of rows fit shared memory
- * (up to ngrid 333), beyond that on the tiled two-pass ADI. Choices are cached per
- * (precision, npart, ngrid, nfield, solver) for the life of the process. Requires
- * the lattice, beam and fields to be loaded. *push_block, *field_threads and
- * *field_kernel (each may be NULL) receive the choice. No reference counterpart. */
+ * (one step per candidate; beam and field are restored afterwards): threads per block
+ * of the push, threads per CTA of the fused field kernel, and the fused field kernel
+ * itself (0: one CTA per slice, or a cluster of 2 to 8 CTAs for grids too large for one,
+ * ngrid > 168, and for windows that leave SMs idle, 1: a cluster of two CTAs per slice,
+ * each holding half the rows, 2: the whole step of a slice in one CTA, push, deposition
+ * and ADI, for one-field windows without space charge; steps it does not apply to run
+ * kernel 0). Grids beyond ngrid 333 run on the tiled two-pass ADI. The handle takes a
+ * size where it beats the automatic one, by the window's slices and particles, which a
+ * handle has from the start. *push_block, *field_threads and *field_kernel (each may be
+ * NULL) receive the fastest that g4gpu_set_launch_shapes can set. Choices are cached per
+ * (precision, nslice, npart, ngrid, nfield, solver) for the life of the process. Requires
+ * the lattice, beam and fields to be loaded. No reference counterpart. */
 int g4gpu_autotune(g4gpu_handle h, int *push_block, int *field_threads, int *field_kernel);
-/* Sets the launch shapes g4gpu_autotune would choose: push_block a multiple of 32 in
+/* Sets the launch shapes in place of the automatic ones: push_block a multiple of 32 in
  * [32, 512], field_threads a multiple of 32 in [2 ngrid, 1024] (mixed ADI form; the kernel
  * that keeps a slice's stencil term in tensor memory takes at most 768 of them, and its
  * cluster form, for windows of few slices and large grids, a size of its own), and
