@@ -588,7 +588,8 @@ void sc_launch(const Launch &L, const ScConst &c, const typename F::Step &step, 
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(configured.load() & (1ull << dev))) {
-    cudaFuncSetAttribute(k_sc_field<F, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_max_smem());
+    if constexpr (!F::kPlain)
+      cudaFuncSetAttribute(k_sc_field<F, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_max_smem());
     cudaFuncSetAttribute(k_sc_field<F, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_max_smem());
     configured.fetch_or(1ull << dev);
   }
@@ -598,11 +599,25 @@ void sc_launch(const Launch &L, const ScConst &c, const typename F::Step &step, 
     return;
   }
   const size_t smem = c.shortrange ? (size_t)c.modes_per_pass * sc_bytes_per_mode(c.ng, !F::kPlain) : 0;
-  // particles' loads issued together: four with one or two modes, two with more, where the
-  // modes' arithmetic hides them and four cost registers (4096 x 8192, FP32: 1, 6, 15 modes 397,
-  // 953, 1834 us by fours, 402, 890, 1660 by twos)
-  const bool few = (2 * c.nphi + 1) * c.nz <= 2;
-  (few ? k_sc_field<F, 4> : k_sc_field<F, 2>)<<<c.ns, kScThreads, smem, s>>>(sb, buf.st, (typename F::R *)buf.ez, c);
+  // Particles' loads issued together: four; in FP32 with more than two modes two where their
+  // fewer registers save a round of CTAs (four CTAs of 256 threads an SM by fours, five by twos).
+  // FP32, 6 modes, us by fours / twos: 512 slices of 8192 particles 141 / 147, 608 143 / 149, 700
+  // 210 / 173, 900 of 4096 129 / 138, 1500 199 / 184, 4096 of 2048 304 / 289; 1 mode, 4096 of 8192
+  // 397 / 402. FP64, bound by its pipe: 300 of 8192, 3 and 6 modes 1680 / 1691, 2649 / 2655.
+  if constexpr (!F::kPlain) {
+    if ((2 * c.nphi + 1) * c.nz > 2) {
+      int four = 0, two = 0, sms = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&four, k_sc_field<F, 4>, kScThreads, smem);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, k_sc_field<F, 2>, kScThreads, smem);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      auto rounds = [&](int per_sm) { return (c.ns + per_sm * sms - 1) / (per_sm * sms); };
+      if (four > 0 && two > 0 && sms > 0 && rounds(two) < rounds(four)) {
+        k_sc_field<F, 2><<<c.ns, kScThreads, smem, s>>>(sb, buf.st, (typename F::R *)buf.ez, c);
+        return;
+      }
+    }
+  }
+  k_sc_field<F, 4><<<c.ns, kScThreads, smem, s>>>(sb, buf.st, (typename F::R *)buf.ez, c);
 }
 
 }  // namespace
