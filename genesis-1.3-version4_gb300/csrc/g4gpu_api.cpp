@@ -1016,7 +1016,7 @@ static int field_threads(g4gpu_handle h, int W) {
 static int push_threads(g4gpu_handle h) {
   if (h->push_block > 0) return h->push_block;
   if (h->mixed) return 128;
-  return (long long)h->cfg.nslice * h->cfg.npart < 512 * 152 ? 64 : 256;
+  return (long long)h->cfg.nslice * h->cfg.npart < 512LL * g4::device_sms() ? 64 : 256;
 }
 
 // Queues the kernels and copies of steps istep0 .. istep0+nsteps-1 on the handle's
@@ -1955,9 +1955,10 @@ bool records_beside(g4gpu_handle h, int istep0, int nsteps) {
   if (h->prof || h->field_kernel == 2) return false;
   for (int s = istep0; s < istep0 + nsteps && s < (int)h->substeps.size(); s++)
     if (h->substeps[s] > 1) return false;
-  if (!h->mixed) return c.nslice * c.ngrid <= 304 || c.nslice >= 64;  // lines: two a SM
+  const int sms = g4::device_sms();
+  if (!h->mixed) return (long long)c.nslice * c.ngrid <= 2 * sms || c.nslice >= 64;  // lines: two an SM
   const int cluster = c.solver == G4GPU_SOLVER_ADI ? g4::field_cluster(c.ngrid, c.nslice, h->steps[istep0].f[0].tw) : 0;
-  return c.nslice <= 38 || c.nslice * std::max(cluster, 1) >= 608;  // a quarter of, or four times the SMs
+  return c.nslice <= sms / 4 || (long long)c.nslice * std::max(cluster, 1) >= 4 * sms;
 }
 }  // namespace
 

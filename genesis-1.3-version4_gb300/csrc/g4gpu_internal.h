@@ -137,6 +137,9 @@ struct Launch {
   int *err;  // device error flag
 };
 
+// SMs of the current device, asked for once (kernels_util.cu)
+int device_sms();
+
 // kernels_plain.cu (FP64, the reference's arithmetic)
 // block: threads per block of the push (128, 256 or 512)
 void launch_push_plain(const Launch &L, const StepConst &sc, const DeviceBeam &b,

@@ -726,19 +726,6 @@ int fft_ctas_per_sm(int regs_bound, size_t smem) {
   return k;
 }
 
-int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return 152;
-  if (!cached[dev]) {
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    cached[dev] = v > 0 ? v : 152;
-  }
-  return cached[dev];
-}
-
 template <typename T2, bool GAP>
 void launch_fft(void *stream, void *field, const void *src, void *work, const void *roots, double k2c,
                 const void *sig, int filtered, double delz, const FFTPlan &pl, int ns, int first) {
@@ -754,7 +741,7 @@ void launch_fft(void *stream, void *field, const void *src, void *work, const vo
     cudaFuncSetAttribute(k_fft_cols<T2, GAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     configured.fetch_or(1ull << dev);
   }
-  const int nsm = sm_count();
+  const int nsm = device_sms();
   const int rows_ctas = es == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64, cols_ctas = rows_ctas;
   auto grid = [&](int L, size_t smem, int regs_bound) {
     const long long tiles = (long long)ns * ((n + L - 1) / L);
@@ -805,7 +792,7 @@ void launch_fft_diag_t(void *stream, const void *field, void *work, const void *
     configured.fetch_or(1ull << dev);
   }
   const int ctas = es == 8 ? FFT_CTAS_FP32 : FFT_CTAS_FP64;
-  const long long nsm = sm_count();
+  const long long nsm = device_sms();
   auto grid = [&](int lines, size_t smem) {
     const long long tiles = (long long)ns * ((n + lines - 1) / lines);
     const long long cap = nsm * fft_ctas_per_sm(ctas, smem);

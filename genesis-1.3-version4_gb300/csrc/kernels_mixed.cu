@@ -2535,17 +2535,6 @@ namespace {
 bool field_tm_fits(int ngrid, int threads, int W) {
   return tm_shape(ngrid, threads, W).threads > 0 && tm_smem_bytes(ngrid, W, threads) <= 227u * 1024u - 16;
 }
-int field_sms() {
-  static std::atomic<int> sms[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int n = dev < 64 ? sms[dev].load() : 0;
-  if (!n) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 152;
-    if (dev < 64) sms[dev].store(n);
-  }
-  return n;
-}
 // CTAs of k_field_tm_f an SM holds: one, or two where the shared memory and the tensor memory
 // of two fit (its 80 registers a thread allow two of 384)
 int field_tm_per_sm(size_t smem, int threads) {
@@ -2565,7 +2554,7 @@ void launch_field_tm(const Launch &L, const StepConstF &sc, int k, const PtrsF &
   const TmShape t = tm_shape(ngrid, threads, W);
   threads = t.threads;
   const size_t smem = tm_smem_bytes(ngrid, W, threads);
-  chain_launch(k_field_tm_f<LA, REC>, std::min(ns, field_sms() * field_tm_per_sm(smem, threads)), threads, smem,
+  chain_launch(k_field_tm_f<LA, REC>, std::min(ns, device_sms() * field_tm_per_sm(smem, threads)), threads, smem,
                (cudaStream_t)L.stream, 0, sc, k, p, (float2 *)field, (const float2 *)coef, (const float2 *)pow, ns, np,
                ngrid, deposit, t.nseg, W, t.words, t.cols, dfield);
 }
@@ -2578,7 +2567,7 @@ void launch_field_tm(const Launch &L, const StepConstF &sc, int k, const PtrsF &
 int field_threads_auto(int ngrid, int ns, int W) {
   if (!field_tm_fits(ngrid, kTmMaxThreads, W)) return 512;
   const int two = (2 * ngrid + 31) / 32 * 32 > 384 ? 0 : 384;
-  if (two && ns > field_sms() && field_tm_fits(ngrid, two, W) && field_tm_per_sm(tm_smem_bytes(ngrid, W, two), two) == 2)
+  if (two && ns > device_sms() && field_tm_fits(ngrid, two, W) && field_tm_per_sm(tm_smem_bytes(ngrid, W, two), two) == 2)
     return two;
   return kTmMaxThreads;
 }
@@ -2597,7 +2586,7 @@ void launch_field_cl(const Launch &L, const StepConstF &sc, int k, const PtrsF &
   const ClShape t = cl_shape(ngrid, W, cl);
   chain_launch(k_field_cl_f<LA, REC>, cl * ns, t.threads, t.smem, (cudaStream_t)L.stream, cl, sc, k, p, (float2 *)field,
                (const float2 *)coef, (const float2 *)pow, ns, np, ngrid, deposit, t.nseg, W, t.words, t.cols,
-               field_sms() / cl, dfield);
+               device_sms() / cl, dfield);
 }
 }  // namespace
 
@@ -2620,7 +2609,7 @@ static int cluster_slots(int cl) {
   cfg.numAttrs = 1;
   if (cudaOccupancyMaxActiveClusters(&n, k_field_cl_f<8, false>, &cfg) != cudaSuccess || n < 1) {
     cudaGetLastError();
-    n = std::max(1, field_sms() / cl);
+    n = std::max(1, device_sms() / cl);
   }
   if (dev < 64) slots[dev][cl].store(n);
   return n;
@@ -2641,8 +2630,8 @@ int field_cluster(int ngrid, int ns, int W) {
   double best = 1e30;
   int cl = 0;
   if (tm || ngrid <= fused_max_ngrid()) {
-    if (ns > field_sms() && tm) return 0;
-    best = (17 + 36 * cells) * (tm ? 1 : 1.25) * ((ns + field_sms() - 1) / field_sms());
+    if (ns > device_sms() && tm) return 0;
+    best = (17 + 36 * cells) * (tm ? 1 : 1.25) * ((ns + device_sms() - 1) / device_sms());
   } else if (!band_cluster(ngrid, W)) {
     return 0;
   }

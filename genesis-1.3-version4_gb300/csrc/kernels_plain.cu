@@ -929,8 +929,8 @@ AdiShape adi_shape(int ns, int ng, int W) {
   if (most < 2) return {0, 0, 128};
   AdiShape s{8, 4 * std::max(1, (ng + 70) / 144), 64};
   const long long bands = (long long)ns * ((ng + 7) / 8);
-  if (bands < 4 * 152) {
-    s.L = bands < 152 ? 2 : 4;
+  if (bands < 4 * device_sms()) {
+    s.L = bands < device_sms() ? 2 : 4;
     s.threads = 128;
     s.nseg = s.threads / s.L;
   } else if (most < 4) {
@@ -1009,12 +1009,12 @@ int diag_threads(int ng) {
 // fewer in a window of few slices (1 slice x 8192: 32 CTAs of 256).
 int diag_chunk(int ns, int np, int nt) {
   int m = 8;
-  while (m > 1 && (long long)ns * ((np + m * nt - 1) / (m * nt)) < 2 * 152) m /= 2;
+  while (m > 1 && (long long)ns * ((np + m * nt - 1) / (m * nt)) < 2 * device_sms()) m /= 2;
   return m * nt;
 }
 // Rows a CTA: 32, or fewer down to 2 for about four CTAs an SM.
 int diag_rows(int nslice, int ng) {
-  return (int)std::max(2LL, std::min(32LL, (long long)nslice * ng / (4 * 152)));
+  return (int)std::max(2LL, std::min(32LL, (long long)nslice * ng / (4 * device_sms())));
 }
 template <int NH>
 void launch_diag_nh(cudaStream_t s, const diag64::Args &a, unsigned blocks, int nt) {

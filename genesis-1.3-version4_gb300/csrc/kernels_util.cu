@@ -6,6 +6,7 @@
 //   fields:    host double2 <-> device float2 in the mixed form
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "g4gpu_internal.h"
@@ -105,11 +106,24 @@ __global__ void k_f2d(const float2 *in, double2 *out, size_t n) {
 }
 
 unsigned grid_for(size_t n) {
-  size_t b = (n + 255) / 256;
-  return (unsigned)(b < 152 * 32 ? (b > 0 ? b : 1) : 152 * 32);
+  const size_t b = (n + 255) / 256, most = (size_t)device_sms() * 32;
+  return (unsigned)(b < most ? (b > 0 ? b : 1) : most);
 }
 
 }  // namespace
+
+int device_sms() {
+  static std::atomic<int> sms[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int n = dev >= 0 && dev < 64 ? sms[dev].load() : 0;
+  if (!n) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 152;
+    if (dev >= 0 && dev < 64) sms[dev].store(n);
+  }
+  return n;
+}
+
 
 void launch_aos_to_soa(void *stream, const double *aos, void *const *soa, int mixed, double gref,
                        size_t n) {
