@@ -1944,21 +1944,28 @@ namespace {
 // Whether g4gpu_run_diag forms the records beside the steps: not where a step's kernel forms
 // them itself, moves the beam outside the push (coarse steps), or is being timed. Windows that
 // leave SMs idle and windows of several rounds of CTAs gain; between them the record's CTAs
-// take the place and the pipes of CTAs of the step that would all have run at once. In line /
-// beside, us a step: mixed 1 x 8192 particles, 151^2 40 / 29, 22 x 4096 37 / 30, 75 x 8192
-// 53 / 62, 300 x 8192, 101^2 98 / 102, 300 x 8192, 255^2 297 / 279, 700 x 4096 212 / 196,
-// 2048 x 8192 596 / 567; FP64 1 x 8192, 255^2 87 / 77, 2 x 8192, 151^2 70 / 62, 255^2 106 / 108,
-// 22 x 2052, 101^2 94 / 119, 64 x 4096 243 / 252, 64 x 4096, 151^2 310 / 303, 150 x 2048, 101^2
-// 354 / 338, 320 x 8192, 151^2 1969 / 1933.
+// take the place and the pipes of CTAs of the step that would all have run at once.
+// Mixed, us a step in line / beside: 1 x 8192 particles, 151^2 34 / 26, 38 x 8192 48 / 39, 75 x
+// 8192 52 / 59, 152 x 8192 68 / 75, 300 x 8192, 101^2 97 / 100, 700 x 4096 212 / 196, 608 x 8192,
+// 151^2 240 / 233. FP64: 1 x 8192, 255^2 83 / 71, 2 x 8192, 151^2 72 / 63, 255^2 102 / 109, 16 x
+// 4096, 101^2 108 / 122. An FP64 window of many slices gains from about eight bands of eight
+// lines an SM on (1216): 100 x 4096, 65^2 (900 bands) 301 / 321, 130 x 4096, 65^2 (1170) 375 /
+// 388, 64 x 4096, 101^2 (832) 247 / 257, 80 x 4096 (1040) 297 / 302, 94 x 4096 (1222) 346 / 330,
+// 64 x 4096, 151^2 (1216) 318 / 308, 150 x 2048, 65^2 (1350) 280 / 257, 320 x 8192, 151^2 1948 /
+// 1933. Its FFT solver gains from 32 slices on or so: 16 x 4096, 128^2 151 / 166, 32 x 4096 257 /
+// 238, 64 x 4096, 33^2 227 / 211.
 bool records_beside(g4gpu_handle h, int istep0, int nsteps) {
   const g4gpu_config &c = h->cfg;
   if (h->prof || h->field_kernel == 2) return false;
   for (int s = istep0; s < istep0 + nsteps && s < (int)h->substeps.size(); s++)
     if (h->substeps[s] > 1) return false;
-  const int sms = g4::device_sms();
-  if (!h->mixed) return (long long)c.nslice * c.ngrid <= 2 * sms || c.nslice >= 64;  // lines: two an SM
+  const long long ns = c.nslice, sms = g4::device_sms();
+  if (!h->mixed) {
+    if (ns * c.ngrid <= 2 * sms) return true;
+    return c.solver == G4GPU_SOLVER_FFT ? ns >= 64 : ns * ((c.ngrid + 7) / 8) >= 8 * sms;
+  }
   const int cluster = c.solver == G4GPU_SOLVER_ADI ? g4::field_cluster(c.ngrid, c.nslice, h->steps[istep0].f[0].tw) : 0;
-  return c.nslice <= sms / 4 || (long long)c.nslice * std::max(cluster, 1) >= 4 * sms;
+  return ns <= sms / 4 || ns * std::max(cluster, 1) >= 4 * sms;
 }
 }  // namespace
 
