@@ -180,8 +180,10 @@ __global__ void k_adi_cols(double2 *field, const double2 *s1, const double2 *tmp
   const double2 *w = tmp + (size_t)ii * ncell + c0;
   const int line = threadIdx.x % L, row0 = threadIdx.x / L, dr = blockDim.x / L;
   // with `edge` also the term of the columns whose cbet in the row solve has not settled
-  // (column_tables)
-  const C2 fix = c0 + line < nco ? ld(cf.pw + 3 * kSegPow + c0 + line) : C2{0, 0};
+  // (column_tables): its distance from the settled one falls by kappa^2 a column, below 2^-62
+  // after half of W
+  const int nedge = nco / 2 + 1;
+  const C2 fix = c0 + line < nedge ? ld(cf.pw + 3 * kSegPow + c0 + line) : C2{0, 0};
   auto fill = [&](bool edge) {
 #pragma unroll 4
     for (int r = row0; r < ng; r += dr) {
@@ -194,7 +196,7 @@ __global__ void k_adi_cols(double2 *field, const double2 *s1, const double2 *tmp
       T[r * L + line] = v;
     }
   };
-  if (c0 < nco)
+  if (c0 < nedge)
     fill(true);
   else
     fill(false);
