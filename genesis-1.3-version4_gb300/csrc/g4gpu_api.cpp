@@ -1276,7 +1276,7 @@ static int enqueue_coarse_step(g4gpu_handle h, int istep, int cnt) {
   {
     Timed t(h, G4GPU_K_ADI_X);
     g4::launch_field_fused_mixed(L, scf, 0, h->beam, h->field[0], cb, seg_powers(h, sc.f[0].coef), ns, np, ng, 0,
-                                 field_threads(h, sc.f[0].tw), nullptr, nullptr, 1, c.gammaref);
+                                 field_threads(h, sc.f[0].tw), nullptr);
   }
   G4_CUDA(h, cudaGetLastError());
   return G4GPU_OK;
@@ -1479,9 +1479,8 @@ static int enqueue_steps(g4gpu_handle h, int istep0, int nsteps, int stages) {
                                         band_cl);
           else
             g4::launch_field_fused_mixed(L, scf, k, h->beam, h->field[k], cb, seg_powers(h, sc.f[k].coef), ns, np, ng,
-                                         sc.f[k].dep_on, field_threads(h, sc.f[k].tw), nullptr,
-                                         rec ? h->diag_rec + (size_t)ns * bw + (size_t)k * ns * fw : nullptr,
-                                         h->diag_nharm, c.gammaref);
+                                         sc.f[k].dep_on, field_threads(h, sc.f[k].tw),
+                                         rec ? h->diag_rec + (size_t)ns * bw + (size_t)k * ns * fw : nullptr);
         }
         if (rec) h->diag_fields_in_step = true;
       }

@@ -186,13 +186,12 @@ constexpr int kMaxBandCluster = 4;
 int band_cluster(int ngrid, int W);
 void launch_field_band_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b, void *field,
                              const void *coef, int ns, int np, int ngrid, int deposit, int cl);
-// threads: CTA size, a multiple of 32 in [2 ngrid, 1024]. dbeam / dfield (may be
-// null): the step's diagnostic record, beam [nslice][beam_diag_width(nharm)] (formed by
-// the launch of field 0) and this field's [nslice][kFieldSums + 2] in storage order.
+// threads: CTA size, a multiple of 32 in [2 ngrid, 1024]. dfield (may be null): this
+// field's diagnostic record of the step, [nslice][kFieldSums + 2] in storage order.
 // pow: the coefficient set's [4][kSegPow] tables.
 void launch_field_fused_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b,
                               void *field, const void *coef, const void *pow, int ns, int np, int ngrid, int deposit,
-                              int threads, double *dbeam, double *dfield, int nharm, double gref);
+                              int threads, double *dfield);
 // The fused field step with a slice's rows split between the cl CTAs of a cluster
 // (k_field_cl_f): field_cluster gives the cluster size for a window of ns slices, 0 where one
 // CTA a slice is better or no size fits; dfield as launch_field_fused_mixed's.
@@ -233,8 +232,8 @@ void launch_isr_advance(void *stream, unsigned long long *ctr);
 
 // The whole step of a one-field window in one kernel, one CTA per slice: push,
 // deposition and ADI (mixed form, slice in shared memory, no space charge). Usable
-// where step_fused_ok; threads, dbeam, dfield as launch_field_fused_mixed's; wake and
-// isr as the push's.
+// where step_fused_ok; threads, dfield as launch_field_fused_mixed's, dbeam (may be null)
+// the beam's record [nslice][beam_diag_width(nharm)]; wake and isr as the push's.
 bool step_fused_ok(int nfield, int ngrid, int threads, bool dbeam, bool dfield, int nharm);
 void launch_step_fused_mixed(const Launch &L, const StepConstF &sc, const DeviceBeam &b, void *field,
                              const void *coef, int ns, int np, int ngrid, int deposit, int threads,

@@ -1213,8 +1213,8 @@ __device__ __forceinline__ void bulk_store(float2 *g, const float2 *s, int count
 
 // ---- diagnostics of a step recorded by the fused field kernel -----------------
 //
-// With the slice and its particles on chip, the fused kernel forms the per-slice sums
-// of k_diag_beam_f (first field only) and k_diag_field_f into the run's diagnostic
+// With the slice (and, where it pushes them, its particles) on chip, a fused kernel forms
+// the per-slice sums of k_diag_field_f (and of k_diag_beam_f) into the run's diagnostic
 // record, in the layouts of those kernels. A thread takes np / blockDim particles
 // (or ngrid^2 / blockDim cells), few enough for FP32 partial sums; the CTA folds the
 // partials in FP64.
@@ -1353,7 +1353,7 @@ __device__ __forceinline__ void slice_field_sums(const float2 *S, int ng, double
 __global__ void __launch_bounds__(kFusedMaxThreads, 1)
     k_field_fused_f(StepConstF sc, int k, PtrsF p, float2 *__restrict__ field,
                     const float2 *__restrict__ coef, int ns, int np, int ng, int deposit, int *err,
-                    double *dbeam, double *dfield, int nharm, double gref) {
+                    double *dfield) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int ncell = ng * ng;
   const FieldStepF &fs = sc.f[k];
@@ -1394,8 +1394,6 @@ __global__ void __launch_bounds__(kFusedMaxThreads, 1)
   double *dsh = reinterpret_cast<double *>(smem_raw + ((soff + (size_t)ncell * 8 + 15) & ~(size_t)15));
   double *dres = dsh + (blockDim.x >> 5) * kFusedDiagValues;
   bulk_load_issue(S, u, ncell, bar_s);
-  // the beam record of this slice while the field is in flight
-  if (dbeam) slice_beam_sums(p, gref, is, np, nharm, dsh, dres, dbeam + (size_t)is * beam_diag_width(nharm));
   if (!bulk_load_wait(bar_s, err)) return;
   const float cs = fs.cstep;
   const int tid = threadIdx.x;
@@ -2672,18 +2670,18 @@ int fused_max_ngrid() {
 
 void launch_field_fused_mixed(const Launch &L, const StepConstF &sc, int k, const DeviceBeam &b,
                               void *field, const void *coef, const void *pow, int ns, int np, int ngrid, int deposit,
-                              int threads, double *dbeam, double *dfield, int nharm, double gref) {
+                              int threads, double *dfield) {
   static std::atomic<unsigned long long> configured{0};  // one bit per device
   threads = fused_threads(ngrid, threads);
   const int W = sc.f[k].tw;
-  if (!dbeam && field_tm_fits(ngrid, threads, W)) {
+  if (field_tm_fits(ngrid, threads, W)) {
     PtrsF p = make_ptrs_f(b, nullptr, nullptr, 0);
     const auto launch = W <= 9 ? (dfield ? launch_field_tm<8, true> : launch_field_tm<8, false>)
                                : (dfield ? launch_field_tm<kTmLook, true> : launch_field_tm<kTmLook, false>);
     launch(L, sc, k, p, field, coef, pow, ns, np, ngrid, deposit, threads, dfield);
     return;
   }
-  size_t smem = (dbeam || dfield) ? fused_diag_smem_bytes(ngrid, threads) : fused_smem_bytes(ngrid);
+  size_t smem = dfield ? fused_diag_smem_bytes(ngrid, threads) : fused_smem_bytes(ngrid);
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(configured.load() & (1ull << dev))) {
@@ -2692,7 +2690,7 @@ void launch_field_fused_mixed(const Launch &L, const StepConstF &sc, int k, cons
   }
   PtrsF p = make_ptrs_f(b, nullptr, nullptr, 0);
   k_field_fused_f<<<ns, threads, smem, (cudaStream_t)L.stream>>>(
-      sc, k, p, (float2 *)field, (const float2 *)coef, ns, np, ngrid, deposit, L.err, dbeam, dfield, nharm, gref);
+      sc, k, p, (float2 *)field, (const float2 *)coef, ns, np, ngrid, deposit, L.err, dfield);
 }
 
 void launch_source_substep_mixed(const Launch &L, const StepConstF &sc, const DeviceBeam &b, const void *tp,
