@@ -331,8 +331,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   const int nq = words >> 4;  // batches of eight rows
   const int nchunk = ((ng + nseg - 1) / nseg + kTmChunk - 1) / kTmChunk;
   const float cs = fs.cstep;
-  // settled cbet of the row and of the column solve (column_tables, g4gpu_api.cpp)
-  const float2 cb = coef[2 * ng - 1], cbc = pows[3 * kSegPow - 1], kap = PW[0], zero = make_float2(0.f, 0.f);
+  const float2 cb = coef[2 * ng - 1], kap = PW[0], zero = make_float2(0.f, 0.f);
   // the part of a segment's solution that reaches it over its ends: its neighbour's at the
   // end, times kappa per row; at the grid's edges minus the mirror image of its own (the
   // field is zero one row outside)
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
     // neighbours' carries (writing the rows without carries from the solve itself: 631 against
     // 640 us for 4096 slices of 151^2, 257 against 250 us for 2000 of 117^2)
     float2 *L = S + line;
-    tm_solve_cols<LA>(L, tm, st, b, e, nq, nchunk, cs, cbc, kap);
+    tm_solve_cols<LA>(L, tm, st, b, e, nq, nchunk, cs, cb, kap);
     __syncthreads();
     float2 f[8];
     {
@@ -520,8 +519,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   const bool left = act && r0 + b > 0, right = act && r0 + e < ng;
   const int nq = words >> 4;  // batches of eight rows
   const float cs = fs.cstep;
-  // settled cbet of the row and of the column solve (column_tables, g4gpu_api.cpp)
-  const float2 cb = coef[2 * ng - 1], cbc = pows[3 * kSegPow - 1], kap = PW[0], zero = make_float2(0.f, 0.f);
+  const float2 cb = coef[2 * ng - 1], kap = PW[0], zero = make_float2(0.f, 0.f);
   auto carry = [&](bool inner, float2 other, float2 own) { return inner ? other : cmulf(make_float2(-kap.x, -kap.y), own); };
 
   const bool cols_on = __any_sync(0xffffffffu, act);  // warps without a column have nothing to issue
@@ -575,7 +573,7 @@ __global__ void __launch_bounds__(kTmMaxThreads, 1)
   }
   __syncthreads();
   float2 *L = S + line;
-  if (cols_on) tm_solve_cols<LA>(L, tm, st, b, e, nq, ((nmax + nseg - 1) / nseg + kTmChunk - 1) / kTmChunk, cs, cbc, kap);
+  if (cols_on) tm_solve_cols<LA>(L, tm, st, b, e, nq, ((nmax + nseg - 1) / nseg + kTmChunk - 1) / kTmChunk, cs, cb, kap);
   __syncwarp();
   cl.sync();  // the neighbours' edge rows are solved, and nobody reads u any more
   float2 f[8];

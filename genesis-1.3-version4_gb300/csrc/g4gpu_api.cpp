@@ -163,19 +163,20 @@ void adi_coefficients(double delz, double dgrid, double xks, int ngrid, std::vec
   }
 }
 
-// Two tables of kSegPow entries for the steps whose second right-hand side is 2 u' - S1
-// (adi_plain.cuh, field_tm.cuh): cbet of the column solve, whose last entry is the settled
-// value, and what the first columns add to 2 u' - S1, as a multiple of u'. A rounded cbet
+// Two tables of kSegPow entries for the FP64 steps whose second right-hand side is 2 u' - S1
+// (adi_plain.cuh): cbet of the column solve, whose last entry is the settled value, and
+// what the first columns add to 2 u' - S1, as a multiple of u'. A rounded cbet
 // scales every solution by 1 + e, the same e in every step, which outgrows the random
 // roundings; 2 u' - S1 carries the row solve's e twice. The column solve's cbet is therefore
 // the rounded (1 - 2 e) beta: what is left of a step's 3 e is the rounding of one number.
-// Before it settles, cbet has another e in every entry, so the FP64 solve's first columns add
-// their 2 (e - e_j) u'. Field of 151^2 after 100 FP64 steps of factor 0.034, rms error against
+// Before it settles, cbet has another e in every entry, so the solve's first columns add
+// their 2 (e - e_j) u'. Field of 151^2 after 100 steps of factor 0.034, rms error against
 // extended precision 1.25e-14 -> 3.1e-15 (8.2e-15 with the stencil's second right-hand side and
-// cbet for both); after 60 mixed steps, against FP64, 4.0e-6 -> 1.2e-6 (3.9e-6).
+// cbet for both). The mixed form keeps one cbet: its field would gain as much (4.0e-6 -> 1.2e-6
+// of it after 60 steps), but its results move by 1e-5 over a run, as far as they are from FP64.
 // The exact beta_i = 1 / (w2 - c cwet_i) = 1 / (1 + 2 i r + r^2 beta_{i-1}) is cbet[i] + low[i]:
 // one Newton step from the residual, formed with exact products.
-std::vector<std::complex<double>> column_tables(const std::vector<std::complex<double>> &cbet, double r, bool mixed) {
+std::vector<std::complex<double>> column_tables(const std::vector<std::complex<double>> &cbet, double r) {
   typedef std::complex<double> cd;
   struct Two {
     double hi, lo;
@@ -205,9 +206,7 @@ std::vector<std::complex<double>> column_tables(const std::vector<std::complex<d
                -(((ri.hi + ir.hi) + ri.lo) + ir.lo + tr.lo * b.imag() + ti.lo * b.real()));
     low[i] = b * e;
   }
-  // the row solve's settled cbet, as its kernel holds it, relative to beta
-  const cd bs = cbet[n - 1], held = mixed ? cd((float)bs.real(), (float)bs.imag()) : bs;
-  const cd e = ((held - bs) - low[n - 1]) / bs;
+  const cd e = -low[n - 1] / cbet[n - 1];  // of the row solve's settled cbet
   std::vector<cd> out(2 * g4::kSegPow);
   for (int j = 0; j < g4::kSegPow; j++) {
     const int i = std::min(j, n - 1);
@@ -589,7 +588,7 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
           }
           pows.insert(pows.end(), pw.begin(), pw.end());
           for (const cd &v : pw) pows.push_back(v * q);
-          pw = column_tables(cb, cs, h->mixed);
+          pw = column_tables(cb, cs);
           pows.insert(pows.end(), pw.begin(), pw.end());
         }
         it = sets.find(key);
