@@ -172,33 +172,22 @@ __global__ void k_adi_cols(double2 *field, const double2 *s1, const double2 *tmp
   extern __shared__ __align__(16) unsigned char adi_smem[];
   const Lines ln = lines_setup(adi_smem, L, nseg, nco, W, ng, cf);  // tables: no kernel writes them
   const int ii = blockIdx.x / nband, c0 = (blockIdx.x - ii * nband) * L, nc = min(L, ng - c0);
-  const int line = threadIdx.x % L, row0 = threadIdx.x / L, dr = blockDim.x / L;
-  // the columns whose cbet in the row solve has not settled, and their term (column_tables): its
-  // distance from the settled one falls by kappa^2 a column, below 2^-62 after half of W
-  const int nedge = nco / 2 + 1;
-  const C2 fix = c0 + line < nedge ? ld(cf.pw + 3 * kSegPow + c0 + line) : C2{0, 0};
   chain_wait();
   C2 *T = ln.T;
   const size_t ncell = (size_t)ng * ng;
   double2 *u = field + (size_t)((ii + first) % ns) * ncell + c0;
   const double2 *a = s1 + (size_t)ii * ncell + c0;
   const double2 *w = tmp + (size_t)ii * ncell + c0;
-  auto fill = [&](bool edge) {
+  const int line = threadIdx.x % L, row0 = threadIdx.x / L, dr = blockDim.x / L;
 #pragma unroll 4
-    for (int r = row0; r < ng; r += dr) {
-      C2 v = {0, 0};
-      if (line < nc) {
-        const C2 wv = ld(w + (size_t)r * ng + line), av = ld(a + (size_t)r * ng + line);
-        v = C2{fma(2., wv.x, -av.x), fma(2., wv.y, -av.y)};
-        if (edge) v = sub_cmul(v, C2{-fix.x, -fix.y}, wv);
-      }
-      T[r * L + line] = v;
+  for (int r = row0; r < ng; r += dr) {
+    C2 v = {0, 0};
+    if (line < nc) {
+      const C2 wv = ld(w + (size_t)r * ng + line), av = ld(a + (size_t)r * ng + line);
+      v = C2{fma(2., wv.x, -av.x), fma(2., wv.y, -av.y)};
     }
-  };
-  if (c0 < nedge)
-    fill(true);
-  else
-    fill(false);
+    T[r * L + line] = v;
+  }
   __syncthreads();
   solve_lines(ln, L, 1, L, ng, nseg, nco, W, c);
   if (line < nc)

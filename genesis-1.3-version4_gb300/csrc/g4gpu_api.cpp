@@ -163,20 +163,20 @@ void adi_coefficients(double delz, double dgrid, double xks, int ngrid, std::vec
   }
 }
 
-// Two tables of kSegPow entries for the FP64 steps whose second right-hand side is 2 u' - S1
-// (adi_plain.cuh): cbet of the column solve, whose last entry is the settled value, and
-// what the first columns add to 2 u' - S1, as a multiple of u'. A rounded cbet
+// cbet of the column and of the row solve ([2][kSegPow], the last entries the settled values) for
+// the FP64 steps whose second right-hand side is 2 u' - S1 (adi_plain.cuh). A rounded cbet
 // scales every solution by 1 + e, the same e in every step, which outgrows the random
 // roundings; 2 u' - S1 carries the row solve's e twice. The column solve's cbet is therefore
 // the rounded (1 - 2 e) beta: what is left of a step's 3 e is the rounding of one number.
-// Before it settles, cbet has another e in every entry, so the solve's first columns add
-// their 2 (e - e_j) u'. Field of 151^2 after 100 steps of factor 0.034, rms error against
-// extended precision 1.25e-14 -> 3.1e-15 (8.2e-15 with the stencil's second right-hand side and
-// cbet for both). The mixed form keeps one cbet: its field would gain as much (4.0e-6 -> 1.2e-6
+// The row solve's entries before it settles are rounded from (1 + e) beta_i, so that every
+// column finds about the same e (a term for what is left in the first columns cost 2 to 8 % of
+// the column pass). Field of 151^2 after 100 steps of factor 0.034, rms error against extended
+// precision 1.25e-14 -> 3.2e-15 (8.2e-15 with the stencil's second right-hand side and one
+// cbet). The mixed form keeps one cbet: its field would gain as much (4.0e-6 -> 1.2e-6
 // of it after 60 steps), but its results move by 1e-5 over a run, as far as they are from FP64.
 // The exact beta_i = 1 / (w2 - c cwet_i) = 1 / (1 + 2 i r + r^2 beta_{i-1}) is cbet[i] + low[i]:
 // one Newton step from the residual, formed with exact products.
-std::vector<std::complex<double>> column_tables(const std::vector<std::complex<double>> &cbet, double r) {
+std::vector<std::complex<double>> solve_cbets(const std::vector<std::complex<double>> &cbet, double r) {
   typedef std::complex<double> cd;
   struct Two {
     double hi, lo;
@@ -211,7 +211,7 @@ std::vector<std::complex<double>> column_tables(const std::vector<std::complex<d
   for (int j = 0; j < g4::kSegPow; j++) {
     const int i = std::min(j, n - 1);
     out[j] = cbet[i] + (low[i] - 2. * e * cbet[i]);
-    out[g4::kSegPow + j] = 2. * (e + low[i] / cbet[i]);
+    out[g4::kSegPow + j] = cbet[i] + (low[i] + e * cbet[i]);
   }
   return out;
 }
@@ -588,7 +588,7 @@ int g4gpu_set_lattice(g4gpu_handle h, int nsteps, const double *tab) {
           }
           pows.insert(pows.end(), pw.begin(), pw.end());
           for (const cd &v : pw) pows.push_back(v * q);
-          pw = column_tables(cb, cs);
+          pw = solve_cbets(cb, cs);
           pows.insert(pows.end(), pw.begin(), pw.end());
         }
         it = sets.find(key);

@@ -17,8 +17,8 @@ constexpr double kEev = 510998.95069;
 constexpr double kCe = 4.8032045e-11;
 
 // Entries of a coefficient set's four tables for the segmented solves: kappa^{j+1},
-// kappa^{j+1} / (1 - kappa^2), cbet of the column solve and the first columns' factors
-// (column_tables, g4gpu_api.cpp): the largest warm-up length segment_warmup returns for 62 bits
+// kappa^{j+1} / (1 - kappa^2), cbet of the FP64 column and row solve
+// (solve_cbets, g4gpu_api.cpp): the largest warm-up length segment_warmup returns for 62 bits
 constexpr int kSegPow = 41;
 
 // Per field, per integration step constants.

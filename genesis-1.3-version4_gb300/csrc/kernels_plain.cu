@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(256) k_deposit(StepConst sc, Ptrs p, int ns, i
 
 // ADI coefficient set: c[ng], cbet[ng], cwet[ng] (FieldSolverADI.cpp:125-182), and the
 // segmented solves' powers [2][kSegPow]: kappa^{j+1}, kappa^{j+1} / (1 - kappa^2), followed
-// by column_tables' two (g4gpu_api.cpp)
+// by cbet of the column and of the row solve (solve_cbets, g4gpu_api.cpp)
 struct Coef {
   const double2 *c, *cbet, *cwet, *pw;
 };
@@ -977,7 +977,7 @@ void launch_adi_plain(const Launch &L, const StepConst &sc, int k, int phase, vo
   const FieldStep &f = sc.f[k];
   const double2 *pw = (const double2 *)pow;
   const AdiShape a = adi_shape(ns, ngrid, f.tw);
-  const Coef cf{cb, phase == 1 && a.L ? pw + 2 * kSegPow : cb + ngrid, cb + 2 * ngrid, pw};
+  const Coef cf{cb, a.L ? pw + (phase == 1 ? 2 : 3) * kSegPow : cb + ngrid, cb + 2 * ngrid, pw};
   double2 *u = (double2 *)field, *sv = (double2 *)src, *w = (double2 *)tmp;
   switch (a.L) {
     case 2: return launch_adi_lines<2>(s, phase, a, u, sv, w, cf, f.cstep, ns, ngrid, f.first, f.tw, has_src);
