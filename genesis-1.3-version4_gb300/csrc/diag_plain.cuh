@@ -63,13 +63,17 @@ __device__ __forceinline__ void fold(const long long (&v)[NV], int nsum, int nmi
     long long a = r[i];
     if (k < nsum) {
       // four partial sums: shorter chains of roundings and of latencies (n4 is a multiple of 8)
-      double s[4] = {0, 0, 0, 0};
-      for (int j = 0; j < n4; j += 4)
+      double s[4];
+      auto next = [&] {
+        const double v = __longlong_as_double(r[i]);
+        i = i + 1 < n4 ? i + 1 : 0;
+        return v;
+      };
 #pragma unroll
-        for (int w = 0; w < 4; w++) {
-          s[w] += __longlong_as_double(r[i]);
-          i = i + 1 < n4 ? i + 1 : 0;
-        }
+      for (int w = 0; w < 4; w++) s[w] = next();
+      for (int j = 4; j < n4; j += 4)
+#pragma unroll
+        for (int w = 0; w < 4; w++) s[w] += next();
       a = __double_as_longlong((s[0] + s[1]) + (s[2] + s[3]));
     } else {
       const bool lo = k < nsum + nmin;
@@ -211,8 +215,8 @@ __device__ __forceinline__ void field_rows(const Args &a, int k, int i, int c, l
   double s[NV] = {0};
   for (int col = tid; col < ng; col += blockDim.x) {
     double s2[2] = {0, 0};
-    auto row = [&](int r, double &sw) {
-      const double2 u = f[(size_t)(r0 + r) * ng + col], d = dy[r];
+    auto row = [&](int r, double2 u, double &sw) {
+      const double2 d = dy[r];
       const double w = fma(u.x, u.x, u.y * u.y);
       sw += w;
       s[3] = fma(d.x, w, s[3]);
@@ -220,13 +224,14 @@ __device__ __forceinline__ void field_rows(const Args &a, int k, int i, int c, l
       s[5] += u.x;
       s[6] += u.y;
     };
-    int r = 0;
-#pragma unroll 2
-    for (; r + 1 < nr; r += 2) {
-      row(r, s2[0]);
-      row(r + 1, s2[1]);
+    for (int r4 = 0; r4 < nr; r4 += 4) {  // four rows' loads together
+      double2 u[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) u[q] = f[(size_t)(r0 + min(r4 + q, nr - 1)) * ng + col];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (r4 + q < nr) row(r4 + q, u[q], s2[q & 1]);
     }
-    if (r < nr) row(r, s2[0]);
     const double sw = s2[0] + s2[1];
     const double dx = (double)col + shift, t = dx * sw;
     s[0] += sw;
