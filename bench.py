@@ -200,7 +200,7 @@ TRAFFIC_SOURCE = "ncu capture of a 608-slice window, scaled to the launch's slic
 # per cell of the plain ADI's row and column pass, from ncu captures of a 152-slice window
 # (profiles/ncu_step_kernels.md); nominal GB300 FP64 rate: 1.25 TFLOP/s
 # with FMA counted as two operations, i.e. 625 G FP64 instructions/s.
-FP64_INSTR = {"push_per_particle": 222.1, "rows_per_cell": 20.7, "cols_per_cell": 14.7}
+FP64_INSTR = {"push_per_particle": 223.1, "rows_per_cell": 20.7, "cols_per_cell": 14.7}
 FP64_NOMINAL_GINSTR = 625.0
 
 

@@ -27,9 +27,9 @@
 // they are written to u. Rows have an odd stride st, so that the row solve, whose lanes walk
 // different rows, finds different banks on even grids too.
 // Measured (after 20 steps, k_field_fused_f at its best CTA size before): 4096 slices x 8192
-// particles, 151^2 1000 -> 641 us (3.4 TB/s of the algorithmic bytes, half of the copy
-// bandwidth); 700 x 8192, 151^2 197 -> 134 us; 2000 x 4096, 117^2 253 -> 197 us; 700 x 8192,
-// 128^2 336 -> 112 us. Of a slice's 46 thousand cycles the deposition takes 12, the column solve
+// particles, 151^2 1000 -> 630 us (3.4 TB/s of the algorithmic bytes; the DRAM traffic, part of
+// the particles still being in L2, is 44 % of the copy bandwidth); 700 x 8192, 151^2 197 ->
+// 128 us; 2000 x 4096, 117^2 253 -> 193 us; 700 x 8192, 128^2 336 -> 106 us. Of a slice's 46 thousand cycles the deposition takes 12, the column solve
 // 10, the row solve 7, the last pass 7, S1 5, the rows' carries 3.
 
 // Sixteen words (eight complex values) of this thread's tensor memory.

@@ -1007,11 +1007,11 @@ static int field_threads(g4gpu_handle h, int W) {
 }
 
 // Threads a block of the push: as set (g4gpu_set_launch_shapes, g4gpu_autotune), else by
-// the window. The FP64 push holds a scheduler for ~400 x 64 cycles a warp, so a window of
+// the window. The FP64 push holds a scheduler for 223 x 64 cycles a warp, so a window of
 // few particles takes small blocks that spread over the SMs (64 against 256 threads:
-// 1 x 8192 particles 26 / 40 us, 22 x 2052 49 / 71, 4 x 8192 41 / 43; 64 x 4096 235 / 231).
-// The mixed push is bound by memory and issue: 128 (700 x 8192 94.7 us, 256 threads 97.1,
-// 512 104.6, 32 115).
+// 1 x 8192 particles 20 / 27 us, 22 x 2052 31 / 43, 4 x 8192 26 / 29, 9 x 8192 43 / 43; 64 x
+// 4096 131 / 129). The mixed push is bound by memory and issue: 128 (700 x 8192 94 us, 256
+// threads 95, 512 102, 32 185).
 static int push_threads(g4gpu_handle h) {
   if (h->push_block > 0) return h->push_block;
   if (h->mixed) return 128;

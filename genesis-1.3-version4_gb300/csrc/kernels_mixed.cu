@@ -2533,8 +2533,11 @@ namespace {
 bool field_tm_fits(int ngrid, int threads, int W) {
   return tm_shape(ngrid, threads, W).threads > 0 && tm_smem_bytes(ngrid, W, threads) <= 227u * 1024u - 16;
 }
-// CTAs of k_field_tm_f an SM holds: one, or two where the shared memory and the tensor memory
-// of two fit (its 80 registers a thread allow two of 384)
+// CTAs of k_field_tm_f launched an SM: one, or two where the shared memory and the registers of
+// two fit (80 a thread: two of 384). 288 to 320 threads on grids of 97 to 119 leave tensor
+// memory for one, and the second waits until the first has done its slices; one CTA an SM would
+// take as long (103 us for 700 slices of 101^2) but lets the next launch's CTAs find room for two
+// on one SM and for none on another (a step 161 us by twos, 237 by ones).
 int field_tm_per_sm(size_t smem, int threads) {
   return threads <= 384 && 2 * (smem + 1024 + 16) <= 228 * 1024 ? 2 : 1;
 }

@@ -1,10 +1,13 @@
-// FP64 kernels of the undulator step with the reference's arithmetic.
+// FP64 kernels of the undulator step.
 //
-// This translation unit is compiled with --fmad=false so that every product and
-// sum rounds separately, as the reference's x86-64 build does; together with the
-// IEEE-rounded division and square root of CUDA, only the transcendental
-// functions (sin, cos, sinh, cosh of the CUDA math library) differ in the last
-// bits from the reference. Operation order follows the cited reference lines.
+// The values are the reference's to a few roundings, not bit for bit: products are fused
+// into sums where the code says fma (the unit is compiled with --fmad=false, so nowhere
+// else), quotients by gamma and gammaz are products with reciprocals, phases are turned
+// instead of passed through sin and cos, the focusing maps and the undulator's factor are
+// short series in their usual range, and the ADI's lines are solved in segments
+// (adi_plain.cuh). Where a last bit is amplified, it is the reference's: 1 / btpar0 is the
+// rounded quotient of the rounded root (recip_sqrt_1m). Operation order otherwise follows
+// the cited reference lines.
 //
 // Layout: particles are structure-of-arrays, slice-major (index is*np + ip);
 // fields are [nslice][ngrid*ngrid] double2, storage order with the ring start
@@ -237,7 +240,7 @@ __device__ __forceinline__ double recip_sqrt_near1(double a) {
 //   sqrt(a) = 1 - S 2^-53:  S = M/2 + M^2 2^-56 + M^3 2^-110, to the nearest integer;
 //   1 / sqrt = 1 + Q 2^-52: Q = S/2 + S^2 2^-54 + S^3 2^-107, to the nearest integer;
 // the terms left out are below 2^-44 of a unit, and neither value is ever halfway between
-// two doubles. Equal to 1. / sqrt(a) on 3e8 random M and the first 5e6. About 45 integer
+// two doubles. Equal to 1. / sqrt(a) for every M of the range. About 45 integer
 // instructions for 12 FP64 ones, four times a particle.
 __device__ __forceinline__ void recip_sqrt_1m(double a, double &ib, double &om) {
   constexpr long long kOne = 0x3FF0000000000000LL;
